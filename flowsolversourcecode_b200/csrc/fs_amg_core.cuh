@@ -1,68 +1,76 @@
-// Krylov solve with the V-cycle preconditioner (PCycle) and the grid
-// reductions it uses.  Included twice by fs_mg.cu:
-//   FS_GROUPS 0: the whole cooperative grid solves one system; CTA index and
-//     count are the grid's and the grid barrier is the cooperative one;
+// Krylov solve with the V-cycle preconditioner and the grid reductions it
+// uses.  Included twice by fs_mg.cu:
+//   FS_GROUPS 0: the whole cooperative grid solves one system;
 //   FS_GROUPS 1: the CTAs of one cooperative launch are split into groups, one
 //     per system (the batched p' solve of an ensemble); CTA index and count are
-//     relative to the group, held in shared memory, and the grid barrier is a
-//     bounded barrier among the group's CTAs in global memory.
-#if FS_GROUPS
-struct GroupState {
-  int cta, ncta, q;   // this CTA within its group, the group's CTAs, its system
-  unsigned gen;       // generation of the group barrier this CTA waits to leave
-  unsigned *bar;      // [0] arrivals, [1] generation (zero at launch)
-  int32_t *status;    // [0] set when a barrier timed out
+//     relative to the group, held in shared memory.
+// Either way the grid barrier is a bounded one in global memory among the CTAs
+// of the system.
+struct GridState {
+  int cta, ncta, q;    // this CTA within its group, the group's CTAs, its system
+  unsigned target;     // arrivals in all when the next barrier opens, less `arrivals`
+  unsigned arrivals;   // arrivals per barrier
+  unsigned *bar;       // arrival count, zero at launch, never reset
+  int32_t *status;     // [0] set when a barrier timed out
 };
-__device__ __forceinline__ GroupState &gstate() {
-  __shared__ GroupState g;
+__device__ __forceinline__ GridState &gstate() {
+  __shared__ GridState g;
   return g;
 }
+#if FS_GROUPS
 __device__ __forceinline__ int cta_id() { return gstate().cta; }
 __device__ __forceinline__ int cta_count() { return gstate().ncta; }
-// barrier among the group's CTAs: the last arrival resets the count and bumps
-// the generation the others poll; polls are bounded, a timeout is recorded in
-// the system's status word, and once it is set no barrier waits any more
-__device__ void group_sync() {
-  GroupState &G = gstate();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned gen = G.gen;
-    if (atomicAdd(&G.bar[0], 1u) == (unsigned)G.ncta - 1) {
-      atomicExch(&G.bar[0], 0u);
-      __threadfence();
-      atomicAdd(&G.bar[1], 1u);
-    } else {
-      const volatile unsigned *vg = G.bar + 1;
-      const volatile int32_t *vs = G.status;
-      long spins = 0;
-      while (*vg == gen && *vs == 0) {
-        if (++spins > FS_PC_SPIN_LIMIT) { atomicExch(G.status, 1); break; }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-    G.gen = gen + 1;
-  }
-  __syncthreads();
-}
 #else
 __device__ __forceinline__ int cta_id() { return (int)blockIdx.x; }
 __device__ __forceinline__ int cta_count() { return (int)gridDim.x; }
 #endif
+// before the first barrier, by every thread; `extra` arrivals never come (only
+// to test the timeout)
+__device__ __forceinline__ void grid_state_init(unsigned *bar, int32_t *status, int extra) {
+  if (threadIdx.x == 0) {
+    GridState &G = gstate();
+    G.target = 0;
+    G.arrivals = (unsigned)(cta_count() + extra);
+    G.bar = bar;
+    G.status = status;
+  }
+  __syncthreads();
+}
+// Barrier among the system's CTAs, all co-resident (cooperative launch): one
+// release-add per CTA on a count that only grows, then acquire polls until it
+// reaches the next multiple of the CTA count -- one round trip to the L2 for
+// the arrival and one for the poll that sees the last one, no reset and no
+// second word.  Polls are bounded; a timeout is recorded in the system's
+// status word, and once that is set no barrier waits for long any more.
+__device__ __noinline__ void grid_barrier() {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    GridState &G = gstate();
+    const unsigned target = G.target + G.arrivals;
+    unsigned *bar = G.bar;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    long spins = 0;
+    unsigned seen;
+    while (true) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+      if ((int)(seen - target) >= 0) break;
+      if ((++spins & 63) == 0) {
+        if (*(const volatile int32_t *)G.status != 0) break;
+        if (spins > FS_PC_SPIN_LIMIT) { atomicExch(G.status, 1); break; }
+      }
+    }
+    G.target = target;
+  }
+  __syncthreads();
+}
 
 struct Sync {
-  cg::grid_group grid;
   double *part;
   int buf, buf3;
-  __device__ Sync(double *p) : grid(cg::this_grid()), part(p), buf(0), buf3(0) {}
-  __device__ __forceinline__ void gbar() {
-#if FS_GROUPS
-    group_sync();
-#else
-    grid.sync();
-#endif
+  __device__ Sync(double *p, unsigned *bar, int32_t *status, int extra) : part(p), buf(0), buf3(0) {
+    grid_state_init(bar, status, extra);
   }
+  __device__ __forceinline__ void gbar() { grid_barrier(); }
   __device__ void all() { gbar(); }
   // grid-deterministic sum of two values (every CTA gets the same result)
   __device__ void sum2(double a0, double a1, double &o0, double &o1) {
@@ -215,7 +223,6 @@ struct PCycle {
   int32_t *status;       // [0] set when a team barrier timed out
   unsigned gen;          // generation this CTA waits to leave
   int extra;             // arrivals waited for beyond the team (0; >0 only to test the timeout)
-  bool synced;           // the next enter() needs no barrier (the caller has just passed one)
   __device__ R om(int l) const { return l == 0 ? omega0 : omega; }
   __device__ R al(int l) const { return l == 0 ? alpha0 : alpha; }
   // barrier among the team CTAs: the arrival count in global memory, the last
@@ -255,8 +262,7 @@ struct PCycle {
   // the barrier before a phase: grid-wide when the grid is involved on either
   // side, among the team when the team is, else within CTA 0
   __device__ void enter(const Scope &sc) {
-    if (synced) synced = false;
-    else if (sc.grid || last.grid) S.all();
+    if (sc.grid || last.grid) S.all();
     else if (sc.team || last.team) { if (cta_id() < team_size()) team_sync(); }
     else __syncthreads();
     last = sc;
@@ -406,306 +412,6 @@ struct PCycle {
     enter(g);
   }
 
-  // ------------------------------------------------------------ fused V-cycle
-  // The same V-cycle (one pre- and one post-sweep, dense coarsest inverse) in
-  // one barrier phase per level and leg, with the same arithmetic in the same
-  // order as run():
-  //   down: the restriction into level l+1 forms the residual of each child
-  //     on the fly (no residual array, no phase of its own) for the first
-  //     FS_PC_FUSE_DOWN levels; a warp takes a chunk of coarse rows, a lane
-  //     two children, and each coarse row sums its children's residuals in
-  //     ascending order through shuffles;
-  //   up: the sweep of a row of level l >= 2 scatters its new value, times
-  //     alpha, to the row's children on level l-1 (the prolongation: every
-  //     finer row has one parent, so no two writes meet), and the coarsest
-  //     level's dense solve does the same; level 1's sweep keeps its values
-  //     and level 0 gathers them through parent (prolong0); level 0's sweep
-  //     writes `out`.  (The restriction fused with the residual measured
-  //     slower than the two phases on every level, so FS_PC_FUSE_DOWN is 0.)
-  // The caller has set x_0 = omega0 in / ac_0 and passed a grid barrier.
-  __device__ void restrict_fused(int l, const double *__restrict__ in) {
-    const LevelDev<R> L = lev[l], C = lev[l + 1];
-    Scope sc = pc_scope(L);
-    enter(sc);
-    if (!sc.active()) return;
-    const bool first_sweep = l + 1 < lc || !direct;
-    const R omc = om(l + 1);
-    const int lane = threadIdx.x & 31;
-    const long w0 = sc.tid0() >> 5, nw = sc.nth() >> 5;
-    for (long k = w0; k < C.nchunk; k += nw) {
-      const int P0 = C.chunk[k], P1 = C.chunk[k + 1];
-      const int e0 = C.rptr[P0], e1 = C.rptr[P1];
-      const int P = P0 + lane;
-      const bool hasP = P < P1;
-      const int ra0 = hasP ? C.rptr[P] : e1, ra1 = hasP ? C.rptr[P + 1] : e1;
-      R s = 0.;
-      for (int base = e0; base < e1; base += 64) {
-        const int ea = base + lane, eb = ea + 32;
-        const bool hb = eb < e1;
-        const long ia = C.rlist[ea < e1 ? ea : e0], ib = C.rlist[hb ? eb : e0];
-        R t1 = 0., t2 = 0.;
-        ell_acc2<6, false>(t1, t2, L.n, L.w, L.nbr, L.anb, ia, ib, hb, [&](int q) { return L.x[q]; });
-        const R va = (l == 0 ? (R)in[ia] : L.b[ia]) - L.ac[ia] * L.x[ia] - t1;
-        R vb = 0.;
-        if (hb) vb = (l == 0 ? (R)in[ib] : L.b[ib]) - L.ac[ib] * L.x[ib] - t2;
-        // this lane's coarse row: its children inside [base, base+64), in order
-        const int lo = ra0 > base ? ra0 : base, hi = ra1 < base + 64 ? ra1 : base + 64;
-        const int cnt = hi > lo ? hi - lo : 0;
-        const int mx = __reduce_max_sync(0xffffffffu, cnt);
-        for (int m = 0; m < mx; m++) {
-          const int off = lo + m - base;
-          const R xa = __shfl_sync(0xffffffffu, va, off & 31);
-          const R xb = __shfl_sync(0xffffffffu, vb, off & 31);
-          if (m < cnt) s = s + (off < 32 ? xa : xb);
-        }
-      }
-      if (hasP) {
-        C.b[P] = s;
-        if (first_sweep) C.x[P] = omc * s / C.ac[P];
-      }
-    }
-  }
-  // the residual phase and the restriction of run() (levels past FS_PC_FUSE_DOWN)
-  __device__ void restrict_plain(int l, const double *__restrict__ in) {
-    const LevelDev<R> L = lev[l], C = lev[l + 1];
-    residual(l, in, L.x, L.r);
-    Scope scc = pc_scope(C);
-    enter(scc);
-    if (!scc.active()) return;
-    const bool first_sweep = l + 1 < lc || !direct;
-    if (scc.nth() < 2L * C.n) {
-      for (long P = scc.tid0(); P < C.n; P += scc.nth()) {
-        R s = 0.;
-        const int c0 = C.rptr[P], c1 = C.rptr[P + 1];
-        // children's residuals eight at a time: their list entries, then their
-        // values, all in flight before the (ascending) sum
-        for (int c = c0; c < c1; c += 8) {
-          int f[8];
-          R v[8];
-#pragma unroll
-          for (int u = 0; u < 8; u++) f[u] = c + u < c1 ? C.rlist[c + u] : -1;
-#pragma unroll
-          for (int u = 0; u < 8; u++) v[u] = f[u] >= 0 ? L.r[f[u]] : (R)0.;
-#pragma unroll
-          for (int u = 0; u < 8; u++) if (f[u] >= 0) s = s + v[u];
-        }
-        C.b[P] = s;
-        if (first_sweep) C.x[P] = om(l + 1) * s / C.ac[P];
-      }
-    } else
-      level_rows(scc, C.n, l + 1, [&](auto gg, long P, bool act, int q) {
-        constexpr int G = decltype(gg)::value;
-        R s = 0.;
-        if (act)
-          for (int c = C.rptr[P] + q; c < C.rptr[P + 1]; c += G) s = s + L.r[C.rlist[c]];
-        s = gsum<G>(s);
-        if (act && q == 0) {
-          C.b[P] = s;
-          if (first_sweep) C.x[P] = om(l + 1) * s / C.ac[P];
-        }
-      });
-  }
-  // x_{l-1}[c] += d for the children c of row i of level l (d = alpha x_l[i])
-  __device__ __forceinline__ void scatter_children(const LevelDev<R> &L, R *__restrict__ xf, long i, R d, int q0,
-                                                   int step) {
-    const int c1 = L.rptr[i + 1];
-    for (int c = L.rptr[i] + q0; c < c1; c += 4 * step) {
-      int f[4];
-      R v[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) f[u] = c + u * step < c1 ? L.rlist[c + u * step] : -1;
-#pragma unroll
-      for (int u = 0; u < 4; u++) if (f[u] >= 0) v[u] = xf[f[u]];
-#pragma unroll
-      for (int u = 0; u < 4; u++) if (f[u] >= 0) xf[f[u]] = v[u] + d;
-    }
-  }
-  // the post-sweep of level l, then its prolongation into level l-1 (l >= 1)
-  // or the result into `out` (l = 0)
-  __device__ void smooth_scatter(int l, const double *__restrict__ in, double *__restrict__ out) {
-    const LevelDev<R> L = lev[l];
-    Scope sl = pc_scope(L);
-    enter(sl);
-    if (!sl.active()) return;
-    R *__restrict__ xf = l > 0 ? lev[l - 1].x : nullptr;
-    const R af = l > 0 ? al(l - 1) : (R)0.;
-    if (l == 0 || sl.nth() < 2L * L.n) {   // a thread per row, two rows per step
-      const long t0 = sl.tid0(), nt = sl.nth();
-      for (long i = t0; i < L.n; i += 2 * nt) {
-        const long i2 = i + nt;
-        const bool h2 = i2 < L.n;
-        R t1 = 0., t2 = 0.;
-        ell_acc2<6, false>(t1, t2, L.n, L.w, L.nbr, L.anb, i, i2, h2, [&](int k) { return L.x[k]; });
-        R xi = L.x[i], bi = l == 0 ? (R)in[i] : L.b[i];
-        R xn = xi + om(l) * (bi - L.ac[i] * xi - t1) / L.ac[i];
-        R xm = 0.;
-        if (h2) {
-          R xj = L.x[i2], bj = l == 0 ? (R)in[i2] : L.b[i2];
-          xm = xj + om(l) * (bj - L.ac[i2] * xj - t2) / L.ac[i2];
-        }
-        if (l == 0) {
-          out[i] = (double)xn;
-          if (h2) out[i2] = (double)xm;
-        } else if (gather_into(l)) {
-          L.r[i] = xn;
-          if (h2) L.r[i2] = xm;
-        } else {
-          scatter_children(L, xf, i, af * xn, 0, 1);
-          if (h2) scatter_children(L, xf, i2, af * xm, 0, 1);
-        }
-      }
-      return;
-    }
-    level_rows(sl, L.n, l, [&](auto gg, long i, bool act, int q) {
-      constexpr int G = decltype(gg)::value;
-      R t = 0.;
-      if (act) t = ell_part<G, G == 1 ? 8 : 4>(L.n, L.w, L.nbr, L.anb, i, q, [&](int k) { return L.x[k]; });
-      t = gsum<G>(t);
-      if (act) {
-        R xi = L.x[i], bi = L.b[i];
-        R xn = xi + om(l) * (bi - L.ac[i] * xi - t) / L.ac[i];
-        if (!gather_into(l)) scatter_children(L, xf, i, af * xn, q, G);
-        else if (q == 0) L.r[i] = xn;
-      }
-    });
-  }
-  // level 1's post-sweep leaves its result in its r, and level 0 gathers the
-  // correction through parent in a phase of its own (x_0 += alpha x_1[parent],
-  // the same sum the scatter forms): a coalesced pass over the fine rows
-  // instead of one read-modify-write per fine row in agglomerate order.  At
-  // 128^3 the extra grid barrier costs less than the scattered writes: the
-  // FP64 p' solve 2 % faster, and the FP32 one, which ran the unfused cycle
-  // before, 10 %.
-  __device__ __forceinline__ bool gather_into(int l) const { return l == 1 && lc >= 2; }
-  __device__ void prolong0() {
-    const LevelDev<R> L = lev[0];
-    const R *__restrict__ xc = lev[1].r;
-    Scope g;
-    g.grid = true;
-    enter(g);
-    const R a0 = al(0);
-    for (long i = g.tid0(); i < L.n; i += g.nth()) L.x[i] = L.x[i] + a0 * xc[L.parent[i]];
-  }
-  // the dense coarsest solve (CTA 0, warps on rows), scattered into level lc-1
-  __device__ void coarsest_scatter() {
-    Scope c0;
-    c0.grid = false;
-    enter(c0);
-    if (cta_id() != 0) return;
-    const LevelDev<R> Cc = lev[lc];
-    R *__restrict__ xf = lev[lc - 1].x;
-    const R af = al(lc - 1);
-    const int n = Cc.n, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int i = threadIdx.x >> 5; i < n; i += nw) {
-      double t = 0.;
-      for (int j = lane; j < n; j += 32) t += sinv[(long)i * n + j] * (double)Cc.b[j];
-      t = wsum(t);
-      t = __shfl_sync(0xffffffffu, t, 0);
-      scatter_children(Cc, xf, i, af * (R)t, lane, 32);
-    }
-  }
-  // ------------------------------------------------------------ Gauss-Seidel V-cycle
-  // One multicolour Gauss-Seidel pass over level l in place: the colours in
-  // order (forward) or reversed (backward); rows of one colour read only
-  // rows of other colours, so each colour is one phase of independent rows.
-  __device__ void gs_colours(int l, const double *__restrict__ in, R *__restrict__ x, bool backward) {
-    const LevelDev<R> L = lev[l];
-    Scope sc = pc_scope(L);
-    for (int cc = 0; cc < L.ncolors; cc++) {
-      const int c = backward ? L.ncolors - 1 - cc : cc;
-      enter(sc);
-      if (!sc.active()) continue;
-      const int r0 = L.color_ptr[c], r1 = L.color_ptr[c + 1];
-      for (long q = r0 + sc.tid0(); q < r1; q += sc.nth()) {
-        const int i = L.color_rows[q];
-        const R t = ell_acc<6, false>((R)0., L.n, L.w, L.nbr, L.anb, i, [&](int k) { return x[k]; });
-        const R bi = l == 0 ? (R)in[i] : L.b[i];
-        x[i] = (bi - t) / L.ac[i];
-      }
-    }
-  }
-  // The V-cycle with symmetric multicolour Gauss-Seidel smoothing on the
-  // levels below FS_PC_GS_LEVELS (a forward pass from zero before the
-  // restriction and, after the correction x += alpha x_c[parent], a backward
-  // pass) and the damped Jacobi sweeps of run() on the others; the coarsest
-  // level by the dense inverse.  Results stay in each level's x.  out =
-  // M^-1 in; callers have made `in` visible.
-  __device__ void run_gs(const double *__restrict__ in, double *__restrict__ out) {
-    Scope g;
-    g.grid = true;
-    const LevelDev<R> L0 = lev[0];
-    for (long i = g.tid0(); i < L0.n; i += g.nth()) L0.x[i] = (R)0.;
-    last.grid = true;
-    last.team = false;
-    gs_colours(0, in, L0.x, false);
-    for (int l = 0; l < lc; l++) {
-      const LevelDev<R> L = lev[l], C = lev[l + 1];
-      residual(l, in, L.x, L.r);
-      Scope scc = pc_scope(C);
-      enter(scc);
-      const bool gsc = l + 1 < FS_PC_GS_LEVELS;
-      const R omc = (gsc || l + 1 == lc) ? (R)0. : om(l + 1);   // Jacobi: the first sweep from zero
-      if (scc.active())
-        for (long P = scc.tid0(); P < C.n; P += scc.nth()) {
-          R s = 0.;
-          for (int c = C.rptr[P]; c < C.rptr[P + 1]; c++) s = s + L.r[C.rlist[c]];
-          C.b[P] = s;
-          C.x[P] = omc * s / C.ac[P];
-        }
-      if (l + 1 < lc && gsc) gs_colours(l + 1, in, C.x, false);
-    }
-    {
-      Scope c0;
-      c0.grid = false;
-      enter(c0);
-      if (cta_id() == 0) {
-        const LevelDev<R> Cc = lev[lc];
-        const int n = Cc.n, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-        for (int i = threadIdx.x >> 5; i < n; i += nw) {
-          double t = 0.;
-          for (int j = lane; j < n; j += 32) t += sinv[(long)i * n + j] * (double)Cc.b[j];
-          t = wsum(t);
-          if (lane == 0) Cc.x[i] = (R)t;
-        }
-      }
-    }
-    for (int l = lc - 1; l >= 0; l--) {
-      const LevelDev<R> L = lev[l];
-      const R *__restrict__ xc = lev[l + 1].x;
-      Scope sl = pc_scope(L);
-      enter(sl);
-      if (sl.active())
-        for (long i = sl.tid0(); i < L.n; i += sl.nth()) L.x[i] = L.x[i] + al(l) * xc[L.parent[i]];
-      if (l < FS_PC_GS_LEVELS) {
-        gs_colours(l, in, L.x, true);
-      } else {   // one damped Jacobi sweep in place: residual into t, then the update
-        residual(l, in, L.x, L.t);
-        enter(sl);
-        if (sl.active()) for (long i = sl.tid0(); i < L.n; i += sl.nth()) L.x[i] = L.x[i] + om(l) * L.t[i] / L.ac[i];
-      }
-    }
-    enter(g);
-    for (long i = g.tid0(); i < L0.n; i += g.nth()) out[i] = (double)L0.x[i];
-    enter(g);
-  }
-
-  __device__ void run_fused(const double *__restrict__ in, double *__restrict__ out) {
-    Scope g;
-    g.grid = true;
-    last.grid = true;
-    last.team = false;
-    synced = true;   // the caller's grid barrier stands for the first phase's
-    for (int l = 0; l < lc; l++) {
-      if (l < FS_PC_FUSE_DOWN) restrict_fused(l, in);
-      else restrict_plain(l, in);
-    }
-    coarsest_scatter();
-    for (int l = lc - 1; l >= 0; l--) {
-      if (l == 0 && gather_into(1)) prolong0();
-      smooth_scatter(l, in, out);
-    }
-    enter(g);
-  }
 };
 
 // rows i and i2 (when h2) of A x at once (ell_acc2)
@@ -718,19 +424,375 @@ __device__ __forceinline__ void row_ax2(const A &a, long i, long i2, bool h2, co
   ell_acc2<6, false>(t1, t2, a.N, a.W, a.cn, a.anb, i, i2, h2, [&](int k) { return x[k]; });
 }
 
+// ------------------------------------------------------------ V-cycle in one phase per level and leg
+// One damped-Jacobi pre- and post-sweep per level and a dense coarsest solve,
+// with the arithmetic and the order of every sum of PCycle::run():
+//   down  the residual of each row of level l and its sum over the aggregates
+//         in one phase: a CTA takes consecutive aggregates, whose rows are
+//         consecutive too (levels >= 1 are renumbered aggregate by aggregate,
+//         level 0 has a copy of the matrix in that order), so a block barrier
+//         stands between the residuals and their sums instead of a grid barrier;
+//   up    the post-sweep of a row, then its prolongation x += alpha x_row into
+//         the consecutive rows of its aggregate on the finer level; level 0
+//         forms x_0 + alpha x_1[parent] on the fly for a row and its neighbours.
+// A level costs two grid barriers a cycle where separate residual,
+// restriction, prolongation and sweep phases cost three to four, and the passes
+// over the level that went with them.  What bounds a phase on a small level is
+// the barrier (1.2 us) and its chain of dependent loads, on a large one DRAM.
+// Measured against the phases it replaces (p' solve, B200): 128^3 75.1 -> 60.0
+// ms for 92 iterations, 295k cells 38.5 -> 24.8 ms for 130, 124k cells 29.5 ->
+// 17.0 ms for 124.  Tried and slower: a warp per chunk of aggregates with the
+// residuals in its own shared array (a chain of six dependent loads per chunk:
+// level 0 of 128^3 72 us against 63, level 1 54 against 19).
+template <class R>
+__device__ __forceinline__ VcDev<R> &vstate() {
+  __shared__ VcDev<R> s;
+  return s;
+}
+
+// lanes per row of a level, from the threads that the cycle of PCycle gives it
+// (pc_scope, level_rows): it fixes the order of a row's sum
+__device__ __forceinline__ int vc_lanes(int n) {
+  const long nth = (long)blockDim.x * (n > FS_PC_TEAM_MAX ? cta_count() : n > FS_PC_SMALL ? team_size() : 1);
+  const long per = nth / (n > 0 ? n : 1);
+  return per < 2 ? 1 : per < 4 ? 2 : per < 8 ? 4 : 8;
+}
+
+// lanes per row and this CTA's aggregates of every level: consecutive ones
+// holding an equal share of the level's rows
+template <class R>
+__device__ __forceinline__ void vc_split() {
+  VcDev<R> &V = vstate<R>();
+  const int t = threadIdx.x;
+  if (t <= V.lc) V.G[t] = vc_lanes(V.L[t].n);
+  if (t < 2 * V.lc) {
+    const int l = t >> 1, nc = V.L[l + 1].n;
+    const long want = (long)V.L[l].n * (cta_id() + (t & 1)) / cta_count();
+    int lo = 0, hi = nc;   // first aggregate whose rows start at or after `want`
+    while (lo < hi) {
+      const int m = (lo + hi) >> 1;
+      if (V.L[l].kp[m] >= want) hi = m; else lo = m + 1;
+    }
+    if (t & 1) { V.p1[l] = lo; V.e1[l] = V.L[l].kp[lo]; }
+    else { V.p0[l] = lo; V.e0[l] = V.L[l].kp[lo]; }
+  }
+}
+
+// the warps that work on a phase: the grid's, or CTA 0's on small levels
+struct Warps {
+  int w0, nw;
+  // with items for every warp a CTA takes neighbouring ones; with fewer they
+  // are spread over the CTAs
+  __device__ Warps(bool grid, int items) {
+    const int wid = threadIdx.x >> 5, wpc = blockDim.x >> 5;
+    nw = grid ? wpc * cta_count() : wpc;
+    w0 = !grid ? wid : items >= nw ? cta_id() * wpc + wid : wid * cta_count() + cta_id();
+  }
+};
+
+template <class R>
+__device__ __forceinline__ R lanes_sum(R v, int G) {
+  for (int o = G >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// residuals of level l summed into the rows of level l+1: b, and the first
+// sweep from zero x = omega b / ac unless that is the coarsest.  A CTA takes the
+// aggregates [p0, p1) and with them the consecutive rows [e0, e1): residuals
+// first (G lanes a row, two rows in flight), kept in shared memory or, when they
+// do not fit, in the level's r, then after a block barrier the sums.  FINE:
+// level 0 with b = in and x = x0 in mesh order (row a is cell cells[a]).
+template <class R, bool FINE>
+__device__ __forceinline__ void vc_down(const VcDev<R> &V, int l, int Gc, bool sweep, const double *in, const R *x0) {
+  __shared__ R sh[FS_VC_ROWS];
+  const VcLevel<R> &F = V.L[l], &C = V.L[l + 1];
+  const int G = FINE ? 1 : V.G[l];
+  const int e0 = V.e0[l], e1 = V.e1[l], n = F.n, W0 = F.w;
+  R *rs = e1 - e0 <= FS_VC_ROWS ? sh : F.r + e0;
+  const int32_t *__restrict__ sb = F.sb, *__restrict__ col = F.col, *__restrict__ cells = F.cells;
+  const R *__restrict__ val = F.val, *__restrict__ ac = F.ac;
+  const R *x = FINE ? x0 : F.x, *b = F.b;
+  const int q = (threadIdx.x & 31) % G, rpp = blockDim.x / G, rw = (threadIdx.x & 31) / G;
+  constexpr int U = FINE ? 6 : 4;
+  for (int a = e0 + (int)(threadIdx.x & ~31u) / G; a < e1; a += 2 * rpp) {
+    const int a0 = a + rw, a1 = a0 + rpp;
+    const bool h0 = a0 < e1, h1 = a1 < e1;
+    long p0, p1;
+    int w0, w1;
+    const int st = FINE ? n : 32;
+    if (FINE) {
+      p0 = a0; p1 = a1;
+      w0 = h0 ? W0 : 0; w1 = h1 ? W0 : 0;
+    } else {
+      const int s0 = h0 ? __ldg(sb + (a0 >> 5)) : 0, s1 = h1 ? __ldg(sb + (a1 >> 5)) : 0;
+      w0 = h0 ? __ldg(sb + (a0 >> 5) + 1) - s0 : 0;
+      w1 = h1 ? __ldg(sb + (a1 >> 5) + 1) - s1 : 0;
+      p0 = (long)s0 * 32 + (a0 & 31);
+      p1 = (long)s1 * 32 + (a1 & 31);
+    }
+    const int i0 = FINE ? (h0 ? __ldg(cells + a0) : 0) : a0, i1 = FINE ? (h1 ? __ldg(cells + a1) : 0) : a1;
+    R t0 = (R)0, t1 = (R)0;
+    const int wm = w0 > w1 ? w0 : w1;
+    for (int j0 = q; j0 < wm; j0 += U * G) {
+      int k0[U], k1[U];
+      R c0[U], c1[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int j = j0 + u * G;
+        const bool g0 = j < w0, g1 = j < w1;
+        k0[u] = g0 ? __ldg(col + p0 + (long)j * st) : -1;
+        c0[u] = g0 ? __ldg(val + p0 + (long)j * st) : (R)0;
+        k1[u] = g1 ? __ldg(col + p1 + (long)j * st) : -1;
+        c1[u] = g1 ? __ldg(val + p1 + (long)j * st) : (R)0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (k0[u] >= 0) t0 = t0 + c0[u] * x[k0[u]];
+        if (k1[u] >= 0) t1 = t1 + c1[u] * x[k1[u]];
+      }
+    }
+    if (G > 1) { t0 = lanes_sum(t0, G); t1 = lanes_sum(t1, G); }
+    if (q == 0) {
+      if (h0) rs[a0 - e0] = (FINE ? (R)in[i0] : b[i0]) - __ldg(ac + a0) * x[i0] - t0;
+      if (h1) rs[a1 - e0] = (FINE ? (R)in[i1] : b[i1]) - __ldg(ac + a1) * x[i1] - t1;
+    }
+  }
+  __syncthreads();
+  const int32_t *__restrict__ kp = F.kp;
+  const int P1 = V.p1[l], qc = (threadIdx.x & 31) % Gc;
+  for (int Pw = V.p0[l] + (int)(threadIdx.x & ~31u) / Gc; Pw < P1; Pw += blockDim.x / Gc) {
+    const int P = Pw + (threadIdx.x & 31) / Gc;
+    const bool h = P < P1;
+    const int c0 = h ? __ldg(kp + P) - e0 + qc : 0, c1 = h ? __ldg(kp + P + 1) - e0 : 0;
+    const R d = h && sweep ? __ldg(C.ac + P) : (R)1;
+    R s = (R)0;
+    for (int c = c0; c < c1; c += 4 * Gc) {
+      R v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[u] = c + u * Gc < c1 ? rs[c + u * Gc] : (R)0;
+#pragma unroll
+      for (int u = 0; u < 4; u++) if (c + u * Gc < c1) s = s + v[u];
+    }
+    if (Gc > 1) s = lanes_sum(s, Gc);
+    if (h && qc == 0) {
+      C.b[P] = s;
+      if (sweep) C.x[P] = (R)FS_MG_OMEGA * s / d;
+    }
+  }
+}
+
+// post-sweep of level L's rows, then the prolongation into the finer level F's
+// x (last: level 1, whose result goes to x1)
+template <class R>
+__device__ __forceinline__ void vc_up(const VcLevel<R> &L, const VcLevel<R> &F, int G, bool last, R *x1, const Warps w) {
+  const int lane = threadIdx.x & 31, q = lane % G, rpw = 32 / G, n = L.n;
+  const int32_t *__restrict__ sb = L.sb, *__restrict__ col = L.col, *__restrict__ kp = F.kp;
+  const R *__restrict__ val = L.val, *__restrict__ ac = L.ac;
+  const R *x = L.x, *b = L.b;
+  R *xf = F.x;
+  constexpr int U = 8;
+  for (int s = w.w0; s * rpw < n; s += w.nw) {
+    const int i = s * rpw + lane / G;
+    const bool act = i < n;
+    const int s0 = act ? __ldg(sb + (i >> 5)) : 0, wd = act ? __ldg(sb + (i >> 5) + 1) - s0 : 0;
+    const long p = (long)s0 * 32 + (i & 31);
+    const R xi = act ? x[i] : (R)0, bi = act ? b[i] : (R)0, d = act ? __ldg(ac + i) : (R)1;
+    int c = 0, c1 = 0;
+    R f0 = (R)0, f1 = (R)0;
+    if (!last && act) {
+      c = __ldg(kp + i) + q;
+      c1 = __ldg(kp + i + 1);
+      if (c < c1) f0 = xf[c];
+      if (c + G < c1) f1 = xf[c + G];
+    }
+    R t = (R)0;
+    for (int j0 = q; j0 < wd; j0 += U * G) {
+      int k[U];
+      R v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int j = j0 + u * G;
+        k[u] = j < wd ? __ldg(col + p + (long)j * 32) : -1;
+        v[u] = j < wd ? __ldg(val + p + (long)j * 32) : (R)0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) if (k[u] >= 0) t = t + v[u] * x[k[u]];
+    }
+    if (G > 1) t = lanes_sum(t, G);
+    if (!act) continue;
+    const R xn = xi + (R)FS_MG_OMEGA * (bi - d * xi - t) / d;
+    if (last) {
+      if (q == 0) x1[i] = xn;
+    } else {
+      const R add = (R)FS_MG_ALPHA * xn;
+      if (c < c1) xf[c] = f0 + add;
+      if (c + G < c1) xf[c + G] = f1 + add;
+      for (c += 2 * G; c < c1; c += G) xf[c] = xf[c] + add;
+    }
+  }
+}
+
+// the coarsest level by its dense inverse (a warp per row), prolonged into the
+// next finer level, or left in x1 when that is level 0
+template <class R>
+__device__ __forceinline__ void vc_dense(const VcLevel<R> &C, const VcLevel<R> &F, const double *__restrict__ sinv,
+                                         bool last, R *x1, const Warps w) {
+  const int lane = threadIdx.x & 31, n = C.n;
+  const R *b = C.b;
+  R *xf = F.x;
+  for (int i = w.w0; i < n; i += w.nw) {
+    double m[5], y[5];   // n <= FS_MG_DIRECT = 160
+#pragma unroll
+    for (int u = 0; u < 5; u++) {
+      const int j = lane + 32 * u;
+      m[u] = j < n ? __ldg(sinv + (long)i * n + j) : 0.;
+      y[u] = j < n ? (double)b[j] : 0.;
+    }
+    double t = 0.;
+#pragma unroll
+    for (int u = 0; u < 5; u++) if (lane + 32 * u < n) t += m[u] * y[u];
+    t = wsum(t);
+    const R xn = (R)__shfl_sync(0xffffffffu, t, 0);
+    if (last) {
+      if (lane == 0) x1[i] = xn;
+    } else {
+      const R add = (R)FS_MG_ALPHA * xn;
+      for (int c = __ldg(F.kp + i) + lane; c < __ldg(F.kp + i + 1); c += 32) xf[c] = xf[c] + add;
+    }
+  }
+}
+
+// levels 1 and below: from b_1, x_1 to the corrected x_1 in V.x1; ends with a
+// grid barrier.  GS: the restriction sums a coarse row's children in sequence.
+template <class R, bool GS>
+__device__ __forceinline__ void vcycle_coarse(Sync &S) {
+  const VcDev<R> &V = vstate<R>();
+  const int lc = V.lc;
+  for (int l = 1; l < lc; l++) {
+    vc_down<R, false>(V, l, GS ? 1 : V.G[l + 1], l + 1 < lc, nullptr, nullptr);
+    S.all();
+  }
+  vc_dense<R>(V.L[lc], V.L[lc - 1], V.sinv, lc == 1, V.x1, Warps(true, V.L[lc].n));
+  S.all();
+  for (int l = lc - 1; l >= 1; l--) {
+    const int rpw = 32 / V.G[l];
+    vc_up<R>(V.L[l], V.L[l - 1], V.G[l], l == 1, V.x1, Warps(true, (V.L[l].n + rpw - 1) / rpw));
+    S.all();
+  }
+}
+
+// out = M^-1 in.  The caller has set x_0 = omega0 in / ac_0 and passed a grid
+// barrier; ends with one.
+template <class R>
+__device__ __forceinline__ void vcycle(Sync &S, const double *in, double *out) {
+  const VcDev<R> &V = vstate<R>();
+  const LevelDev<R> &L = V.L0;
+  vc_down<R, true>(V, 0, V.G[1], V.lc > 1, in, L.x);
+  S.all();
+  vcycle_coarse<R, false>(S);
+  const long t0 = (long)cta_id() * blockDim.x + threadIdx.x, nt = (long)cta_count() * blockDim.x;
+  const int n = L.n, w = L.w;
+  const int32_t *__restrict__ nbr = L.nbr, *__restrict__ par = V.par0;
+  const R *__restrict__ anb = L.anb, *__restrict__ ac = L.ac;
+  const R *x0 = L.x, *x1 = V.x1;
+  const R al0 = (R)FS_MG_ALPHA0, om0 = (R)FS_MG_OMEGA0;
+  for (long i = t0; i < n; i += 2 * nt) {
+    const long i2 = i + nt;
+    const bool h2 = i2 < n;
+    R t1 = (R)0, t2 = (R)0;
+    for (int j0 = 0; j0 < w; j0 += 3) {
+      int k1[3], k2[3], q1[3], q2[3];
+      R c1[3], c2[3], y1[3], y2[3];
+#pragma unroll
+      for (int u = 0; u < 3; u++) {
+        const bool h = j0 + u < w;
+        k1[u] = h ? __ldg(nbr + (long)(j0 + u) * n + i) : -1;
+        k2[u] = h && h2 ? __ldg(nbr + (long)(j0 + u) * n + i2) : -1;
+        c1[u] = h ? anb[(long)(j0 + u) * n + i] : (R)0;
+        c2[u] = h && h2 ? anb[(long)(j0 + u) * n + i2] : (R)0;
+      }
+#pragma unroll
+      for (int u = 0; u < 3; u++) {
+        q1[u] = k1[u] >= 0 ? __ldg(par + k1[u]) : 0;
+        q2[u] = k2[u] >= 0 ? __ldg(par + k2[u]) : 0;
+        y1[u] = k1[u] >= 0 ? x0[k1[u]] : (R)0;
+        y2[u] = k2[u] >= 0 ? x0[k2[u]] : (R)0;
+      }
+#pragma unroll
+      for (int u = 0; u < 3; u++) {
+        if (k1[u] >= 0) t1 = t1 + c1[u] * (y1[u] + al0 * x1[q1[u]]);
+        if (k2[u] >= 0) t2 = t2 + c2[u] * (y2[u] + al0 * x1[q2[u]]);
+      }
+    }
+    {
+      const R aci = ac[i], xi = x0[i] + al0 * x1[__ldg(par + i)];
+      out[i] = (double)(xi + om0 * ((R)in[i] - aci * xi - t1) / aci);
+    }
+    if (h2) {
+      const R aci = ac[i2], xi = x0[i2] + al0 * x1[__ldg(par + i2)];
+      out[i2] = (double)(xi + om0 * ((R)in[i2] - aci * xi - t2) / aci);
+    }
+  }
+  S.all();
+}
+
+// One multicolour Gauss-Seidel pass over level 0 in place: the colours in
+// order (forward) or reversed (backward); rows of one colour read only rows of
+// other colours, so each colour is one phase of independent rows.
+template <class R>
+__device__ __forceinline__ void gs_colours(Sync &S, const LevelDev<R> &L, const double *in, R *x, bool backward) {
+  const long t0 = (long)cta_id() * blockDim.x + threadIdx.x, nt = (long)cta_count() * blockDim.x;
+  for (int cc = 0; cc < L.ncolors; cc++) {
+    const int c = backward ? L.ncolors - 1 - cc : cc;
+    S.all();
+    const int r0 = L.color_ptr[c], r1 = L.color_ptr[c + 1];
+    for (long q = r0 + t0; q < r1; q += nt) {
+      const int i = L.color_rows[q];
+      const R t = ell_acc<6, false>((R)0., L.n, L.w, L.nbr, L.anb, i, [&](int k) { return x[k]; });
+      x[i] = ((R)in[i] - t) / L.ac[i];
+    }
+  }
+}
+
+// The V-cycle with symmetric multicolour Gauss-Seidel smoothing on level 0 (a
+// forward pass from zero before the restriction and, after the correction
+// x += alpha x_1[parent], a backward pass) and damped Jacobi on the others.
+// out = M^-1 in; callers have made `in` visible.
+template <class R>
+__device__ __forceinline__ void vcycle_gs(Sync &S, const double *in, double *out) {
+  const VcDev<R> &V = vstate<R>();
+  const LevelDev<R> &L = V.L0;
+  const long t0 = (long)cta_id() * blockDim.x + threadIdx.x, nt = (long)cta_count() * blockDim.x;
+  R *x = L.x;
+  for (long i = t0; i < L.n; i += nt) x[i] = (R)0.;
+  gs_colours(S, L, in, x, false);
+  S.all();
+  vc_down<R, true>(V, 0, 1, V.lc > 1, in, x);
+  S.all();
+  vcycle_coarse<R, true>(S);
+  const R al0 = (R)FS_MG_ALPHA0;
+  for (long i = t0; i < L.n; i += nt) x[i] = x[i] + al0 * V.x1[V.par0[i]];
+  gs_colours(S, L, in, x, true);
+  S.all();
+  for (long i = t0; i < L.n; i += nt) out[i] = (double)x[i];
+  S.all();
+}
+
 // apply the preconditioner: out (FP64) = M^-1 in (FP64), via the R-precision
-// V-cycle; `fused`: the caller has set x_0 = omega0 in / ac_0 (run_fused)
-// MODE: 0 the V-cycle of run(), 1 run_fused(), 2 run_gs()
+// V-cycle.  MODE: 0 the V-cycle of PCycle::run(), 1 vcycle() (the caller has
+// set x_0 = omega0 in / ac_0), 2 vcycle_gs()
 template <class R, int MODE>
-__device__ void apply_prec(Sync &S, const AmgKArgs<R> &a, const double *in, double *out, unsigned &gen) {
-  Scope all;
-  all.grid = true;
-  PCycle<R> C{S, a.lev, a.lc, a.direct != 0, a.sinv, a.pre, a.post, 20, (R)FS_MG_OMEGA, (R)FS_MG_ALPHA, all,
-               (R)FS_MG_OMEGA0, (R)FS_MG_ALPHA0, a.teambar, a.status, gen, a.team_extra, false};
-  if (MODE == 1) C.run_fused(in, out);
-  else if (MODE == 2) C.run_gs(in, out);
-  else C.run(in, out);
-  gen = C.gen;
+__device__ __forceinline__ void apply_prec(Sync &S, const AmgKArgs<R> &a, const double *in, double *out, unsigned &gen) {
+  if (MODE == 1) vcycle<R>(S, in, out);
+  else if (MODE == 2) vcycle_gs<R>(S, in, out);
+  else {
+    Scope all;
+    all.grid = true;
+    PCycle<R> C{S, a.lev, a.lc, a.direct != 0, a.sinv, a.pre, a.post, 20, (R)FS_MG_OMEGA, (R)FS_MG_ALPHA, all,
+                (R)FS_MG_OMEGA0, (R)FS_MG_ALPHA0, a.teambar, a.status, gen, a.team_extra};
+    C.run(in, out);
+    gen = C.gen;
+  }
 }
 
 // mean of the right-hand side of a pure-Neumann system (every row sums to
@@ -762,7 +824,7 @@ __device__ double rhs_mean(Sync &S, const AmgKArgs<R> &a) {
 template <class R, int NX>
 __device__ __forceinline__ void guess_fit_body(const AmgKArgs<R> a) {
   constexpr int NG = NX * (NX + 1) / 2, K = NG + NX + 1;
-  Sync S(a.part);
+  Sync S(a.part, a.gridbar + FS_GRIDBAR_FIT, a.status, a.team_extra);
   const double bmean = rhs_mean(S, a);
   double c[NX];
   bool fell_back;
@@ -869,8 +931,8 @@ __device__ __forceinline__ void guess_fit_body(const AmgKArgs<R> a) {
 
 
 // right-preconditioned BiCGSTAB (van der Vorst 1992) with a multigrid V-cycle:
-// MODE 0 run(), 2 run_gs() (multicolour Gauss-Seidel smoothing), 1 the fused
-// V-cycle (one pre- and one post-sweep, dense coarsest level), whose first
+// MODE 0 PCycle::run(), 2 vcycle_gs() (multicolour Gauss-Seidel smoothing), 1
+// vcycle() (one pre- and one post-sweep, dense coarsest level), whose first
 // sweep from zero, x_0 = omega0 in / ac_0, rides on the loops that form p and s.
 // Four grid synchronisations per iteration besides the V-cycles': the sums
 // after v = A y and after s, the sums after t = A z, and the barrier after one
@@ -885,7 +947,14 @@ __device__ __forceinline__ void guess_fit_body(const AmgKArgs<R> a) {
 // continues with p formed in a separate pass.
 template <class R, int MODE>
 __device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> a) {
-  Sync S(a.part);
+  if (MODE != 0) {   // the operators' descriptors, read in every phase
+    const int32_t *src = (const int32_t *)a.vc;
+    int32_t *dst = (int32_t *)&vstate<R>();
+    for (int q = threadIdx.x; q < (int)(sizeof(VcDev<R>) / 4); q += blockDim.x) dst[q] = src[q];
+    __syncthreads();
+    vc_split<R>();
+  }
+  Sync S(a.part, a.gridbar, a.status, a.team_extra);
   unsigned gen = 0;   // team-barrier generation (the counters are zeroed before the launch)
   const int N = a.N;
   Scope g; g.grid = true;
@@ -1031,4 +1100,3 @@ __device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> a) {
   for (long i = t0; i < N; i += nt) a.dphi[i] = a.x[i];
   if (cta_id() == 0 && threadIdx.x == 0) { *a.iters = k; a.diag[0] = resn; a.diag[1] = normb; }
 }
-

@@ -70,11 +70,32 @@ struct LevelDev {
   R *b, *x, *r, *t;
   const int32_t *parent;        // this level -> next coarser (nullptr on the coarsest)
   const int32_t *rptr, *rlist;  // restriction into this level: finer rows per coarse row, ascending
-  // warp chunks of this level's rows for the fused restriction into it:
-  // chunk k is rows [chunk[k], chunk[k+1]), at most 32 rows and, unless one
-  // row alone has more, at most 64 finer rows (children) in all
-  const int32_t *chunk;
-  int nchunk;
+};
+
+// One level of the V-cycle (fs_amg_core.cuh).  Rows of levels >= 1 are numbered
+// aggregate by aggregate, so the rows of coarse row P are [kp[P], kp[P+1]); row
+// a of level 0 is cell cells[a].  Off-diagonals: levels >= 1 in slices of 32
+// rows, slot j of row a at (sb[a/32] + j) * 32 + a % 32 (a slice as wide as its
+// widest row, padded with value 0 and the row itself); level 0 slot j at j * n
+// + a, columns in mesh order, unused slots -1.
+template <class R>
+struct VcLevel {
+  int n, w;
+  const int32_t *sb, *col, *cells;
+  const R *val, *ac;
+  const int32_t *kp;
+  R *b, *x, *r;
+};
+template <class R>
+struct VcDev {
+  int lc;
+  // set by each CTA of the kernel: lanes per row, its aggregates and their rows
+  int G[FS_MG_MAXLEV], p0[FS_MG_MAXLEV], p1[FS_MG_MAXLEV], e0[FS_MG_MAXLEV], e1[FS_MG_MAXLEV];
+  VcLevel<R> L[FS_MG_MAXLEV];
+  R *x1;                 // result of level 1
+  const double *sinv;
+  LevelDev<R> L0;        // level 0 in mesh order
+  const int32_t *par0;   // level-1 row of each cell
 };
 
 template <class R>
@@ -84,6 +105,7 @@ struct AmgKArgs {
   const double *ac, *anb, *bc;
   double *x, *r, *r0, *p, *v, *s, *t, *y, *z, *dphi;
   const LevelDev<R> *lev;
+  const VcDev<R> *vc;
   int lc, direct, pre, post, maxit;
   const double *sinv;
   double tol;
@@ -94,13 +116,35 @@ struct AmgKArgs {
   int nx;             // vectors in xs (0: zero start)
   int32_t *fit;       // [0]: k_guess_fit found a guess (device)
   int32_t *nncnt;     // [fallbacks, uses] of the initial guess, or nullptr
-  unsigned *teambar;  // team barrier words of the V-cycle (zeroed before the launch)
+  unsigned *gridbar;  // grid barrier counts: the solve's, then (FS_GRIDBAR_FIT) the guess fit's; zero at launch
+  unsigned *teambar;  // team barrier words of PCycle (zeroed before the launch)
   int32_t *status;    // [0] team-barrier timeout flag
   int team_extra;     // fs_test_wait_timeout
 };
 
+// one array of the k_mg_layout launch: dst[q] = src[map[q]], 0 where map is -1
+struct LayoutSeg {
+  int block0, n;
+  const int32_t *map;
+  const double *src;
+  double *d64;
+  float *d32;
+};
+
 struct fs_mg_dev {
   int nlev = 0;
+  // V-cycle layout (mg_vc_build): maps and index arrays, values per precision
+  bool vc_map = false, vc_ready[2] = {false, false};
+  std::vector<int32_t> h_nnb[FS_MG_MAXLEV], h_nbr[FS_MG_MAXLEV];   // coarse connectivity until then
+  int32_t *vsb[FS_MG_MAXLEV] = {}, *vcol[FS_MG_MAXLEV] = {}, *vmap[FS_MG_MAXLEV] = {}, *vrow[FS_MG_MAXLEV] = {};
+  int32_t *vkp[FS_MG_MAXLEV] = {}, *par0 = nullptr;
+  int vnpos[FS_MG_MAXLEV] = {};
+  void *vval[2][FS_MG_MAXLEV] = {}, *vac[2][FS_MG_MAXLEV] = {}, *vb[2][FS_MG_MAXLEV] = {}, *vx[2][FS_MG_MAXLEV] = {};
+  VcDev<double> *vc64 = nullptr;
+  VcDev<float> *vc32 = nullptr;
+  LayoutSeg *seg[2] = {nullptr, nullptr};   // k_mg_layout tables in FP64, FP32; level 0 first
+  int nseg = 0, seg_blocks = 0, nseg0 = 0, seg0_blocks = 0;
+  unsigned *gridbar = nullptr;
   int n[FS_MG_MAXLEV] = {}, w[FS_MG_MAXLEV] = {}, ncol[FS_MG_MAXLEV] = {};
   std::vector<int32_t> h_parent[FS_MG_MAXLEV];
   // device
@@ -108,8 +152,6 @@ struct fs_mg_dev {
   int32_t *cptr[FS_MG_MAXLEV] = {}, *clist[FS_MG_MAXLEV] = {}, *cmap[FS_MG_MAXLEV] = {};
   int32_t *rptr[FS_MG_MAXLEV] = {}, *rlist[FS_MG_MAXLEV] = {};
   int32_t *colors[FS_MG_MAXLEV] = {};   // rows by colour, then ncol+1 offsets
-  int32_t *chunk[FS_MG_MAXLEV] = {};    // warp chunks of coarse rows (fused restriction)
-  int nchunk[FS_MG_MAXLEV] = {};
   double *ac[FS_MG_MAXLEV] = {}, *anb[FS_MG_MAXLEV] = {}, *b[FS_MG_MAXLEV] = {}, *x[FS_MG_MAXLEV] = {}, *r[FS_MG_MAXLEV] = {};
   double *t[FS_MG_MAXLEV] = {};
   float *acf[FS_MG_MAXLEV] = {}, *anbf[FS_MG_MAXLEV] = {}, *bf[FS_MG_MAXLEV] = {}, *xf[FS_MG_MAXLEV] = {}, *rf[FS_MG_MAXLEV] = {};
@@ -169,13 +211,10 @@ __device__ double bsum(double v) {
 #ifndef FS_PC_TEAM_MAX
 #define FS_PC_TEAM_MAX 4096   // levels up to this many rows run on the CTA team
 #endif
-#define FS_PC_SPIN_LIMIT (1L << 20)   // polls of a team barrier before it reports a timeout
-#ifndef FS_PC_GS_LEVELS
-#define FS_PC_GS_LEVELS 1     // amg32gs_bicgs: Gauss-Seidel on the levels below this one, Jacobi above
-#endif
-#ifndef FS_PC_FUSE_DOWN
-#define FS_PC_FUSE_DOWN 0     // restrictions from levels below this one form the residual on the fly
-#endif
+#define FS_PC_SPIN_LIMIT (1L << 20)   // polls of a barrier before it reports a timeout
+#define FS_VC_ROWS 2048        // residuals of a down leg that a CTA keeps in shared memory
+#define FS_GRIDBAR_FIT 32     // word of the guess fit's barrier count (another cache line)
+#define FS_GRIDBAR_WORDS 64
 
 // the same Krylov/V-cycle code for one system on the whole grid (g1) and for
 // groups of CTAs that each solve their own system (gb)
@@ -350,11 +389,13 @@ struct MgSolveArgs {
   double rrf; const double *ires;
   double *part;
   int32_t *iters;
+  unsigned *gridbar;
+  int32_t *status;
 };
 
 // AlgebraicMultigrid cycle loop (AlgebraicMultiGridMainRoutine.for:330-345)
 __global__ void __launch_bounds__(FS_COOP_BLOCK) k_mg_solve(MgSolveArgs a) {
-  Sync S(a.part);
+  Sync S(a.part, a.gridbar, a.status, 0);
   // dphiMG = 0 on every level
   for (int l = 0; l < a.nlev; l++) {
     Scope sc; sc.grid = true;
@@ -390,23 +431,19 @@ __global__ void __launch_bounds__(FS_COOP_BLOCK, FS_AMG_MINB) k_amg_bicgstab(Amg
 }
 
 // the same solve for n systems at once (the p' solves of an ensemble, one
-// cooperative launch): CTAs [start[q], start[q+1]) solve system q with their
-// own bounded barriers (gbar[2q..2q+1], zero at launch), so systems of uneven
-// size share the GPU instead of each holding all of it in turn
+// cooperative launch): CTAs [start[q], start[q+1]) solve system q behind their
+// own bounded barrier, so systems of uneven size share the GPU instead of each
+// holding all of it in turn
 template <class R, int MODE>
 __global__ void __launch_bounds__(FS_COOP_BLOCK, FS_AMG_MINB)
-    k_amg_bicgstab_batch(const AmgKArgs<R> *__restrict__ as, const int32_t *__restrict__ start, int n,
-                         unsigned *gbar) {
-  gb::GroupState &G = gb::gstate();
+    k_amg_bicgstab_batch(const AmgKArgs<R> *__restrict__ as, const int32_t *__restrict__ start, int n) {
+  gb::GridState &G = gb::gstate();
   if (threadIdx.x == 0) {
     int q = 0;
     while (q + 1 < n && (int)blockIdx.x >= start[q + 1]) q++;
     G.q = q;
     G.cta = (int)blockIdx.x - start[q];
     G.ncta = start[q + 1] - start[q];
-    G.gen = 0;
-    G.bar = gbar + 2 * q;
-    G.status = as[q].status;
   }
   __syncthreads();
   const AmgKArgs<R> a = as[G.q];
@@ -417,17 +454,14 @@ __global__ void __launch_bounds__(FS_COOP_BLOCK, FS_AMG_MINB)
 // whose system has no basis vectors does nothing)
 template <class R, int NX>
 __global__ void __launch_bounds__(FS_COOP_BLOCK, 1)
-    k_guess_fit_batch(const AmgKArgs<R> *__restrict__ as, const int32_t *__restrict__ start, int n, unsigned *gbar) {
-  gb::GroupState &G = gb::gstate();
+    k_guess_fit_batch(const AmgKArgs<R> *__restrict__ as, const int32_t *__restrict__ start, int n) {
+  gb::GridState &G = gb::gstate();
   if (threadIdx.x == 0) {
     int q = 0;
     while (q + 1 < n && (int)blockIdx.x >= start[q + 1]) q++;
     G.q = q;
     G.cta = (int)blockIdx.x - start[q];
     G.ncta = start[q + 1] - start[q];
-    G.gen = 0;
-    G.bar = gbar + 2 * q;
-    G.status = as[q].status;
   }
   __syncthreads();
   const AmgKArgs<R> a = as[G.q];
@@ -591,6 +625,19 @@ __global__ void __launch_bounds__(1024) k_mg_dense_inverse(int n, const int32_t 
     for (int i = tid; i < n; i += nt) A[(long)i * n + n - 1] = 0.;
   __syncthreads();
   for (int q = tid; q < n * n; q += nt) sinv[q] = A[q];
+}
+
+// the levels' matrices into the V-cycle's layout and precision
+__global__ void k_mg_layout(const LayoutSeg *__restrict__ segs, int nseg) {
+  int k = 0;
+  while (k + 1 < nseg && (int)blockIdx.x >= segs[k + 1].block0) k++;
+  const LayoutSeg g = segs[k];
+  const int q = ((int)blockIdx.x - g.block0) * blockDim.x + threadIdx.x;
+  if (q >= g.n) return;
+  const int m = g.map[q];
+  const double v = m >= 0 ? g.src[m] : 0.;
+  if (g.d64) g.d64[q] = v;
+  else g.d32[q] = (float)v;
 }
 
 }  // namespace
@@ -768,17 +815,6 @@ int fs_mg_build(fs_ctx *ctx) {
       for (int i = 0; i < h.n; i++) rlist[pos[M->h_parent[q][i]]++] = i;
       if ((rc = upv(ctx, &M->rptr[q + 1], rptr))) return rc;
       if ((rc = upv(ctx, &M->rlist[q + 1], rlist))) return rc;
-      // warp chunks of the coarse rows: consecutive rows, <= 32 of them and
-      // <= 64 children in all (a row with more children is a chunk alone)
-      std::vector<int32_t> ck(1, 0);
-      for (int P = 0, rows = 0, kids = 0; P < c.n; P++) {
-        const int k = rptr[P + 1] - rptr[P];
-        if (rows > 0 && (rows == 32 || kids + k > 64)) { ck.push_back(P); rows = 0; kids = 0; }
-        rows++; kids += k;
-      }
-      ck.push_back(c.n);
-      M->nchunk[q + 1] = (int)ck.size() - 1;
-      if ((rc = upv(ctx, &M->chunk[q + 1], ck))) return rc;
     }
     size_t n = h.n, nw = (size_t)h.w * h.n;
     if (q == 0) { M->ac[0] = ctx->ac; M->anb[0] = ctx->anb; }
@@ -806,14 +842,12 @@ int fs_mg_build(fs_ctx *ctx) {
     d.ac = M->ac[q]; d.anb = M->anb[q]; d.b = M->b[q]; d.x = M->x[q]; d.r = M->r[q]; d.t = M->t[q];
     d.parent = (q + 1 < M->nlev) ? M->parent[q] : nullptr;
     d.rptr = M->rptr[q]; d.rlist = M->rlist[q];
-    d.chunk = M->chunk[q]; d.nchunk = M->nchunk[q];
     L64[q] = d;
     LevelDev<float> e{};
     e.n = d.n; e.w = d.w; e.ncolors = d.ncolors; e.ncf = d.ncf; e.nbr = d.nbr; e.color_rows = d.color_rows;
     e.color_ptr = d.color_ptr; e.ac = M->acf[q]; e.anb = M->anbf[q]; e.b = M->bf[q]; e.x = M->xf[q]; e.r = M->rf[q];
     e.t = M->tf[q];
     e.parent = d.parent; e.rptr = d.rptr; e.rlist = d.rlist;
-    e.chunk = d.chunk; e.nchunk = d.nchunk;
     L32[q] = e;
   }
   FS_CK(cudaMalloc(&M->lev64, sizeof(LevelDev<double>) * M->nlev));
@@ -821,6 +855,8 @@ int fs_mg_build(fs_ctx *ctx) {
   FS_CK(cudaMalloc(&M->lev32, sizeof(LevelDev<float>) * M->nlev));
   FS_CK(cudaMemcpy(M->lev32, L32.data(), sizeof(LevelDev<float>) * M->nlev, cudaMemcpyHostToDevice));
   FS_CK(cudaMalloc(&M->red, sizeof(double) * (6 + FS_SUMK + 9) * FS_RED_BLOCKS));
+  FS_CK(cudaMalloc(&M->gridbar, sizeof(unsigned) * FS_GRIDBAR_WORDS));
+  for (int q = 1; q < M->nlev; q++) { M->h_nnb[q] = std::move(H[q].nnb); M->h_nbr[q] = std::move(H[q].nbr); }
   // preconditioner: stop at the first level small enough for the dense inverse
   M->lc = M->nlev - 1;
   for (int q = 0; q < M->nlev; q++)
@@ -853,11 +889,18 @@ int fs_mg_free(fs_ctx *ctx) {
   fs_mg_dev *M = ctx->mg;
   if (!M) return FS_OK;
   for (int q = 0; q < M->nlev; q++) {
-    void *p[] = {M->colors[q], M->chunk[q], q ? M->nnb[q] : nullptr, q ? M->nbr[q] : nullptr, M->parent[q], M->cptr[q], M->clist[q],
+    void *p[] = {M->colors[q], q ? M->nnb[q] : nullptr, q ? M->nbr[q] : nullptr, M->parent[q], M->cptr[q], M->clist[q],
                  M->cmap[q], M->rptr[q], M->rlist[q], q ? M->ac[q] : nullptr, q ? M->anb[q] : nullptr, M->b[q], M->x[q],
                  M->r[q], M->acf[q], M->anbf[q], M->bf[q], M->xf[q], M->rf[q], M->t[q], M->tf[q]};
     for (void *x : p) if (x) cudaFree(x);
   }
+  for (int q = 0; q < FS_MG_MAXLEV; q++) {
+    void *p[] = {M->vsb[q], M->vcol[q], M->vmap[q], M->vrow[q], M->vkp[q],
+                 M->vval[0][q], M->vac[0][q], M->vb[0][q], M->vx[0][q], M->vval[1][q], M->vac[1][q], M->vb[1][q], M->vx[1][q]};
+    for (void *x : p) if (x) cudaFree(x);
+  }
+  cudaFree(M->par0);
+  cudaFree(M->vc64); cudaFree(M->vc32); cudaFree(M->seg[0]); cudaFree(M->seg[1]); cudaFree(M->gridbar);
   cudaFree(M->lev64); cudaFree(M->lev32); cudaFree(M->red); cudaFree(M->sinv);
   delete M;
   ctx->mg = nullptr;
@@ -894,6 +937,140 @@ static int mg_coarse_matrices(fs_ctx *ctx, int last, bool f32) {
   return FS_OK;
 }
 
+// ---------------------------------------------------------------- V-cycle layout
+// Once per context: levels 1 .. lc-1 renumbered aggregate by aggregate (the
+// coarsest keeps its numbering, so its dense inverse is used as it is; within
+// an aggregate rows stay in ascending original order, which keeps every sum's
+// order), their sliced layout, and for the
+// precision asked for the arrays and the descriptor.
+static int mg_vc_build(fs_ctx *ctx, bool f32) {
+  fs_mg_dev *M = ctx->mg;
+  if (M->vc_ready[f32]) return FS_OK;
+  const int lc = M->lc;
+  int rc;
+  if (!M->vc_map) {
+    std::vector<int32_t> up(M->n[lc]), id;   // new numbers of the coarser level, of this one
+    for (int i = 0; i < M->n[lc]; i++) up[i] = i;
+    for (int l = lc; l >= 0; l--) {
+      const int n = M->n[l];
+      const std::vector<int32_t> &nnb = l ? M->h_nnb[l] : ctx->h_ncf, &nbr = l ? M->h_nbr[l] : ctx->h_cn;
+      std::vector<int32_t> row(n);           // original row of each new one
+      if (l == lc) id = up;
+      else {
+        const std::vector<int32_t> &par = M->h_parent[l];
+        const int nc = M->n[l + 1];
+        std::vector<int32_t> kp(nc + 1, 0);
+        for (int i = 0; i < n; i++) kp[up[par[i]] + 1]++;
+        for (int P = 0; P < nc; P++) kp[P + 1] += kp[P];
+        std::vector<int32_t> at(kp.begin(), kp.end() - 1);
+        id.resize(n);
+        for (int i = 0; i < n; i++) id[i] = at[up[par[i]]]++;
+        if ((rc = upv(ctx, &M->vkp[l], kp))) return rc;
+        if (l == 0) {
+          std::vector<int32_t> p0(n);
+          for (int i = 0; i < n; i++) p0[i] = up[par[i]];
+          if ((rc = upv(ctx, &M->par0, p0))) return rc;
+        }
+      }
+      for (int i = 0; i < n; i++) row[id[i]] = i;
+      std::vector<int32_t> col, map;
+      if (l == 0) {
+        const int w = M->w[0];
+        col.resize((size_t)w * n);
+        map.resize((size_t)w * n);
+        for (int j = 0; j < w; j++)
+          for (int a = 0; a < n; a++) {
+            const size_t src = (size_t)j * n + row[a], dst = (size_t)j * n + a;
+            col[dst] = nbr[src];
+            map[dst] = nbr[src] >= 0 ? (int32_t)src : -1;
+          }
+      } else {
+        const int nsl = (n + 31) / 32;
+        std::vector<int32_t> sb(nsl + 1, 0);
+        for (int s = 0; s < nsl; s++) {
+          int wd = 0;
+          for (int a = 32 * s; a < std::min(n, 32 * s + 32); a++) wd = std::max(wd, (int)nnb[row[a]]);
+          sb[s + 1] = sb[s] + wd;
+        }
+        col.assign((size_t)sb[nsl] * 32, 0);
+        map.assign((size_t)sb[nsl] * 32, -1);
+        for (int a = 0; a < n; a++)
+          for (int j = 0; j < sb[a / 32 + 1] - sb[a / 32]; j++) {
+            const size_t dst = ((size_t)sb[a / 32] + j) * 32 + a % 32, src = (size_t)j * n + row[a];
+            col[dst] = a;
+            if (j < nnb[row[a]] && nbr[src] >= 0) { col[dst] = id[nbr[src]]; map[dst] = (int32_t)src; }
+          }
+        if ((rc = upv(ctx, &M->vsb[l], sb))) return rc;
+      }
+      M->vnpos[l] = (int)col.size();
+      if ((rc = upv(ctx, &M->vcol[l], col)) || (rc = upv(ctx, &M->vmap[l], map)) || (rc = upv(ctx, &M->vrow[l], row)))
+        return rc;
+      up.swap(id);
+    }
+    for (int q = 0; q < M->nlev; q++) { M->h_nnb[q] = std::vector<int32_t>(); M->h_nbr[q] = std::vector<int32_t>(); }
+    M->vc_map = true;
+  }
+  const size_t es = f32 ? sizeof(float) : sizeof(double);
+  std::vector<LayoutSeg> segs;
+  int blocks = 0;
+  auto seg = [&](int n, const int32_t *map, const double *src, void *dst) {
+    LayoutSeg g{};
+    g.block0 = blocks; g.n = n; g.map = map; g.src = src;
+    (f32 ? (void *&)g.d32 : (void *&)g.d64) = dst;
+    blocks += fs_grid(n);
+    segs.push_back(g);
+  };
+  for (int l = 0; l <= lc; l++) {
+    FS_CK(cudaMalloc(&M->vval[f32][l], es * std::max(1, M->vnpos[l])));
+    FS_CK(cudaMalloc(&M->vac[f32][l], es * M->n[l]));
+    seg(M->vnpos[l], M->vmap[l], M->anb[l], M->vval[f32][l]);
+    seg(M->n[l], M->vrow[l], M->ac[l], M->vac[f32][l]);
+    if (l == 0) { M->nseg0 = (int)segs.size(); M->seg0_blocks = blocks; }
+    FS_CK(cudaMalloc(&M->vx[f32][l], es * M->n[l == 0 ? 1 : l]));   // [0]: the result of level 1
+    if (l > 0) FS_CK(cudaMalloc(&M->vb[f32][l], es * M->n[l]));
+  }
+  M->nseg = (int)segs.size(); M->seg_blocks = blocks;
+  FS_CK(cudaMalloc(&M->seg[f32], sizeof(LayoutSeg) * segs.size()));
+  FS_CK(cudaMemcpy(M->seg[f32], segs.data(), sizeof(LayoutSeg) * segs.size(), cudaMemcpyHostToDevice));
+  auto desc = [&](auto *tag, auto **dev, const LevelDev<std::remove_pointer_t<decltype(tag)>> *levs) -> int {
+    using R = std::remove_pointer_t<decltype(tag)>;
+    VcDev<R> v{};
+    v.lc = lc;
+    for (int l = 0; l <= lc; l++) {
+      VcLevel<R> &d = v.L[l];
+      d.n = M->n[l]; d.w = M->w[l];
+      d.sb = M->vsb[l]; d.col = M->vcol[l]; d.cells = M->vrow[l];
+      d.val = (const R *)M->vval[f32][l]; d.ac = (const R *)M->vac[f32][l];
+      d.kp = M->vkp[l];
+      d.b = (R *)M->vb[f32][l]; d.x = l > 0 ? (R *)M->vx[f32][l] : nullptr;
+      d.r = (R *)(f32 ? (void *)M->rf[l] : (void *)M->r[l]);
+    }
+    v.x1 = (R *)M->vx[f32][0];
+    v.sinv = M->sinv;
+    FS_CK(cudaMemcpy(&v.L0, levs, sizeof(LevelDev<R>), cudaMemcpyDeviceToHost));
+    v.par0 = M->par0;
+    FS_CK(cudaMalloc(dev, sizeof(VcDev<R>)));
+    FS_CK(cudaMemcpy(*dev, &v, sizeof(VcDev<R>), cudaMemcpyHostToDevice));
+    return FS_OK;
+  };
+  if (f32) rc = desc((float *)nullptr, &M->vc32, M->lev32);
+  else rc = desc((double *)nullptr, &M->vc64, M->lev64);
+  if (rc) return rc;
+  FS_CK(cudaStreamSynchronize(cudaStreamLegacy));   // the uploads, before the solver's stream reads them
+  M->vc_ready[f32] = true;
+  return FS_OK;
+}
+
+// the current matrices in the V-cycle's layout (level0: level 0 alone, the
+// coarse levels being kept)
+static int mg_vc_values(fs_ctx *ctx, bool f32, bool level0) {
+  fs_mg_dev *M = ctx->mg;
+  k_mg_layout<<<level0 ? M->seg0_blocks : M->seg_blocks, FS_BLOCK, 0, ctx->st>>>(M->seg[f32],
+                                                                             level0 ? M->nseg0 : M->nseg);
+  FS_LAUNCH_CHECK();
+  return FS_OK;
+}
+
 int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   int rc = fs_mg_build(ctx);
   if (rc) return rc;
@@ -912,6 +1089,8 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
     a.lev = M->lev64; a.nlev = M->nlev; a.type = ctx->cfg.mg_cycle; a.pre = ctx->cfg.mg_pre; a.post = ctx->cfg.mg_post;
     a.maxcycles = ctx->cfg.mg_max_cycles; a.b0 = ctx->bc; a.x0 = ctx->dphi; a.r0 = M->r[0];
     a.rrf = rrf; a.ires = ctx->resblk + RB_ABS + (nf - 1); a.part = M->red; a.iters = ctx->d_iters + (nf - 1);
+    a.gridbar = M->gridbar; a.status = ctx->d_status;
+    FS_CK(cudaMemsetAsync(M->gridbar, 0, sizeof(unsigned) * FS_GRIDBAR_WORDS, ctx->st));
     void *args[] = {&a};
     FS_TIMING(FS_CK(cudaEventRecord(ctx->kev[nf - 1][0], ctx->st)));
     FS_CK(fs_coop_launch((const void *)k_mg_solve, G, fs_coop_block(ctx), args, ctx->st));
@@ -923,6 +1102,10 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   // of the same system (1: every solve); in between the V-cycle keeps them and
   // only level 0 (the current system) is new -- a fixed preconditioner within
   // each solve, which still runs to its tolerance
+  // the one-phase V-cycle needs one pre- and one post-sweep and a dense coarsest level
+  const bool fused = std::max(1, ctx->cfg.mg_pre) == 1 && M->direct && M->lc > 0;
+  const bool vc = gs || fused;
+  if (vc && (rc = mg_vc_build(ctx, f32))) return rc;
   const int refresh = std::max(1, ctx->cfg.pc_refresh);
   const bool reuse = M->built_nf == nf && M->built_f32 == f32 && M->age + 1 < refresh;
   if (reuse) {
@@ -940,12 +1123,14 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   }
   // team-barrier counters of the V-cycle start at zero for every launch
   FS_CK(cudaMemsetAsync(ctx->d_status + 4, 0, sizeof(int32_t) * 2, ctx->st));
+  FS_CK(cudaMemsetAsync(M->gridbar, 0, sizeof(unsigned) * FS_GRIDBAR_WORDS, ctx->st));
   if (M->direct && !reuse) {
     const int n = M->n[M->lc];
     k_mg_dense_inverse<<<1, 1024, sizeof(double) * ((size_t)n * n + 5 * (size_t)n), ctx->st>>>(
         n, M->nnb[M->lc], M->nbr[M->lc], M->ac[M->lc], M->anb[M->lc], M->sinv);
     FS_LAUNCH_CHECK();
   }
+  if (vc && (rc = mg_vc_values(ctx, f32, reuse))) return rc;
   auto fill = [&](auto &a) {
     a.N = ctx->N; a.W = ctx->W; a.ncf = ctx->ncf; a.cn = ctx->cn; a.ac = ctx->ac; a.anb = ctx->anb; a.bc = ctx->bc;
     a.x = ctx->kx; a.r = ctx->kr; a.r0 = ctx->kr0; a.p = ctx->kp; a.v = ctx->kv; a.s = ctx->ks; a.t = ctx->kt;
@@ -960,12 +1145,11 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
       for (int j = 0; j < ctx->pc_nguess && j < FS_GUESS_MAX; j++) a.xs[a.nx++] = ctx->pc_guess[j];
     a.fit = ctx->d_status + 6;
     a.nncnt = ctx->pc_nn ? fs_nn_counters(ctx) : nullptr;   // the network's guess is in the basis
+    a.gridbar = M->gridbar;
     a.teambar = (unsigned *)(ctx->d_status + 4);
     a.status = ctx->d_status;
     a.team_extra = ctx->test_wait_extra;
   };
-  // the fused V-cycle needs one pre- and one post-sweep and a dense coarsest level
-  const bool fused = std::max(1, ctx->cfg.mg_pre) == 1 && M->direct && M->lc > 0;
   if (ctx->pc_defer && nf == FS_VAR_PC) {   // prepared here, launched with other contexts' by fs_pc_batch_launch
     int form = -1;
     if ((rc = fs_pc_batch_form(ctx, &form))) return rc;
@@ -974,18 +1158,18 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
     if (!f32) {
       M->pend64 = AmgKArgs<double>{};
       fill(M->pend64);
-      M->pend64.lev = M->lev64;
+      M->pend64.lev = M->lev64; M->pend64.vc = M->vc64;
     } else {
       M->pend32 = AmgKArgs<float>{};
       fill(M->pend32);
-      M->pend32.lev = M->lev32;
+      M->pend32.lev = M->lev32; M->pend32.vc = M->vc32;
     }
     return FS_OK;
   }
   if (!f32) {
     AmgKArgs<double> a{};
     fill(a);
-    a.lev = M->lev64;
+    a.lev = M->lev64; a.vc = M->vc64;
     void *args[] = {&a};
     if (a.nx > 0) FS_CK(fs_coop_launch(guess_fit_kernel<double>(a.nx), G, fs_coop_block(ctx), args, ctx->st));
     FS_TIMING(FS_CK(cudaEventRecord(ctx->kev[nf - 1][0], ctx->st)));
@@ -994,7 +1178,7 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   } else {
     AmgKArgs<float> a{};
     fill(a);
-    a.lev = M->lev32;
+    a.lev = M->lev32; a.vc = M->vc32;
     void *args[] = {&a};
     if (a.nx > 0) FS_CK(fs_coop_launch(guess_fit_kernel<float>(a.nx), G, fs_coop_block(ctx), args, ctx->st));
     FS_TIMING(FS_CK(cudaEventRecord(ctx->kev[nf - 1][0], ctx->st)));
@@ -1090,7 +1274,7 @@ struct fs_pc_batch {
   void *h_args = nullptr;       // pinned: the n argument blocks, copied to d_args by each launch
   void *d_args = nullptr;
   int32_t *d_start = nullptr;   // n + 1 CTA offsets
-  unsigned *d_words = nullptr;  // 2n team-barrier words, then 2n group-barrier words (zero at each launch)
+  unsigned *d_words = nullptr;  // per context FS_GRIDBAR_WORDS barrier counts, then 2 team words each (zero at each launch)
   std::vector<int32_t> start;
 };
 
@@ -1142,7 +1326,7 @@ int fs_pc_batch_create(fs_ctx **cs, int n, const double *weight, fs_pc_batch **o
   if ((e = cudaHostAlloc(&B->h_args, B->argsz * n, cudaHostAllocDefault)) != cudaSuccess ||
       (e = cudaMalloc(&B->d_args, B->argsz * n)) != cudaSuccess ||
       (e = cudaMalloc(&B->d_start, sizeof(int32_t) * (n + 1))) != cudaSuccess ||
-      (e = cudaMalloc(&B->d_words, sizeof(unsigned) * 4 * n)) != cudaSuccess ||
+      (e = cudaMalloc(&B->d_words, sizeof(unsigned) * (FS_GRIDBAR_WORDS + 2) * n)) != cudaSuccess ||
       (e = cudaMemcpy(B->d_start, B->start.data(), sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice)) != cudaSuccess) {
     ctx->err = std::string("batched p' set-up: ") + cudaGetErrorString(e);
     fs_pc_batch_free(B);
@@ -1164,31 +1348,32 @@ int fs_pc_batch_launch(fs_pc_batch *B, fs_ctx **cs, int n, cudaStream_t st) {
     char *dst = (char *)B->h_args + B->argsz * q;
     if (B->form <= 1) {
       AmgKArgs<double> a = M->pend64;
-      a.teambar = B->d_words + 2 * q;
+      a.gridbar = B->d_words + (size_t)FS_GRIDBAR_WORDS * q;
+      a.teambar = B->d_words + (size_t)FS_GRIDBAR_WORDS * n + 2 * q;
       if (a.nx > 0 && a.nx <= FS_GUESS_MAX) nx_mask |= 1u << a.nx;
       memcpy(dst, &a, sizeof(a));
     } else {
       AmgKArgs<float> a = M->pend32;
-      a.teambar = B->d_words + 2 * q;
+      a.gridbar = B->d_words + (size_t)FS_GRIDBAR_WORDS * q;
+      a.teambar = B->d_words + (size_t)FS_GRIDBAR_WORDS * n + 2 * q;
       if (a.nx > 0 && a.nx <= FS_GUESS_MAX) nx_mask |= 1u << a.nx;
       memcpy(dst, &a, sizeof(a));
     }
     M->pend_form = -1;
   }
   FS_CK(cudaMemcpyAsync(B->d_args, B->h_args, B->argsz * n, cudaMemcpyHostToDevice, st));
-  unsigned *gw = B->d_words + 2 * n;
-  void *args[] = {&B->d_args, &B->d_start, &B->n, &gw};
+  void *args[] = {&B->d_args, &B->d_start, &B->n};
   // the initial guesses, same groups: one launch per basis size present (a
   // group sits out the launches of other sizes); the barrier words start from
   // zero for each launch
   for (int nx = 1; nx <= FS_GUESS_MAX; nx++) {
     if (!(nx_mask & (1u << nx))) continue;
-    FS_CK(cudaMemsetAsync(B->d_words, 0, sizeof(unsigned) * 4 * n, st));
+    FS_CK(cudaMemsetAsync(B->d_words, 0, sizeof(unsigned) * (FS_GRIDBAR_WORDS + 2) * n, st));
     FS_CK(fs_coop_launch(B->form <= 1 ? guess_fit_batch_kernel<double>(nx) : guess_fit_batch_kernel<float>(nx),
                          B->ncta, FS_COOP_BLOCK, args, st));
     FS_LAUNCH_CHECK();
   }
-  FS_CK(cudaMemsetAsync(B->d_words, 0, sizeof(unsigned) * 4 * n, st));
+  FS_CK(cudaMemsetAsync(B->d_words, 0, sizeof(unsigned) * (FS_GRIDBAR_WORDS + 2) * n, st));
   FS_CK(fs_coop_launch(batch_kernel(B->form), B->ncta, FS_COOP_BLOCK, args, st));
   FS_LAUNCH_CHECK();
   return FS_OK;
