@@ -12,6 +12,8 @@ struct GridState {
   unsigned arrivals;   // arrivals per barrier
   unsigned *bar;       // arrival count, zero at launch, never reset
   int32_t *status;     // [0] set when a barrier timed out
+  double *part;        // partial sums
+  int buf;             // buffer of the next sums
 };
 __device__ __forceinline__ GridState &gstate() {
   __shared__ GridState g;
@@ -26,22 +28,29 @@ __device__ __forceinline__ int cta_count() { return (int)gridDim.x; }
 #endif
 // before the first barrier, by every thread; `extra` arrivals never come (only
 // to test the timeout)
-__device__ __forceinline__ void grid_state_init(unsigned *bar, int32_t *status, int extra) {
+__device__ __forceinline__ void grid_state_init(double *part, unsigned *bar, int32_t *status, int extra) {
   if (threadIdx.x == 0) {
     GridState &G = gstate();
     G.target = 0;
     G.arrivals = (unsigned)(cta_count() + extra);
     G.bar = bar;
     G.status = status;
+    G.part = part;
+    G.buf = 0;
   }
   __syncthreads();
 }
 // Barrier among the system's CTAs, all co-resident (cooperative launch): one
 // release-add per CTA on a count that only grows, then acquire polls until it
 // reaches the next multiple of the CTA count -- one round trip to the L2 for
-// the arrival and one for the poll that sees the last one, no reset and no
-// second word.  Polls are bounded; a timeout is recorded in the system's
-// status word, and once that is set no barrier waits for long any more.
+// the arrival and one for the poll that sees the last one (1.2 us for 148 CTAs
+// on B200, the empty barrier), no reset and no second word.  Polls are bounded;
+// a timeout is recorded in the system's status word, and once that is set no
+// barrier waits for long any more.
+//
+// Nothing that the solve needs later is left in registers across a barrier
+// (arguments, descriptors and the iteration's scalars live in shared memory):
+// the loops of every phase get the 64 registers that 1024 threads have.
 __device__ __noinline__ void grid_barrier() {
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -64,27 +73,65 @@ __device__ __noinline__ void grid_barrier() {
   __syncthreads();
 }
 
-struct Sync {
-  double *part;
-  int buf, buf3;
-  __device__ Sync(double *p, unsigned *bar, int32_t *status, int extra) : part(p), buf(0), buf3(0) {
-    grid_state_init(bar, status, extra);
+// grid-deterministic sums of K <= 3 values (every CTA gets the same results):
+// the warps' sums into shared memory, warp k adds them and writes the CTA's
+// partial of value k; behind the barrier warp k adds the CTAs' partials, 32 at a
+// time, and the sums of those.  Two block barriers beside the grid barrier's
+// two; three buffers, so a CTA still reading one sum is not overwritten by the
+// next.
+struct Sum3 { double a, b, c; };
+template <int K>
+__device__ __forceinline__ Sum3 grid_sums(Sum3 in) {
+  __shared__ double sh[3][33];
+  GridState &S = gstate();
+  const int G = cta_count(), lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const double w0 = wsum(in.a), w1 = K > 1 ? wsum(in.b) : 0., w2 = K > 2 ? wsum(in.c) : 0.;
+  if (lane == 0) {
+    sh[0][wid] = w0;
+    if (K > 1) sh[1][wid] = w1;
+    if (K > 2) sh[2][wid] = w2;
   }
+  __syncthreads();
+  double *pb = S.part + (long)(3 * S.buf + wid) * G;
+  if (wid < K) {
+    const double v = wsum(lane < nw ? sh[wid][lane] : 0.);
+    if (lane == 0) pb[cta_id()] = v;
+  }
+  grid_barrier();
+  if (wid < K) {
+    double r = 0.;
+    for (int c0 = 0; c0 < nw && c0 * 32 < G; c0 += 5) {   // 148 CTAs: one round
+      double v[5];
+#pragma unroll
+      for (int c = 0; c < 5; c++) {
+        const int q = (c0 + c) * 32 + lane;
+        v[c] = c0 + c < nw && q < G ? 0. + pb[q] : 0.;
+        if (c0 + c < nw) for (int m = q + blockDim.x; m < G; m += blockDim.x) v[c] += pb[m];
+      }
+#pragma unroll
+      for (int c = 0; c < 5; c++) {
+        const double t = __shfl_sync(0xffffffffu, wsum(v[c]), 0);
+        if (lane == c0 + c) r = t;
+      }
+    }
+    r = wsum(r);
+    if (lane == 0) sh[wid][32] = r;
+  }
+  if (threadIdx.x == 0) S.buf = (S.buf + 1) % 3;
+  __syncthreads();
+  return Sum3{sh[0][32], K > 1 ? sh[1][32] : 0., K > 2 ? sh[2][32] : 0.};
+}
+
+struct Sync {
+  __device__ Sync(double *part, unsigned *bar, int32_t *status, int extra) { grid_state_init(part, bar, status, extra); }
   __device__ __forceinline__ void gbar() { grid_barrier(); }
-  __device__ void all() { gbar(); }
-  // grid-deterministic sum of two values (every CTA gets the same result)
-  __device__ void sum2(double a0, double a1, double &o0, double &o1) {
-    int G = cta_count();
-    double b0 = bsum(a0), b1 = bsum(a1);
-    if (threadIdx.x == 0) { part[(2 * buf) * G + cta_id()] = b0; part[(2 * buf + 1) * G + cta_id()] = b1; }
-    gbar();
-    double s0 = 0., s1 = 0.;
-    for (int q = threadIdx.x; q < G; q += blockDim.x) { s0 += part[(2 * buf) * G + q]; s1 += part[(2 * buf + 1) * G + q]; }
-    o0 = bsum(s0); o1 = bsum(s1);
-    buf = (buf + 1) % 3;
+  __device__ __forceinline__ void all() { grid_barrier(); }
+  __device__ __forceinline__ void sum2(double a0, double a1, double &o0, double &o1) {
+    const Sum3 r = grid_sums<2>(Sum3{a0, a1, 0.});
+    o0 = r.a; o1 = r.b;
   }
   // grid-deterministic sums of K <= FS_SUMK values, in the partial slots after
-  // the three buffers of sum2 (every CTA gets the same results), with one
+  // the three buffers of sums (every CTA gets the same results), with one
   // block barrier before and one after the grid barrier: warp sums into shared
   // memory, thread k adds the warps' and then the CTAs' partials of value k in
   // a fixed order
@@ -92,7 +139,7 @@ struct Sync {
   __device__ void sumKt(const double (&in)[K], double (&out)[K]) {
     __shared__ double sh[K][33];
     const int G = cta_count(), lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    double *pk = part + 6L * G;
+    double *pk = gstate().part + 9L * G;
 #pragma unroll
     for (int k = 0; k < K; k++) {
       const double v = wsum(in[k]);
@@ -115,19 +162,6 @@ struct Sync {
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < K; k++) out[k] = sh[k][32];
-  }
-  // grid-deterministic sums of three values, in three rotating buffers of
-  // their own after the sumK slots
-  __device__ void sum3(double a0, double a1, double a2, double &o0, double &o1, double &o2) {
-    const int G = cta_count();
-    double *pb = part + (6L + FS_SUMK + 3L * buf3) * G;
-    const double b0 = bsum(a0), b1 = bsum(a1), b2 = bsum(a2);
-    if (threadIdx.x == 0) { pb[cta_id()] = b0; pb[G + cta_id()] = b1; pb[2 * G + cta_id()] = b2; }
-    gbar();
-    double s0 = 0., s1 = 0., s2 = 0.;
-    for (int q = threadIdx.x; q < G; q += blockDim.x) { s0 += pb[q]; s1 += pb[G + q]; s2 += pb[2 * G + q]; }
-    o0 = bsum(s0); o1 = bsum(s1); o2 = bsum(s2);
-    buf3 = (buf3 + 1) % 3;
   }
 };
 
@@ -414,16 +448,6 @@ struct PCycle {
 
 };
 
-// rows i and i2 (when h2) of A x at once (ell_acc2)
-template <class A>
-__device__ __forceinline__ void row_ax2(const A &a, long i, long i2, bool h2, const double *x, double &t1, double &t2) {
-  t1 = 0.0;
-  t1 = t1 + a.ac[i] * x[i];
-  t2 = 0.0;
-  if (h2) t2 = t2 + a.ac[i2] * x[i2];
-  ell_acc2<6, false>(t1, t2, a.N, a.W, a.cn, a.anb, i, i2, h2, [&](int k) { return x[k]; });
-}
-
 // ------------------------------------------------------------ V-cycle in one phase per level and leg
 // One damped-Jacobi pre- and post-sweep per level and a dense coarsest solve,
 // with the arithmetic and the order of every sum of PCycle::run():
@@ -448,6 +472,16 @@ template <class R>
 __device__ __forceinline__ VcDev<R> &vstate() {
   __shared__ VcDev<R> s;
   return s;
+}
+// the solve's arguments, for the phases
+template <class R>
+__device__ __forceinline__ AmgKArgs<R> &astate() {
+  __shared__ AmgKArgs<R> s;
+  return s;
+}
+template <class T>
+__device__ __forceinline__ void copy_words(T &dst, const T &src) {
+  for (int q = threadIdx.x; q < (int)(sizeof(T) / 4); q += blockDim.x) ((int32_t *)&dst)[q] = ((const int32_t *)&src)[q];
 }
 
 // lanes per row of a level, from the threads that the cycle of PCycle gives it
@@ -478,15 +512,15 @@ __device__ __forceinline__ void vc_split() {
   }
 }
 
-// the warps that work on a phase: the grid's, or CTA 0's on small levels
+// the grid's warps over the items of a phase
 struct Warps {
   int w0, nw;
   // with items for every warp a CTA takes neighbouring ones; with fewer they
   // are spread over the CTAs
-  __device__ Warps(bool grid, int items) {
+  __device__ Warps(int items) {
     const int wid = threadIdx.x >> 5, wpc = blockDim.x >> 5;
-    nw = grid ? wpc * cta_count() : wpc;
-    w0 = !grid ? wid : items >= nw ? cta_id() * wpc + wid : wid * cta_count() + cta_id();
+    nw = wpc * cta_count();
+    w0 = items >= nw ? cta_id() * wpc + wid : wid * cta_count() + cta_id();
   }
 };
 
@@ -496,106 +530,161 @@ __device__ __forceinline__ R lanes_sum(R v, int G) {
   return v;
 }
 
-// residuals of level l summed into the rows of level l+1: b, and the first
-// sweep from zero x = omega b / ac unless that is the coarsest.  A CTA takes the
-// aggregates [p0, p1) and with them the consecutive rows [e0, e1): residuals
-// first (G lanes a row, two rows in flight), kept in shared memory or, when they
-// do not fit, in the level's r, then after a block barrier the sums.  FINE:
-// level 0 with b = in and x = x0 in mesh order (row a is cell cells[a]).
-template <class R, bool FINE>
-__device__ __forceinline__ void vc_down(const VcDev<R> &V, int l, int Gc, bool sweep, const double *in, const R *x0) {
+// the down legs' residuals, one array for all of them
+template <class R>
+__device__ __forceinline__ R *vc_rows() {
   __shared__ R sh[FS_VC_ROWS];
-  const VcLevel<R> &F = V.L[l], &C = V.L[l + 1];
-  const int G = FINE ? 1 : V.G[l];
-  const int e0 = V.e0[l], e1 = V.e1[l], n = F.n, W0 = F.w;
-  R *rs = e1 - e0 <= FS_VC_ROWS ? sh : F.r + e0;
-  const int32_t *__restrict__ sb = F.sb, *__restrict__ col = F.col, *__restrict__ cells = F.cells;
-  const R *__restrict__ val = F.val, *__restrict__ ac = F.ac;
-  const R *x = FINE ? x0 : F.x, *b = F.b;
-  const int q = (threadIdx.x & 31) % G, rpp = blockDim.x / G, rw = (threadIdx.x & 31) / G;
-  constexpr int U = FINE ? 6 : 4;
-  for (int a = e0 + (int)(threadIdx.x & ~31u) / G; a < e1; a += 2 * rpp) {
-    const int a0 = a + rw, a1 = a0 + rpp;
-    const bool h0 = a0 < e1, h1 = a1 < e1;
-    long p0, p1;
-    int w0, w1;
-    const int st = FINE ? n : 32;
-    if (FINE) {
-      p0 = a0; p1 = a1;
-      w0 = h0 ? W0 : 0; w1 = h1 ? W0 : 0;
-    } else {
-      const int s0 = h0 ? __ldg(sb + (a0 >> 5)) : 0, s1 = h1 ? __ldg(sb + (a1 >> 5)) : 0;
-      w0 = h0 ? __ldg(sb + (a0 >> 5) + 1) - s0 : 0;
-      w1 = h1 ? __ldg(sb + (a1 >> 5) + 1) - s1 : 0;
-      p0 = (long)s0 * 32 + (a0 & 31);
-      p1 = (long)s1 * 32 + (a1 & 31);
-    }
-    const int i0 = FINE ? (h0 ? __ldg(cells + a0) : 0) : a0, i1 = FINE ? (h1 ? __ldg(cells + a1) : 0) : a1;
-    R t0 = (R)0, t1 = (R)0;
-    const int wm = w0 > w1 ? w0 : w1;
-    for (int j0 = q; j0 < wm; j0 += U * G) {
-      int k0[U], k1[U];
-      R c0[U], c1[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int j = j0 + u * G;
-        const bool g0 = j < w0, g1 = j < w1;
-        k0[u] = g0 ? __ldg(col + p0 + (long)j * st) : -1;
-        c0[u] = g0 ? __ldg(val + p0 + (long)j * st) : (R)0;
-        k1[u] = g1 ? __ldg(col + p1 + (long)j * st) : -1;
-        c1[u] = g1 ? __ldg(val + p1 + (long)j * st) : (R)0;
-      }
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        if (k0[u] >= 0) t0 = t0 + c0[u] * x[k0[u]];
-        if (k1[u] >= 0) t1 = t1 + c1[u] * x[k1[u]];
-      }
-    }
-    if (G > 1) { t0 = lanes_sum(t0, G); t1 = lanes_sum(t1, G); }
-    if (q == 0) {
-      if (h0) rs[a0 - e0] = (FINE ? (R)in[i0] : b[i0]) - __ldg(ac + a0) * x[i0] - t0;
-      if (h1) rs[a1 - e0] = (FINE ? (R)in[i1] : b[i1]) - __ldg(ac + a1) * x[i1] - t1;
-    }
+  return sh;
+}
+
+// Sums of the residuals of the CTA's rows (rs, from row e0 of level l) over its
+// aggregates: b of level l+1, and unless that is the coarsest its first sweep
+// from zero x = omega b / ac.  Gc lanes an aggregate; (P, c0, c1, d): the
+// thread's first aggregate, its rows and diagonal, loaded before the residuals
+// were done.
+template <class R>
+struct AggFirst { int P, c0, c1; R d; };
+template <class R>
+__device__ __forceinline__ AggFirst<R> vc_agg(const VcDev<R> &V, int l, int Gc, bool sweep, int P) {
+  const int lane = threadIdx.x & 31;
+  AggFirst<R> f{P, 0, 0, (R)1};
+  if (P < V.p1[l]) {
+    f.c0 = __ldg(V.L[l].kp + P) - V.e0[l] + lane % Gc;
+    f.c1 = __ldg(V.L[l].kp + P + 1) - V.e0[l];
+    if (sweep) f.d = __ldg(V.L[l + 1].ac + P);
   }
-  __syncthreads();
-  const int32_t *__restrict__ kp = F.kp;
-  const int P1 = V.p1[l], qc = (threadIdx.x & 31) % Gc;
-  for (int Pw = V.p0[l] + (int)(threadIdx.x & ~31u) / Gc; Pw < P1; Pw += blockDim.x / Gc) {
-    const int P = Pw + (threadIdx.x & 31) / Gc;
-    const bool h = P < P1;
-    const int c0 = h ? __ldg(kp + P) - e0 + qc : 0, c1 = h ? __ldg(kp + P + 1) - e0 : 0;
-    const R d = h && sweep ? __ldg(C.ac + P) : (R)1;
+  return f;
+}
+template <class R>
+__device__ __forceinline__ void vc_restrict(const VcDev<R> &V, int l, int Gc, bool sweep, const R *rs, AggFirst<R> f) {
+  const VcLevel<R> &C = V.L[l + 1];
+  const int lane = threadIdx.x & 31, P1 = V.p1[l];
+  while (f.P - lane / Gc < P1) {
     R s = (R)0;
-    for (int c = c0; c < c1; c += 4 * Gc) {
+    for (int c = f.c0; c < f.c1; c += 4 * Gc) {
       R v[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) v[u] = c + u * Gc < c1 ? rs[c + u * Gc] : (R)0;
+      for (int u = 0; u < 4; u++) v[u] = c + u * Gc < f.c1 ? rs[c + u * Gc] : (R)0;
 #pragma unroll
-      for (int u = 0; u < 4; u++) if (c + u * Gc < c1) s = s + v[u];
+      for (int u = 0; u < 4; u++) if (c + u * Gc < f.c1) s = s + v[u];
     }
     if (Gc > 1) s = lanes_sum(s, Gc);
-    if (h && qc == 0) {
-      C.b[P] = s;
-      if (sweep) C.x[P] = (R)FS_MG_OMEGA * s / d;
+    if (f.P < P1 && lane % Gc == 0) {
+      C.b[f.P] = s;
+      if (sweep) C.x[f.P] = (R)FS_MG_OMEGA * s / f.d;
     }
+    f = vc_agg(V, l, Gc, sweep, f.P + (int)blockDim.x / Gc);
   }
+}
+
+// Down leg of level l >= 1.  A CTA takes the aggregates [p0, p1) and with them
+// the consecutive rows [e0, e1): residuals first (G lanes a row), kept in
+// shared memory or, when they do not fit, in the level's r, then behind a block
+// barrier their sums.  Every phase ends with a grid barrier.
+template <class R>
+__device__ __forceinline__ void vc_down(int l, int Gc, bool sweep) {
+  const VcDev<R> &V = vstate<R>();
+  R *sh = vc_rows<R>();
+  constexpr int U = 8;
+  const VcLevel<R> &F = V.L[l];
+  const int G = V.G[l], e0 = V.e0[l], e1 = V.e1[l], w = F.w;
+  R *rs = e1 - e0 <= FS_VC_ROWS ? sh : F.r + e0;
+  const int32_t *__restrict__ col = F.col;
+  const R *__restrict__ val = F.val, *__restrict__ ac = F.ac;
+  const R *x = F.x, *b = F.b;
+  const int lane = threadIdx.x & 31, q = lane % G, rpp = (int)blockDim.x / G;
+  const AggFirst<R> first = vc_agg(V, l, Gc, sweep, V.p0[l] + (int)threadIdx.x / Gc);
+  for (int a = e0 + (int)threadIdx.x / G; a - lane / G < e1; a += rpp) {
+    const bool h = a < e1;
+    const long p = ((long)(a >> 5) * w) * 32 + (a & 31);
+    const R bi = h ? b[a] : (R)0, xi = h ? x[a] : (R)0, d = h ? __ldg(ac + a) : (R)0;
+    R t = (R)0;
+    for (int j0 = q; j0 < w; j0 += U * G) {
+      int k[U];
+      R c[U], g[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const bool in = h && j0 + u * G < w;
+        k[u] = in ? __ldg(col + p + (long)(j0 + u * G) * 32) : -1;
+        c[u] = in ? __ldg(val + p + (long)(j0 + u * G) * 32) : (R)0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) g[u] = k[u] >= 0 ? x[k[u]] : (R)0;
+#pragma unroll
+      for (int u = 0; u < U; u++) t = t + c[u] * g[u];
+    }
+    if (G > 1) t = lanes_sum(t, G);
+    if (h && q == 0) rs[a - e0] = bi - d * xi - t;
+  }
+  __syncthreads();
+  vc_restrict(V, l, Gc, sweep, rs, first);
+  grid_barrier();
+}
+
+// The same for level 0: b = in and x = x0 in mesh order, row a is cell cells[a],
+// a thread per row.
+template <class R>
+__device__ __forceinline__ void vc_down_fine(int Gc, const double *in, const R *x0) {
+  const VcDev<R> &V = vstate<R>();
+  R *sh = vc_rows<R>();
+  constexpr int U = 6;
+  const VcLevel<R> &F = V.L[0];
+  const int e0 = V.e0[0], e1 = V.e1[0], n = F.n, w = F.w;
+  const bool sweep = V.lc > 1;
+  R *rs = e1 - e0 <= FS_VC_ROWS ? sh : F.r + e0;
+  const int32_t *__restrict__ col = F.col, *__restrict__ cells = F.cells;
+  const R *__restrict__ val = F.val, *__restrict__ ac = F.ac;
+  int a = e0 + (int)threadIdx.x, i = a < e1 ? __ldg(cells + a) : 0, k[U];
+  AggFirst<R> first = vc_agg(V, 0, Gc, sweep, V.p0[0] + (int)threadIdx.x / Gc);
+#pragma unroll
+  for (int u = 0; u < U; u++) k[u] = a < e1 && u < w ? __ldg(col + (long)u * n + a) : -1;
+  while (a < e1) {
+    R c[U], g[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      c[u] = k[u] >= 0 ? __ldg(val + (long)u * n + a) : (R)0;
+      g[u] = k[u] >= 0 ? x0[k[u]] : (R)0;
+    }
+    const R bi = (R)in[i], xi = x0[i], d = __ldg(ac + a);
+    const int an = a + (int)blockDim.x;
+    i = an < e1 ? __ldg(cells + an) : 0;
+#pragma unroll
+    for (int u = 0; u < U; u++) k[u] = an < e1 && u < w ? __ldg(col + (long)u * n + an) : -1;
+    R t = (R)0;
+#pragma unroll
+    for (int u = 0; u < U; u++) t = t + c[u] * g[u];
+    for (int j = U; j < w; j++) {
+      const int kj = __ldg(col + (long)j * n + a);
+      if (kj >= 0) t = t + __ldg(val + (long)j * n + a) * x0[kj];
+    }
+    rs[a - e0] = bi - d * xi - t;
+    a = an;
+  }
+  __syncthreads();
+  vc_restrict(V, 0, Gc, sweep, rs, first);
+  grid_barrier();
 }
 
 // post-sweep of level L's rows, then the prolongation into the finer level F's
 // x (last: level 1, whose result goes to x1)
 template <class R>
-__device__ __forceinline__ void vc_up(const VcLevel<R> &L, const VcLevel<R> &F, int G, bool last, R *x1, const Warps w) {
-  const int lane = threadIdx.x & 31, q = lane % G, rpw = 32 / G, n = L.n;
-  const int32_t *__restrict__ sb = L.sb, *__restrict__ col = L.col, *__restrict__ kp = F.kp;
+__device__ __forceinline__ void vc_up(int l) {
+  const VcDev<R> &V = vstate<R>();
+  const VcLevel<R> &L = V.L[l], &F = V.L[l - 1];
+  const int G = V.G[l];
+  const bool last = l == 1;
+  R *x1 = V.x1;
+  constexpr int U = 8;
+  const int lane = threadIdx.x & 31, q = lane % G, rpw = 32 / G, n = L.n, wd = L.w;
+  const Warps w((n + rpw - 1) / rpw);
+  const int32_t *__restrict__ col = L.col, *__restrict__ kp = F.kp;
   const R *__restrict__ val = L.val, *__restrict__ ac = L.ac;
   const R *x = L.x, *b = L.b;
   R *xf = F.x;
-  constexpr int U = 8;
   for (int s = w.w0; s * rpw < n; s += w.nw) {
     const int i = s * rpw + lane / G;
     const bool act = i < n;
-    const int s0 = act ? __ldg(sb + (i >> 5)) : 0, wd = act ? __ldg(sb + (i >> 5) + 1) - s0 : 0;
-    const long p = (long)s0 * 32 + (i & 31);
+    const long p = ((long)(i >> 5) * wd) * 32 + (i & 31);
     const R xi = act ? x[i] : (R)0, bi = act ? b[i] : (R)0, d = act ? __ldg(ac + i) : (R)1;
     int c = 0, c1 = 0;
     R f0 = (R)0, f1 = (R)0;
@@ -608,15 +697,17 @@ __device__ __forceinline__ void vc_up(const VcLevel<R> &L, const VcLevel<R> &F, 
     R t = (R)0;
     for (int j0 = q; j0 < wd; j0 += U * G) {
       int k[U];
-      R v[U];
+      R v[U], g[U];
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        const int j = j0 + u * G;
-        k[u] = j < wd ? __ldg(col + p + (long)j * 32) : -1;
-        v[u] = j < wd ? __ldg(val + p + (long)j * 32) : (R)0;
+        const bool in = act && j0 + u * G < wd;
+        k[u] = in ? __ldg(col + p + (long)(j0 + u * G) * 32) : -1;
+        v[u] = in ? __ldg(val + p + (long)(j0 + u * G) * 32) : (R)0;
       }
 #pragma unroll
-      for (int u = 0; u < U; u++) if (k[u] >= 0) t = t + v[u] * x[k[u]];
+      for (int u = 0; u < U; u++) g[u] = k[u] >= 0 ? x[k[u]] : (R)0;
+#pragma unroll
+      for (int u = 0; u < U; u++) t = t + v[u] * g[u];
     }
     if (G > 1) t = lanes_sum(t, G);
     if (!act) continue;
@@ -630,14 +721,20 @@ __device__ __forceinline__ void vc_up(const VcLevel<R> &L, const VcLevel<R> &F, 
       for (c += 2 * G; c < c1; c += G) xf[c] = xf[c] + add;
     }
   }
+  grid_barrier();
 }
 
 // the coarsest level by its dense inverse (a warp per row), prolonged into the
 // next finer level, or left in x1 when that is level 0
 template <class R>
-__device__ __forceinline__ void vc_dense(const VcLevel<R> &C, const VcLevel<R> &F, const double *__restrict__ sinv,
-                                         bool last, R *x1, const Warps w) {
+__device__ __forceinline__ void vc_dense() {
+  const VcDev<R> &V = vstate<R>();
+  const VcLevel<R> &C = V.L[V.lc], &F = V.L[V.lc - 1];
+  const double *__restrict__ sinv = V.sinv;
+  const bool last = V.lc == 1;
+  R *x1 = V.x1;
   const int lane = threadIdx.x & 31, n = C.n;
+  const Warps w(n);
   const R *b = C.b;
   R *xf = F.x;
   for (int i = w.w0; i < n; i += w.nw) {
@@ -660,97 +757,95 @@ __device__ __forceinline__ void vc_dense(const VcLevel<R> &C, const VcLevel<R> &
       for (int c = __ldg(F.kp + i) + lane; c < __ldg(F.kp + i + 1); c += 32) xf[c] = xf[c] + add;
     }
   }
+  grid_barrier();
 }
 
-// levels 1 and below: from b_1, x_1 to the corrected x_1 in V.x1; ends with a
-// grid barrier.  GS: the restriction sums a coarse row's children in sequence.
+// levels 1 and below: from b_1, x_1 to the corrected x_1 in V.x1.  GS: the
+// restriction sums a coarse row's children in sequence.
 template <class R, bool GS>
-__device__ __forceinline__ void vcycle_coarse(Sync &S) {
+__device__ __forceinline__ void vcycle_coarse() {
   const VcDev<R> &V = vstate<R>();
   const int lc = V.lc;
-  for (int l = 1; l < lc; l++) {
-    vc_down<R, false>(V, l, GS ? 1 : V.G[l + 1], l + 1 < lc, nullptr, nullptr);
-    S.all();
-  }
-  vc_dense<R>(V.L[lc], V.L[lc - 1], V.sinv, lc == 1, V.x1, Warps(true, V.L[lc].n));
-  S.all();
-  for (int l = lc - 1; l >= 1; l--) {
-    const int rpw = 32 / V.G[l];
-    vc_up<R>(V.L[l], V.L[l - 1], V.G[l], l == 1, V.x1, Warps(true, (V.L[l].n + rpw - 1) / rpw));
-    S.all();
-  }
+  for (int l = 1; l < lc; l++) vc_down<R>(l, GS ? 1 : V.G[l + 1], l + 1 < lc);
+  vc_dense<R>();
+  for (int l = lc - 1; l >= 1; l--) vc_up<R>(l);
 }
 
-// out = M^-1 in.  The caller has set x_0 = omega0 in / ac_0 and passed a grid
-// barrier; ends with one.
+// level 0's post-sweep into out, with its correction formed on the fly; the
+// next row's indices are loaded while a row gathers
 template <class R>
-__device__ __forceinline__ void vcycle(Sync &S, const double *in, double *out) {
+__device__ __forceinline__ void vc_up_fine(const double *in, double *out) {
+  constexpr int U = 6;
   const VcDev<R> &V = vstate<R>();
   const LevelDev<R> &L = V.L0;
-  vc_down<R, true>(V, 0, V.G[1], V.lc > 1, in, L.x);
-  S.all();
-  vcycle_coarse<R, false>(S);
-  const long t0 = (long)cta_id() * blockDim.x + threadIdx.x, nt = (long)cta_count() * blockDim.x;
+  const long nt = (long)cta_count() * blockDim.x;
+  long i = (long)cta_id() * blockDim.x + threadIdx.x;
   const int n = L.n, w = L.w;
   const int32_t *__restrict__ nbr = L.nbr, *__restrict__ par = V.par0;
   const R *__restrict__ anb = L.anb, *__restrict__ ac = L.ac;
   const R *x0 = L.x, *x1 = V.x1;
   const R al0 = (R)FS_MG_ALPHA0, om0 = (R)FS_MG_OMEGA0;
-  for (long i = t0; i < n; i += 2 * nt) {
-    const long i2 = i + nt;
-    const bool h2 = i2 < n;
-    R t1 = (R)0, t2 = (R)0;
-    for (int j0 = 0; j0 < w; j0 += 3) {
-      int k1[3], k2[3], q1[3], q2[3];
-      R c1[3], c2[3], y1[3], y2[3];
+  int k[U];
 #pragma unroll
-      for (int u = 0; u < 3; u++) {
-        const bool h = j0 + u < w;
-        k1[u] = h ? __ldg(nbr + (long)(j0 + u) * n + i) : -1;
-        k2[u] = h && h2 ? __ldg(nbr + (long)(j0 + u) * n + i2) : -1;
-        c1[u] = h ? anb[(long)(j0 + u) * n + i] : (R)0;
-        c2[u] = h && h2 ? anb[(long)(j0 + u) * n + i2] : (R)0;
-      }
+  for (int u = 0; u < U; u++) k[u] = i < n && u < w ? __ldg(nbr + (long)u * n + i) : -1;
+  while (i < n) {
+    R c[U], y[U], z[U];
+    int q[U];
+    const int qi = __ldg(par + i);
 #pragma unroll
-      for (int u = 0; u < 3; u++) {
-        q1[u] = k1[u] >= 0 ? __ldg(par + k1[u]) : 0;
-        q2[u] = k2[u] >= 0 ? __ldg(par + k2[u]) : 0;
-        y1[u] = k1[u] >= 0 ? x0[k1[u]] : (R)0;
-        y2[u] = k2[u] >= 0 ? x0[k2[u]] : (R)0;
-      }
+    for (int u = 0; u < U; u++) q[u] = k[u] >= 0 ? __ldg(par + k[u]) : 0;
 #pragma unroll
-      for (int u = 0; u < 3; u++) {
-        if (k1[u] >= 0) t1 = t1 + c1[u] * (y1[u] + al0 * x1[q1[u]]);
-        if (k2[u] >= 0) t2 = t2 + c2[u] * (y2[u] + al0 * x1[q2[u]]);
-      }
+    for (int u = 0; u < U; u++) {
+      c[u] = k[u] >= 0 ? __ldg(anb + (long)u * n + i) : (R)0;
+      y[u] = k[u] >= 0 ? x0[k[u]] : (R)0;
     }
-    {
-      const R aci = ac[i], xi = x0[i] + al0 * x1[__ldg(par + i)];
-      out[i] = (double)(xi + om0 * ((R)in[i] - aci * xi - t1) / aci);
+    const R aci = __ldg(ac + i), bi = (R)in[i], yi = x0[i], zi = x1[qi];
+#pragma unroll
+    for (int u = 0; u < U; u++) z[u] = k[u] >= 0 ? x1[q[u]] : (R)0;
+    const long in1 = i + nt;
+#pragma unroll
+    for (int u = 0; u < U; u++) k[u] = in1 < n && u < w ? __ldg(nbr + (long)u * n + in1) : -1;
+    R t = (R)0;
+#pragma unroll
+    for (int u = 0; u < U; u++) t = t + c[u] * (y[u] + al0 * z[u]);
+    for (int j = U; j < w; j++) {
+      const int kj = __ldg(nbr + (long)j * n + i);
+      if (kj >= 0) t = t + __ldg(anb + (long)j * n + i) * (x0[kj] + al0 * x1[__ldg(par + kj)]);
     }
-    if (h2) {
-      const R aci = ac[i2], xi = x0[i2] + al0 * x1[__ldg(par + i2)];
-      out[i2] = (double)(xi + om0 * ((R)in[i2] - aci * xi - t2) / aci);
-    }
+    const R xi = yi + al0 * zi;
+    out[i] = (double)(xi + om0 * (bi - aci * xi - t) / aci);
+    i = in1;
   }
-  S.all();
+  grid_barrier();
+}
+
+// out = M^-1 in.  The caller has set x_0 = omega0 in / ac_0 and passed a grid
+// barrier; ends with one.
+template <class R>
+__device__ __forceinline__ void vcycle(const double *in, double *out) {
+  const VcDev<R> &V = vstate<R>();
+  vc_down_fine<R>(V.G[1], in, V.L0.x);
+  vcycle_coarse<R, false>();
+  vc_up_fine<R>(in, out);
 }
 
 // One multicolour Gauss-Seidel pass over level 0 in place: the colours in
 // order (forward) or reversed (backward); rows of one colour read only rows of
 // other colours, so each colour is one phase of independent rows.
 template <class R>
-__device__ __forceinline__ void gs_colours(Sync &S, const LevelDev<R> &L, const double *in, R *x, bool backward) {
+__device__ __forceinline__ void gs_colours(const double *in, bool backward) {
+  const LevelDev<R> &L = vstate<R>().L0;
   const long t0 = (long)cta_id() * blockDim.x + threadIdx.x, nt = (long)cta_count() * blockDim.x;
+  R *x = L.x;
   for (int cc = 0; cc < L.ncolors; cc++) {
     const int c = backward ? L.ncolors - 1 - cc : cc;
-    S.all();
     const int r0 = L.color_ptr[c], r1 = L.color_ptr[c + 1];
     for (long q = r0 + t0; q < r1; q += nt) {
       const int i = L.color_rows[q];
       const R t = ell_acc<6, false>((R)0., L.n, L.w, L.nbr, L.anb, i, [&](int k) { return x[k]; });
       x[i] = ((R)in[i] - t) / L.ac[i];
     }
+    grid_barrier();
   }
 }
 
@@ -759,33 +854,33 @@ __device__ __forceinline__ void gs_colours(Sync &S, const LevelDev<R> &L, const 
 // x += alpha x_1[parent], a backward pass) and damped Jacobi on the others.
 // out = M^-1 in; callers have made `in` visible.
 template <class R>
-__device__ __forceinline__ void vcycle_gs(Sync &S, const double *in, double *out) {
+__device__ __forceinline__ void vcycle_gs(const double *in, double *out) {
   const VcDev<R> &V = vstate<R>();
   const LevelDev<R> &L = V.L0;
   const long t0 = (long)cta_id() * blockDim.x + threadIdx.x, nt = (long)cta_count() * blockDim.x;
   R *x = L.x;
   for (long i = t0; i < L.n; i += nt) x[i] = (R)0.;
-  gs_colours(S, L, in, x, false);
-  S.all();
-  vc_down<R, true>(V, 0, 1, V.lc > 1, in, x);
-  S.all();
-  vcycle_coarse<R, true>(S);
+  grid_barrier();
+  gs_colours<R>(in, false);
+  vc_down_fine<R>(1, in, x);
+  vcycle_coarse<R, true>();
   const R al0 = (R)FS_MG_ALPHA0;
   for (long i = t0; i < L.n; i += nt) x[i] = x[i] + al0 * V.x1[V.par0[i]];
-  gs_colours(S, L, in, x, true);
-  S.all();
+  grid_barrier();
+  gs_colours<R>(in, true);
   for (long i = t0; i < L.n; i += nt) out[i] = (double)x[i];
-  S.all();
+  grid_barrier();
 }
 
 // apply the preconditioner: out (FP64) = M^-1 in (FP64), via the R-precision
 // V-cycle.  MODE: 0 the V-cycle of PCycle::run(), 1 vcycle() (the caller has
 // set x_0 = omega0 in / ac_0), 2 vcycle_gs()
 template <class R, int MODE>
-__device__ __forceinline__ void apply_prec(Sync &S, const AmgKArgs<R> &a, const double *in, double *out, unsigned &gen) {
-  if (MODE == 1) vcycle<R>(S, in, out);
-  else if (MODE == 2) vcycle_gs<R>(S, in, out);
+__device__ __forceinline__ void apply_prec(Sync &S, const double *in, double *out, unsigned &gen) {
+  if (MODE == 1) vcycle<R>(in, out);
+  else if (MODE == 2) vcycle_gs<R>(in, out);
   else {
+    const AmgKArgs<R> &a = astate<R>();
     Scope all;
     all.grid = true;
     PCycle<R> C{S, a.lev, a.lc, a.direct != 0, a.sinv, a.pre, a.post, 20, (R)FS_MG_OMEGA, (R)FS_MG_ALPHA, all,
@@ -793,6 +888,119 @@ __device__ __forceinline__ void apply_prec(Sync &S, const AmgKArgs<R> &a, const 
     C.run(in, out);
     gen = C.gen;
   }
+}
+
+// ------------------------------------------------------------ the passes of the Krylov iteration
+// y = A x over the thread's rows in grid-stride order, with the products its
+// sums need: (y.e, y.y, y.f) or (e.y) alone.  The next row's indices are loaded
+// while a row gathers.  Every pass loads all it needs of a row before it
+// stores, so the stores do not hold up the loads.
+template <class R, int K>
+__device__ __forceinline__ Sum3 krylov_ax(const double *x, double *y, const double *e, const double *f) {
+  constexpr int U = 6;
+  const AmgKArgs<R> &A = astate<R>();
+  const int n = A.N, w = A.W;
+  const int32_t *__restrict__ nbr = A.cn;
+  const double *__restrict__ anb = A.anb, *__restrict__ ac = A.ac;
+  const long nt = (long)cta_count() * blockDim.x;
+  long i = (long)cta_id() * blockDim.x + threadIdx.x;
+  Sum3 s{0., 0., 0.};
+  int k[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) k[u] = i < n && u < w ? __ldg(nbr + (long)u * n + i) : -1;
+  while (i < n) {
+    double c[U], g[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      c[u] = k[u] >= 0 ? __ldg(anb + (long)u * n + i) : 0.;
+      g[u] = k[u] >= 0 ? x[k[u]] : 0.;
+    }
+    const double aci = __ldg(ac + i), xi = x[i], ei = e[i], fi = K > 1 ? f[i] : 0.;
+    const long in = i + nt;
+#pragma unroll
+    for (int u = 0; u < U; u++) k[u] = in < n && u < w ? __ldg(nbr + (long)u * n + in) : -1;
+    double t = aci * xi;
+#pragma unroll
+    for (int u = 0; u < U; u++) t = t + c[u] * g[u];
+    for (int j = U; j < w; j++) {
+      const int kj = __ldg(nbr + (long)j * n + i);
+      if (kj >= 0) t = t + __ldg(anb + (long)j * n + i) * x[kj];
+    }
+    y[i] = t;
+    s.a += t * ei;
+    if (K > 1) { s.b += t * t; s.c += fi * t; }
+    i = in;
+  }
+  return s;
+}
+
+// s = r - alpha v with |s|^2 and r0.s, and x_0 = omega0 s / ac_0 of the V-cycle
+template <class R, int MODE>
+__device__ __forceinline__ Sum3 krylov_s(double alpha) {
+  const AmgKArgs<R> &A = astate<R>();
+  const int n = A.N;
+  const long nt = (long)cta_count() * blockDim.x;
+  const double *r = A.r, *v = A.v, *r0 = A.r0;
+  const R *__restrict__ ac0 = A.lev[0].ac;
+  double *s = A.s;
+  R *x0 = A.lev[0].x;
+  const R om0 = (R)FS_MG_OMEGA0;
+  Sum3 o{0., 0., 0.};
+  for (long i = (long)cta_id() * blockDim.x + threadIdx.x; i < n; i += 2 * nt) {
+    const long j = i + nt;
+    const bool h = j < n;
+    const double r1 = r[i], v1 = v[i], q1 = r0[i], r2 = h ? r[j] : 0., v2 = h ? v[j] : 0., q2 = h ? r0[j] : 0.;
+    const R d1 = MODE == 1 ? __ldg(ac0 + i) : (R)1, d2 = MODE == 1 && h ? __ldg(ac0 + j) : (R)1;
+    const double s1 = r1 - alpha * v1, s2 = r2 - alpha * v2;
+    s[i] = s1;
+    o.a += s1 * s1;
+    o.b += q1 * s1;
+    if (MODE == 1) x0[i] = om0 * (R)s1 / d1;
+    if (h) {
+      s[j] = s2;
+      o.a += s2 * s2;
+      o.b += q2 * s2;
+      if (MODE == 1) x0[j] = om0 * (R)s2 / d2;
+    }
+  }
+  return o;
+}
+
+// x += alpha y + omega z, r = s - omega t, and p = r + beta (p - omega v) of the
+// next iteration with x_0 = omega0 p / ac_0
+template <class R, int MODE>
+__device__ __forceinline__ void krylov_xrp(double alpha, double omega, double beta) {
+  const AmgKArgs<R> &A = astate<R>();
+  const int n = A.N;
+  const long nt = (long)cta_count() * blockDim.x;
+  const double *y = A.y, *z = A.z, *s = A.s, *t = A.t, *v = A.v;
+  double *x = A.x, *r = A.r, *p = A.p;
+  const R *__restrict__ ac0 = A.lev[0].ac;
+  R *x0 = A.lev[0].x;
+  const R om0 = (R)FS_MG_OMEGA0;
+  for (long i = (long)cta_id() * blockDim.x + threadIdx.x; i < n; i += 2 * nt) {
+    const long j = i + nt;
+    const bool h = j < n;
+    double x1 = x[i], y1 = y[i], z1 = z[i], s1 = s[i], t1 = t[i], p1 = p[i], v1 = v[i];
+    double x2 = 0., y2 = 0., z2 = 0., s2 = 0., t2 = 0., p2 = 0., v2 = 0.;
+    if (h) { x2 = x[j]; y2 = y[j]; z2 = z[j]; s2 = s[j]; t2 = t[j]; p2 = p[j]; v2 = v[j]; }
+    const R d1 = MODE == 1 ? __ldg(ac0 + i) : (R)1, d2 = MODE == 1 && h ? __ldg(ac0 + j) : (R)1;
+    x[i] = x1 + alpha * y1 + omega * z1;
+    const double r1 = s1 - omega * t1;
+    r[i] = r1;
+    const double n1 = r1 + beta * (p1 - omega * v1);
+    p[i] = n1;
+    if (MODE == 1) x0[i] = om0 * (R)n1 / d1;
+    if (h) {
+      x[j] = x2 + alpha * y2 + omega * z2;
+      const double r2 = s2 - omega * t2;
+      r[j] = r2;
+      const double n2 = r2 + beta * (p2 - omega * v2);
+      p[j] = n2;
+      if (MODE == 1) x0[j] = om0 * (R)n2 / d2;
+    }
+  }
+  grid_barrier();
 }
 
 // mean of the right-hand side of a pure-Neumann system (every row sums to
@@ -945,15 +1153,18 @@ __device__ __forceinline__ void guess_fit_body(const AmgKArgs<R> a) {
 // and r0.r of the stored r instead, so the exit is always decided on a
 // residual summed from its vector, and a solve that has not really converged
 // continues with p formed in a separate pass.
+struct KrylovState {
+  double alpha, omega, rho, rho_next, ss, r0s, resn, normb;
+  int k;
+  bool p_ready;
+};
 template <class R, int MODE>
-__device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> a) {
-  if (MODE != 0) {   // the operators' descriptors, read in every phase
-    const int32_t *src = (const int32_t *)a.vc;
-    int32_t *dst = (int32_t *)&vstate<R>();
-    for (int q = threadIdx.x; q < (int)(sizeof(VcDev<R>) / 4); q += blockDim.x) dst[q] = src[q];
-    __syncthreads();
-    vc_split<R>();
-  }
+__device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> &ap) {
+  copy_words(astate<R>(), ap);
+  if (MODE != 0) copy_words(vstate<R>(), *ap.vc);
+  __syncthreads();
+  if (MODE != 0) vc_split<R>();
+  const AmgKArgs<R> &a = astate<R>();
   Sync S(a.part, a.gridbar, a.status, a.team_extra);
   unsigned gen = 0;   // team-barrier generation (the counters are zeroed before the launch)
   const int N = a.N;
@@ -972,7 +1183,7 @@ __device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> a) {
   // constant null vector is left to the caller (pressure reference cell).
   const double bmean = rhs_mean(S, a);
   const bool has_x = a.nx > 0 && a.fit[0] != 0;
-  double l0 = 0., l1 = 0., l2 = 0.;
+  double l0 = 0., l1 = 0.;
   for (long i = t0; i < N; i += nt) {
     const double b1 = a.bc[i] - bmean;
     double ri = b1;
@@ -990,98 +1201,69 @@ __device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> a) {
     l0 += ri * ri;
     l1 += b1 * b1;
   }
-  double rr, bb, dum;
+  double rr, bb;
   S.sum2(l0, l1, rr, bb);
-  double normb = sqrt(bb), alpha = 1., omega = 1.;
-  int k = 0;
-  double resn = sqrt(rr);
   // rho = r0 . r of the iteration; rho_next that of the next one, summed from
-  // the stored r when p still has to be formed (p_ready false)
-  double rho = rr, rho_next = rr;
-  bool p_ready = true;
-  if (!(rr != 0.) || !isfinite(rr)) p_ready = false;   // the loop's breakdown test takes it
-  while (k < a.maxit && resn > a.tol * normb && normb > 0.) {
-    k++;
-    if (!p_ready) {
-      const double rho1 = rho_next;
+  // the stored r when p still has to be formed (p_ready false).  Thread 0
+  // writes, everyone reads behind a barrier.
+  __shared__ KrylovState K;
+  if (threadIdx.x == 0) {
+    K.normb = sqrt(bb); K.resn = sqrt(rr); K.alpha = K.omega = 1.; K.rho = K.rho_next = rr; K.k = 0;
+    // rr = 0 or not finite: the loop's breakdown test takes it
+    K.p_ready = rr != 0. && isfinite(rr);
+  }
+  __syncthreads();
+  while (K.k < a.maxit && K.resn > a.tol * K.normb && K.normb > 0.) {
+    if (!K.p_ready) {
+      const double rho1 = K.rho_next;
       // breakdown (r0 . r vanished: r at round-off): keep x.  Every CTA holds
       // the same sums, so every CTA takes the same branch.
-      if (!(rho1 != 0.) || !isfinite(rho1)) break;
-      const double beta = (rho1 / rho) * (alpha / omega);
-      rho = rho1;
+      if (!(rho1 != 0.) || !isfinite(rho1)) {
+        __syncthreads();
+        if (threadIdx.x == 0) K.k++;
+        break;
+      }
+      const double beta = (rho1 / K.rho) * (K.alpha / K.omega), omega = K.omega;
       for (long i = t0; i < N; i += nt) {
         const double pi = a.r[i] + beta * (a.p[i] - omega * a.v[i]);
         a.p[i] = pi;
-        if (MODE == 1) x0v[i] = om0 * (R)pi / ac0[i];
+        if (MODE == 1) a.lev[0].x[i] = om0 * (R)pi / a.lev[0].ac[i];
       }
       S.all();
+      if (threadIdx.x == 0) K.rho = rho1;
     }
-    p_ready = false;
-    apply_prec<R, MODE>(S, a, a.p, a.y, gen);                       // y = M^-1 p
-    l0 = 0.;
-    for (long i = t0; i < N; i += 2 * nt) {
-      const long i2 = i + nt;
-      const bool h2 = i2 < N;
-      double v1, v2;
-      row_ax2(a, i, i2, h2, a.y, v1, v2);
-      a.v[i] = v1; l0 += a.r0[i] * v1;
-      if (h2) { a.v[i2] = v2; l0 += a.r0[i2] * v2; }
+    __syncthreads();
+    if (threadIdx.x == 0) { K.k++; K.p_ready = false; }
+    apply_prec<R, MODE>(S, a.p, a.y, gen);                          // y = M^-1 p
+    const double rv = grid_sums<1>(krylov_ax<R, 1>(a.y, a.v, a.r0, nullptr)).a;   // v = A y
+    if (!(rv != 0.) || !isfinite(K.rho / rv)) break;
+    {
+      const double alpha = K.rho / rv;
+      if (threadIdx.x == 0) K.alpha = alpha;
+      const Sum3 sq = grid_sums<2>(krylov_s<R, MODE>(alpha));
+      if (threadIdx.x == 0) { K.ss = sq.a; K.r0s = sq.b; }
+      if (sqrt(sq.a) <= a.tol * K.normb) {
+        for (long i = t0; i < N; i += nt) a.x[i] = a.x[i] + alpha * a.y[i];
+        if (threadIdx.x == 0) K.resn = sqrt(sq.a);
+        break;
+      }
     }
-    double rv;
-    S.sum2(l0, 0., rv, dum);
-    if (!(rv != 0.) || !isfinite(rho / rv)) break;
-    alpha = rho / rv;
-    l0 = 0.; l1 = 0.;
-    for (long i = t0; i < N; i += nt) {
-      const double si = a.r[i] - alpha * a.v[i];
-      a.s[i] = si;
-      l0 += si * si;
-      l1 += a.r0[i] * si;
-      if (MODE == 1) x0v[i] = om0 * (R)si / ac0[i];
-    }
-    double ss, r0s;
-    S.sum2(l0, l1, ss, r0s);
-    if (sqrt(ss) <= a.tol * normb) {
-      for (long i = t0; i < N; i += nt) a.x[i] = a.x[i] + alpha * a.y[i];
-      resn = sqrt(ss);
-      break;
-    }
-    apply_prec<R, MODE>(S, a, a.s, a.z, gen);                       // z = M^-1 s
-    l0 = 0.; l1 = 0.; l2 = 0.;
-    for (long i = t0; i < N; i += 2 * nt) {
-      const long i2 = i + nt;
-      const bool h2 = i2 < N;
-      double t1, t2;
-      row_ax2(a, i, i2, h2, a.z, t1, t2);
-      a.t[i] = t1; l0 += t1 * a.s[i]; l1 += t1 * t1; l2 += a.r0[i] * t1;
-      if (h2) { a.t[i2] = t2; l0 += t2 * a.s[i2]; l1 += t2 * t2; l2 += a.r0[i2] * t2; }
-    }
-    double ts, tt, r0t;
-    S.sum3(l0, l1, l2, ts, tt, r0t);
+    apply_prec<R, MODE>(S, a.s, a.z, gen);                          // z = M^-1 s
+    const Sum3 tq = grid_sums<3>(krylov_ax<R, 3>(a.z, a.t, a.s, a.r0));   // t = A z
+    const double ts = tq.a, tt = tq.b, alpha = K.alpha;
     if (!(tt > 0.) || !(ts != 0.) || !isfinite(ts / tt)) {
       // t = A z vanished or is orthogonal to s: take the half step and stop
       for (long i = t0; i < N; i += nt) a.x[i] = a.x[i] + alpha * a.y[i];
-      resn = sqrt(ss);
+      if (threadIdx.x == 0) K.resn = sqrt(K.ss);
       break;
     }
-    omega = ts / tt;
-    const double rn_est = fmax(ss - omega * ts, 0.);
-    const double rho_est = r0s - omega * r0t;
-    if (k < a.maxit && sqrt(rn_est) > a.tol * normb && rho_est != 0. && isfinite(rho_est)) {
+    const double omega = ts / tt;
+    const double rn_est = fmax(K.ss - omega * ts, 0.);
+    const double rho_est = K.r0s - omega * tq.c;
+    if (K.k < a.maxit && sqrt(rn_est) > a.tol * K.normb && rho_est != 0. && isfinite(rho_est)) {
       // x and r of this iteration and p of the next in one pass
-      const double beta = (rho_est / rho) * (alpha / omega);
-      rho = rho_est;
-      for (long i = t0; i < N; i += nt) {
-        a.x[i] = a.x[i] + alpha * a.y[i] + omega * a.z[i];
-        const double ri = a.s[i] - omega * a.t[i];
-        a.r[i] = ri;
-        const double pi = ri + beta * (a.p[i] - omega * a.v[i]);
-        a.p[i] = pi;
-        if (MODE == 1) x0v[i] = om0 * (R)pi / ac0[i];
-      }
-      S.all();
-      resn = sqrt(rn_est);
-      p_ready = true;
+      krylov_xrp<R, MODE>(alpha, omega, (rho_est / K.rho) * (alpha / omega));
+      if (threadIdx.x == 0) { K.omega = omega; K.rho = rho_est; K.resn = sqrt(rn_est); K.p_ready = true; }
     } else {
       l0 = 0.; l1 = 0.;
       for (long i = t0; i < N; i += nt) {
@@ -1091,12 +1273,14 @@ __device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> a) {
         l0 += ri * ri;
         l1 += a.r0[i] * ri;
       }
-      double rn;
-      S.sum2(l0, l1, rn, rho_next);
-      resn = sqrt(rn);
+      double rn, r0r;
+      S.sum2(l0, l1, rn, r0r);
+      if (threadIdx.x == 0) { K.omega = omega; K.rho_next = r0r; K.resn = sqrt(rn); }
     }
+    __syncthreads();
   }
+  __syncthreads();
   S.all();
   for (long i = t0; i < N; i += nt) a.dphi[i] = a.x[i];
-  if (cta_id() == 0 && threadIdx.x == 0) { *a.iters = k; a.diag[0] = resn; a.diag[1] = normb; }
+  if (cta_id() == 0 && threadIdx.x == 0) { *a.iters = K.k; a.diag[0] = K.resn; a.diag[1] = K.normb; }
 }

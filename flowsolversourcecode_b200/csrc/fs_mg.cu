@@ -75,13 +75,13 @@ struct LevelDev {
 // One level of the V-cycle (fs_amg_core.cuh).  Rows of levels >= 1 are numbered
 // aggregate by aggregate, so the rows of coarse row P are [kp[P], kp[P+1]); row
 // a of level 0 is cell cells[a].  Off-diagonals: levels >= 1 in slices of 32
-// rows, slot j of row a at (sb[a/32] + j) * 32 + a % 32 (a slice as wide as its
-// widest row, padded with value 0 and the row itself); level 0 slot j at j * n
-// + a, columns in mesh order, unused slots -1.
+// rows, slot j of row a at (a/32 * w + j) * 32 + a % 32 (unused slots: value 0
+// and the row itself); level 0 slot j at j * n + a, columns in mesh order,
+// unused slots -1.
 template <class R>
 struct VcLevel {
   int n, w;
-  const int32_t *sb, *col, *cells;
+  const int32_t *col, *cells;
   const R *val, *ac;
   const int32_t *kp;
   R *b, *x, *r;
@@ -136,7 +136,7 @@ struct fs_mg_dev {
   // V-cycle layout (mg_vc_build): maps and index arrays, values per precision
   bool vc_map = false, vc_ready[2] = {false, false};
   std::vector<int32_t> h_nnb[FS_MG_MAXLEV], h_nbr[FS_MG_MAXLEV];   // coarse connectivity until then
-  int32_t *vsb[FS_MG_MAXLEV] = {}, *vcol[FS_MG_MAXLEV] = {}, *vmap[FS_MG_MAXLEV] = {}, *vrow[FS_MG_MAXLEV] = {};
+  int32_t *vcol[FS_MG_MAXLEV] = {}, *vmap[FS_MG_MAXLEV] = {}, *vrow[FS_MG_MAXLEV] = {};
   int32_t *vkp[FS_MG_MAXLEV] = {}, *par0 = nullptr;
   int vnpos[FS_MG_MAXLEV] = {};
   void *vval[2][FS_MG_MAXLEV] = {}, *vac[2][FS_MG_MAXLEV] = {}, *vb[2][FS_MG_MAXLEV] = {}, *vx[2][FS_MG_MAXLEV] = {};
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(FS_COOP_BLOCK, 1) k_guess_fit(AmgKArgs<R> a) {
 // right-preconditioned BiCGSTAB with the V-cycle on the whole cooperative grid
 // (amg_bicgstab_body in fs_amg_core.cuh)
 template <class R, int MODE>
-__global__ void __launch_bounds__(FS_COOP_BLOCK, FS_AMG_MINB) k_amg_bicgstab(AmgKArgs<R> a) {
+__global__ void __launch_bounds__(FS_COOP_BLOCK, FS_AMG_MINB) k_amg_bicgstab(const __grid_constant__ AmgKArgs<R> a) {
   g1::amg_bicgstab_body<R, MODE>(a);
 }
 
@@ -446,8 +446,7 @@ __global__ void __launch_bounds__(FS_COOP_BLOCK, FS_AMG_MINB)
     G.ncta = start[q + 1] - start[q];
   }
   __syncthreads();
-  const AmgKArgs<R> a = as[G.q];
-  gb::amg_bicgstab_body<R, MODE>(a);
+  gb::amg_bicgstab_body<R, MODE>(as[G.q]);
 }
 
 // the initial guesses of the batched solves, in the same CTA groups (a group
@@ -895,7 +894,7 @@ int fs_mg_free(fs_ctx *ctx) {
     for (void *x : p) if (x) cudaFree(x);
   }
   for (int q = 0; q < FS_MG_MAXLEV; q++) {
-    void *p[] = {M->vsb[q], M->vcol[q], M->vmap[q], M->vrow[q], M->vkp[q],
+    void *p[] = {M->vcol[q], M->vmap[q], M->vrow[q], M->vkp[q],
                  M->vval[0][q], M->vac[0][q], M->vb[0][q], M->vx[0][q], M->vval[1][q], M->vac[1][q], M->vb[1][q], M->vx[1][q]};
     for (void *x : p) if (x) cudaFree(x);
   }
@@ -985,22 +984,16 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
             map[dst] = nbr[src] >= 0 ? (int32_t)src : -1;
           }
       } else {
-        const int nsl = (n + 31) / 32;
-        std::vector<int32_t> sb(nsl + 1, 0);
-        for (int s = 0; s < nsl; s++) {
-          int wd = 0;
-          for (int a = 32 * s; a < std::min(n, 32 * s + 32); a++) wd = std::max(wd, (int)nnb[row[a]]);
-          sb[s + 1] = sb[s] + wd;
-        }
-        col.assign((size_t)sb[nsl] * 32, 0);
-        map.assign((size_t)sb[nsl] * 32, -1);
+        const int w = M->w[l];
+        const size_t np = (size_t)(n + 31) / 32 * 32 * w;
+        col.assign(np, 0);
+        map.assign(np, -1);
         for (int a = 0; a < n; a++)
-          for (int j = 0; j < sb[a / 32 + 1] - sb[a / 32]; j++) {
-            const size_t dst = ((size_t)sb[a / 32] + j) * 32 + a % 32, src = (size_t)j * n + row[a];
+          for (int j = 0; j < w; j++) {
+            const size_t dst = ((size_t)(a / 32) * w + j) * 32 + a % 32, src = (size_t)j * n + row[a];
             col[dst] = a;
             if (j < nnb[row[a]] && nbr[src] >= 0) { col[dst] = id[nbr[src]]; map[dst] = (int32_t)src; }
           }
-        if ((rc = upv(ctx, &M->vsb[l], sb))) return rc;
       }
       M->vnpos[l] = (int)col.size();
       if ((rc = upv(ctx, &M->vcol[l], col)) || (rc = upv(ctx, &M->vmap[l], map)) || (rc = upv(ctx, &M->vrow[l], row)))
@@ -1039,7 +1032,7 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
     for (int l = 0; l <= lc; l++) {
       VcLevel<R> &d = v.L[l];
       d.n = M->n[l]; d.w = M->w[l];
-      d.sb = M->vsb[l]; d.col = M->vcol[l]; d.cells = M->vrow[l];
+      d.col = M->vcol[l]; d.cells = M->vrow[l];
       d.val = (const R *)M->vval[f32][l]; d.ac = (const R *)M->vac[f32][l];
       d.kp = M->vkp[l];
       d.b = (R *)M->vb[f32][l]; d.x = l > 0 ? (R *)M->vx[f32][l] : nullptr;
