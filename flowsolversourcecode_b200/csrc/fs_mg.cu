@@ -122,28 +122,30 @@ struct AmgKArgs {
   int team_extra;     // fs_test_wait_timeout
 };
 
-// one array of the k_mg_layout launch: dst[q] = src[map[q]], 0 where map is -1
-struct LayoutSeg {
-  int block0, n;
-  const int32_t *map;
-  const double *src;
-  double *d64;
-  float *d32;
+// sums of a level's matrix entries that make up the next level's: entry q from
+// idx[ptr[q] .. ptr[q+1]), c >= 0 entry c of val, c < 0 row -1-c of ac
+struct CoarseSums {
+  int32_t *ptr = nullptr, *idx = nullptr;
 };
 
 struct fs_mg_dev {
   int nlev = 0;
   // V-cycle layout (mg_vc_build): maps and index arrays, values per precision
   bool vc_map = false, vc_ready[2] = {false, false};
-  std::vector<int32_t> h_nnb[FS_MG_MAXLEV], h_nbr[FS_MG_MAXLEV];   // coarse connectivity until then
-  int32_t *vcol[FS_MG_MAXLEV] = {}, *vmap[FS_MG_MAXLEV] = {}, *vrow[FS_MG_MAXLEV] = {};
-  int32_t *vkp[FS_MG_MAXLEV] = {}, *par0 = nullptr;
+  // coarse connectivity and child lists until then
+  std::vector<int32_t> h_nnb[FS_MG_MAXLEV], h_nbr[FS_MG_MAXLEV], h_cptr[FS_MG_MAXLEV], h_clist[FS_MG_MAXLEV];
+  int32_t *vcol[FS_MG_MAXLEV] = {}, *vrow[FS_MG_MAXLEV] = {}, *vkp[FS_MG_MAXLEV] = {}, *par0 = nullptr;
   int vnpos[FS_MG_MAXLEV] = {};
-  void *vval[2][FS_MG_MAXLEV] = {}, *vac[2][FS_MG_MAXLEV] = {}, *vb[2][FS_MG_MAXLEV] = {}, *vx[2][FS_MG_MAXLEV] = {};
+  CoarseSums csum[FS_MG_MAXLEV], cdiag[FS_MG_MAXLEV];   // level l's entries and diagonals from level l-1
+  // matrices in the layout: FP64 of every level, FP32 copies where the V-cycle is FP32; vectors per precision
+  double *vval[FS_MG_MAXLEV] = {}, *vac[FS_MG_MAXLEV] = {};
+  float *vvalf[FS_MG_MAXLEV] = {}, *vacf[FS_MG_MAXLEV] = {};
+  void *vb[2][FS_MG_MAXLEV] = {}, *vx[2][FS_MG_MAXLEV] = {};
+  unsigned *vbar[2] = {nullptr, nullptr};            // barrier counts, partial sums and coarsest inverse
+  double *vpart[2] = {nullptr, nullptr}, *vinv[2] = {nullptr, nullptr};
+  std::vector<void *> vallocs;
   VcDev<double> *vc64 = nullptr;
   VcDev<float> *vc32 = nullptr;
-  LayoutSeg *seg[2] = {nullptr, nullptr};   // k_mg_layout tables in FP64, FP32; level 0 first
-  int nseg = 0, seg_blocks = 0, nseg0 = 0, seg0_blocks = 0;
   unsigned *gridbar = nullptr;
   int n[FS_MG_MAXLEV] = {}, w[FS_MG_MAXLEV] = {}, ncol[FS_MG_MAXLEV] = {};
   std::vector<int32_t> h_parent[FS_MG_MAXLEV];
@@ -561,28 +563,38 @@ __global__ void k_to_f32(long n, const double *a, float *b) {
   if (i < n) b[i] = (float)a[i];
 }
 
-// Dense inverse of the coarsest level (one CTA, matrix in shared memory):
-// in-place Gauss-Jordan without pivoting, two block barriers per pivot.  The
-// agglomerated matrices are diagonally dominant.  A pure-Neumann level (every
-// row sum ~0: the pressure correction with walls only) is singular with the
-// constant null space; its last equation is replaced by x_{n-1} = 0 and the last
-// column of the inverse is zeroed, so sinv*b solves the remaining equations --
-// the consistent systems the V-cycle restricts.  A zero pivot drops its unknown.
-__global__ void __launch_bounds__(1024) k_mg_dense_inverse(int n, const int32_t *ncf, const int32_t *nbr,
-                                                           const double *ac, const double *anb, double *sinv) {
-  extern __shared__ double sm[];
-  double *A = sm, *col = sm + (long)n * n;
+// Dense inverse of the coarsest level (one CTA of 16 warps, n <= 32 CT): in-place
+// Gauss-Jordan without pivoting, one block barrier per pivot.  Warp y holds
+// rows y + 16 a, lane x columns x + 32 b in registers; the pivot row and column
+// of step k, and the pivot's reciprocal, are read from buffers (by the parity
+// of k) that the update of step k-1 filled.  With the matrix in shared memory a
+// pivot moved 24 bytes per entry through it and took 4 us at n = 157 (0.60 ms in
+// all, a quarter of the 64x64 cavity's p' solve); every entry goes through the
+// same operations.
+// The agglomerated matrices are diagonally dominant.  A pure-Neumann level
+// (every row sum ~0: the pressure correction with walls only) is singular with
+// the constant null space; its last equation is replaced by x_{n-1} = 0 and the
+// last column of the inverse is zeroed, so sinv*b solves the remaining
+// equations -- the consistent systems the V-cycle restricts.  A zero pivot
+// drops its unknown.
+template <int CT>
+__global__ void __launch_bounds__(512, 1) k_mg_dense_inverse(int n, int w, const int32_t *nbr, const double *ac,
+                                                             const double *anb, bool sliced, double *sinv) {
+  constexpr int RT = 2 * CT;
+  extern __shared__ double A[];
+  __shared__ double prow[2][32 * CT], pcol[2][32 * CT], pinv[2];
   __shared__ int singular;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5;
   for (int q = tid; q < n * n; q += nt) A[q] = 0.;
   if (tid == 0) singular = 1;
   __syncthreads();
   for (int i = tid; i < n; i += nt) {
     double d = ac[i], rs = d;
     A[(long)i * n + i] = d;
-    for (int j = 0; j < ncf[i]; j++) {
-      int k = nbr[(long)j * n + i];
-      if (k >= 0) { double a = anb[(long)j * n + i]; A[(long)i * n + k] += a; rs += a; }
+    for (int j = 0; j < w; j++) {
+      const long q = sliced ? ((long)(i >> 5) * w + j) * 32 + (i & 31) : (long)j * n + i;
+      const int k = nbr[q];
+      if (k >= 0 && k != i) { double a = anb[q]; A[(long)i * n + k] += a; rs += a; }
     }
     if (fabs(rs) > 1e-9 * fabs(d)) singular = 0;
   }
@@ -591,52 +603,110 @@ __global__ void __launch_bounds__(1024) k_mg_dense_inverse(int n, const int32_t 
   if (sing)
     for (int j = tid; j < n; j += nt) A[(long)(n - 1) * n + j] = j == n - 1 ? 1. : 0.;
   __syncthreads();
-  // warps take rows, lanes take columns.  The pivot row and column of step k
-  // are read from buffers (prow/pcol, double-buffered by the parity of k) that
-  // the update of step k-1 filled, so one block barrier per pivot suffices;
-  // every entry goes through the same operations as an in-place elimination.
-  const int lane = tid & 31, wid = tid >> 5, nwarp = nt >> 5;
-  double *prow = col + n, *pcol = prow + 2 * n;   // [2][n] each
-  for (int j = tid; j < n; j += nt) { prow[j] = A[j]; pcol[j] = A[(long)j * n]; }
+  double v[RT][CT];
+#pragma unroll
+  for (int a = 0; a < RT; a++)
+#pragma unroll
+    for (int b = 0; b < CT; b++) {
+      const int i = wid + 16 * a, j = lane + 32 * b;
+      v[a][b] = i < n && j < n ? A[(long)i * n + j] : 0.;
+    }
+  for (int j = tid; j < n; j += nt) { prow[0][j] = A[j]; pcol[0][j] = A[(long)j * n]; }
+  if (tid == 0) pinv[0] = A[0] != 0. ? 1. / A[0] : 0.;
   __syncthreads();
   for (int k = 0; k < n; k++) {
-    const int b = k & 1;
-    const double *pr = prow + b * n, *pc = pcol + b * n;
-    double *nr = prow + (b ^ 1) * n, *nc = pcol + (b ^ 1) * n;
-    const double d = pr[k];
-    const double p = d != 0. ? 1. / d : 0.;
-    for (int i = wid; i < n; i += nwarp) {
-      double *ri = A + (long)i * n;
-      const double ci = pc[i];
-      for (int j = lane; j < n; j += 32) {
-        const double rkj = j == k ? p : pr[j] * p;
-        double v;
-        if (i == k) v = rkj;
-        else v = j == k ? -ci * p : ri[j] - ci * rkj;
-        ri[j] = v;
-        if (i == k + 1) nr[j] = v;
-        if (j == k + 1) nc[i] = v;
+    const int c = k & 1, d = c ^ 1;
+    const double p = pinv[c];
+    double rk[CT];
+#pragma unroll
+    for (int b = 0; b < CT; b++) {
+      const int j = lane + 32 * b;
+      rk[b] = j == k ? p : j < n ? prow[c][j] * p : 0.;
+    }
+#pragma unroll
+    for (int a = 0; a < RT; a++) {
+      const int i = wid + 16 * a;
+      if (i < n) {
+        const double ci = pcol[c][i];
+#pragma unroll
+        for (int b = 0; b < CT; b++) {
+          const int j = lane + 32 * b;
+          const double u = i == k ? rk[b] : j == k ? -ci * p : v[a][b] - ci * rk[b];
+          v[a][b] = u;
+          if (j == k + 1) {
+            pcol[d][i] = u;
+            if (i == k + 1) pinv[d] = u != 0. ? 1. / u : 0.;
+          }
+          if (i == k + 1 && j < n) prow[d][j] = u;
+        }
       }
     }
     __syncthreads();
   }
-  if (sing)
-    for (int i = tid; i < n; i += nt) A[(long)i * n + n - 1] = 0.;
-  __syncthreads();
-  for (int q = tid; q < n * n; q += nt) sinv[q] = A[q];
+#pragma unroll
+  for (int a = 0; a < RT; a++)
+#pragma unroll
+    for (int b = 0; b < CT; b++) {
+      const int i = wid + 16 * a, j = lane + 32 * b;
+      if (i < n && j < n) sinv[(long)i * n + j] = sing && j == n - 1 ? 0. : v[a][b];
+    }
 }
 
-// the levels' matrices into the V-cycle's layout and precision
-__global__ void k_mg_layout(const LayoutSeg *__restrict__ segs, int nseg) {
-  int k = 0;
-  while (k + 1 < nseg && (int)blockIdx.x >= segs[k + 1].block0) k++;
-  const LayoutSeg g = segs[k];
-  const int q = ((int)blockIdx.x - g.block0) * blockDim.x + threadIdx.x;
-  if (q >= g.n) return;
-  const int m = g.map[q];
-  const double v = m >= 0 ? g.src[m] : 0.;
-  if (g.d64) g.d64[q] = v;
-  else g.d32[q] = (float)v;
+// level 0 into the V-cycle's layout (row a is cell cells[a]; FP64, and FP32 when
+// that is the cycle's precision, then with an FP32 copy in mesh order too).
+// Unused slots are copied as they are: no one reads them.
+__global__ void k_mg_level0(int n, int w, const int32_t *__restrict__ cells, const double *__restrict__ ac,
+                            const double *__restrict__ anb, double *__restrict__ acL, double *__restrict__ anbL,
+                            float *__restrict__ acLf, float *__restrict__ anbLf, float *__restrict__ acf,
+                            float *__restrict__ anbf) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= n) return;
+  const long i = cells[a];
+  const double d = ac[i];
+  acL[a] = d;
+  if (acf) { acLf[a] = (float)d; acf[a] = (float)ac[a]; }
+  for (int j = 0; j < w; j++) {
+    const double v = anb[(long)j * n + i];
+    anbL[(long)j * n + a] = v;
+    if (acf) { anbLf[(long)j * n + a] = (float)v; anbf[(long)j * n + a] = (float)anb[(long)j * n + a]; }
+  }
+}
+
+// the next level's matrix (AssembleElementBasedAgglomoratedLHS.for:45-150) in
+// the V-cycle's layout: a thread per entry, then per diagonal, sums its static
+// list -- the children in list order, each child's diagonal then its slots --
+// so every entry is summed in the reference's order.  The rows of an
+// aggregate are consecutive in the layout, so neighbouring threads gather from
+// neighbouring lines; a thread per coarse row over the mesh-ordered matrix
+// (k_mg_lhs) reads a sector per value.
+__global__ void k_mg_coarse(int npos, int n, const int32_t *__restrict__ ptr, const int32_t *__restrict__ idx,
+                            const int32_t *__restrict__ dptr, const int32_t *__restrict__ didx,
+                            const double *__restrict__ acF, const double *__restrict__ anbF, double *__restrict__ acC,
+                            double *__restrict__ anbC, float *__restrict__ acCf, float *__restrict__ anbCf) {
+  int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool diag = q >= npos;
+  if (diag) q -= npos;
+  if (diag && q >= n) return;
+  const int32_t *pp = diag ? dptr : ptr, *ii = diag ? didx : idx;
+  const int c1 = pp[q + 1];
+  double t = 0.;
+  for (int c = pp[q]; c < c1; c += 4) {
+    int e[4];
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) e[u] = c + u < c1 ? ii[c + u] : 0;
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = c + u < c1 ? (e[u] >= 0 ? anbF[e[u]] : acF[-1 - e[u]]) : 0.;
+#pragma unroll
+    for (int u = 0; u < 4; u++) if (c + u < c1) t = t + v[u];
+  }
+  if (diag) {
+    acC[q] = t;
+    if (acCf) acCf[q] = (float)t;
+  } else {
+    anbC[q] = t;
+    if (anbCf) anbCf[q] = (float)t;
+  }
 }
 
 }  // namespace
@@ -855,7 +925,10 @@ int fs_mg_build(fs_ctx *ctx) {
   FS_CK(cudaMemcpy(M->lev32, L32.data(), sizeof(LevelDev<float>) * M->nlev, cudaMemcpyHostToDevice));
   FS_CK(cudaMalloc(&M->red, sizeof(double) * (6 + FS_SUMK + 9) * FS_RED_BLOCKS));
   FS_CK(cudaMalloc(&M->gridbar, sizeof(unsigned) * FS_GRIDBAR_WORDS));
-  for (int q = 1; q < M->nlev; q++) { M->h_nnb[q] = std::move(H[q].nnb); M->h_nbr[q] = std::move(H[q].nbr); }
+  for (int q = 1; q < M->nlev; q++) {
+    M->h_nnb[q] = std::move(H[q].nnb); M->h_nbr[q] = std::move(H[q].nbr);
+    M->h_cptr[q] = std::move(cptr[q - 1]); M->h_clist[q] = std::move(clist[q - 1]);
+  }
   // preconditioner: stop at the first level small enough for the dense inverse
   M->lc = M->nlev - 1;
   for (int q = 0; q < M->nlev; q++)
@@ -866,8 +939,11 @@ int fs_mg_build(fs_ctx *ctx) {
     FS_CK(cudaMalloc(&M->sinv, sizeof(double) * nn));
     // the attribute belongs to the function, shared by every context of the
     // process: set it for the largest coarsest level any context may have
-    FS_CK(cudaFuncSetAttribute((const void *)k_mg_dense_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(sizeof(double) * ((size_t)FS_MG_DIRECT * FS_MG_DIRECT + 5 * FS_MG_DIRECT))));
+    const int sm = (int)(sizeof(double) * FS_MG_DIRECT * FS_MG_DIRECT);
+    const void *ks[] = {(const void *)k_mg_dense_inverse<1>, (const void *)k_mg_dense_inverse<2>,
+                        (const void *)k_mg_dense_inverse<3>, (const void *)k_mg_dense_inverse<4>,
+                        (const void *)k_mg_dense_inverse<5>};
+    for (const void *k : ks) FS_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   }
   // cooperative grid: smallest co-resident count of the three kernels, <= 4 CTAs/SM
   int a = 0, b = 0, c = 0;
@@ -894,12 +970,12 @@ int fs_mg_free(fs_ctx *ctx) {
     for (void *x : p) if (x) cudaFree(x);
   }
   for (int q = 0; q < FS_MG_MAXLEV; q++) {
-    void *p[] = {M->vcol[q], M->vmap[q], M->vrow[q], M->vkp[q],
-                 M->vval[0][q], M->vac[0][q], M->vb[0][q], M->vx[0][q], M->vval[1][q], M->vac[1][q], M->vb[1][q], M->vx[1][q]};
+    void *p[] = {M->vcol[q], M->vrow[q], M->vkp[q], M->csum[q].ptr, M->csum[q].idx, M->cdiag[q].ptr, M->cdiag[q].idx};
     for (void *x : p) if (x) cudaFree(x);
   }
+  for (void *x : M->vallocs) cudaFree(x);
   cudaFree(M->par0);
-  cudaFree(M->vc64); cudaFree(M->vc32); cudaFree(M->seg[0]); cudaFree(M->seg[1]); cudaFree(M->gridbar);
+  cudaFree(M->vc64); cudaFree(M->vc32); cudaFree(M->gridbar);
   cudaFree(M->lev64); cudaFree(M->lev32); cudaFree(M->red); cudaFree(M->sinv);
   delete M;
   ctx->mg = nullptr;
@@ -936,6 +1012,77 @@ static int mg_coarse_matrices(fs_ctx *ctx, int last, bool f32) {
   return FS_OK;
 }
 
+// the coarsest level's dense inverse (sliced: the V-cycle's layout, whose unused
+// slots hold 0 and the row itself; else slot-major, unused slots -1)
+static int dense_inverse(fs_ctx *ctx, int n, int w, const int32_t *nbr, const double *ac, const double *anb, bool sliced,
+                         double *sinv) {
+  const size_t sm = sizeof(double) * (size_t)n * n;
+  const int ct = (n + 31) / 32;
+#define FS_INV(CT) k_mg_dense_inverse<CT><<<1, 512, sm, ctx->st>>>(n, w, nbr, ac, anb, sliced, sinv)
+  if (ct <= 1) FS_INV(1);
+  else if (ct == 2) FS_INV(2);
+  else if (ct == 3) FS_INV(3);
+  else if (ct == 4) FS_INV(4);
+  else FS_INV(5);
+#undef FS_INV
+  FS_LAUNCH_CHECK();
+  return FS_OK;
+}
+
+// position of slot j of row a in level l's layout
+static size_t vc_pos(int l, int n, int w, int a, int j) {
+  return l == 0 ? (size_t)j * n + a : ((size_t)(a / 32) * w + j) * 32 + a % 32;
+}
+
+// the entries of level l-1 that each entry and diagonal of level l sums, in the
+// reference's order (children in list order, a child's diagonal, then its slots)
+static int mg_vc_sums(fs_ctx *ctx, int l, const std::vector<int32_t> &idf, const std::vector<int32_t> &idc) {
+  fs_mg_dev *M = ctx->mg;
+  const int n = M->n[l - 1], w = M->w[l - 1], nc = M->n[l], wc = M->w[l];
+  const std::vector<int32_t> &nnb = l > 1 ? M->h_nnb[l - 1] : ctx->h_ncf, &nbr = l > 1 ? M->h_nbr[l - 1] : ctx->h_cn;
+  const std::vector<int32_t> &par = M->h_parent[l - 1], &cnn = M->h_nnb[l], &cnb = M->h_nbr[l];
+  const std::vector<int32_t> &cptr = M->h_cptr[l], &clist = M->h_clist[l];
+  const size_t np = M->vnpos[l];
+  std::vector<int32_t> ptr(np + 1, 0), dptr(nc + 1, 0), slot((size_t)n * w, -1);
+  // pass 1: the coarse slot of every fine slot (-2 inside the aggregate), counts
+  for (int P = 0; P < nc; P++) {
+    const int p = idc[P];
+    for (int q = cptr[P]; q < cptr[P + 1]; q++) {
+      const int c = clist[q];
+      dptr[p + 1]++;
+      for (int j = 0; j < nnb[c]; j++) {
+        const int k = nbr[(size_t)j * n + c];
+        if (k < 0) continue;
+        const int Q = par[k];
+        if (Q == P) { slot[(size_t)j * n + c] = -2; dptr[p + 1]++; continue; }
+        for (int m = 0; m < cnn[P]; m++)
+          if (cnb[(size_t)m * nc + P] == Q) { slot[(size_t)j * n + c] = m; ptr[vc_pos(l, nc, wc, p, m) + 1]++; break; }
+      }
+    }
+  }
+  for (size_t q = 0; q < np; q++) ptr[q + 1] += ptr[q];
+  for (int p = 0; p < nc; p++) dptr[p + 1] += dptr[p];
+  std::vector<int32_t> idx(ptr[np]), didx(dptr[nc]), at(ptr.begin(), ptr.end() - 1), dat(dptr.begin(), dptr.end() - 1);
+  for (int P = 0; P < nc; P++) {
+    const int p = idc[P];
+    for (int q = cptr[P]; q < cptr[P + 1]; q++) {
+      const int c = clist[q], a = idf[c];
+      didx[dat[p]++] = -1 - a;
+      for (int j = 0; j < nnb[c]; j++) {
+        const int t = slot[(size_t)j * n + c];
+        const int32_t e = (int32_t)vc_pos(l - 1, n, w, a, j);
+        if (t == -2) didx[dat[p]++] = e;
+        else if (t >= 0) idx[at[vc_pos(l, nc, wc, p, t)]++] = e;
+      }
+    }
+  }
+  int rc;
+  if ((rc = upv(ctx, &M->csum[l].ptr, ptr)) || (rc = upv(ctx, &M->csum[l].idx, idx)) ||
+      (rc = upv(ctx, &M->cdiag[l].ptr, dptr)) || (rc = upv(ctx, &M->cdiag[l].idx, didx)))
+    return rc;
+  return FS_OK;
+}
+
 // ---------------------------------------------------------------- V-cycle layout
 // Once per context: levels 1 .. lc-1 renumbered aggregate by aggregate (the
 // coarsest keeps its numbering, so its dense inverse is used as it is; within
@@ -949,6 +1096,7 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
   int rc;
   if (!M->vc_map) {
     std::vector<int32_t> up(M->n[lc]), id;   // new numbers of the coarser level, of this one
+    std::vector<std::vector<int32_t>> ids(lc + 1);
     for (int i = 0; i < M->n[lc]; i++) up[i] = i;
     for (int l = lc; l >= 0; l--) {
       const int n = M->n[l];
@@ -972,59 +1120,84 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
         }
       }
       for (int i = 0; i < n; i++) row[id[i]] = i;
-      std::vector<int32_t> col, map;
+      std::vector<int32_t> col;
+      const int w = M->w[l];
       if (l == 0) {
-        const int w = M->w[0];
         col.resize((size_t)w * n);
-        map.resize((size_t)w * n);
         for (int j = 0; j < w; j++)
-          for (int a = 0; a < n; a++) {
-            const size_t src = (size_t)j * n + row[a], dst = (size_t)j * n + a;
-            col[dst] = nbr[src];
-            map[dst] = nbr[src] >= 0 ? (int32_t)src : -1;
-          }
+          for (int a = 0; a < n; a++) col[(size_t)j * n + a] = nbr[(size_t)j * n + row[a]];
       } else {
-        const int w = M->w[l];
-        const size_t np = (size_t)(n + 31) / 32 * 32 * w;
-        col.assign(np, 0);
-        map.assign(np, -1);
+        col.assign((size_t)(n + 31) / 32 * 32 * w, 0);
         for (int a = 0; a < n; a++)
           for (int j = 0; j < w; j++) {
-            const size_t dst = ((size_t)(a / 32) * w + j) * 32 + a % 32, src = (size_t)j * n + row[a];
-            col[dst] = a;
-            if (j < nnb[row[a]] && nbr[src] >= 0) { col[dst] = id[nbr[src]]; map[dst] = (int32_t)src; }
+            const size_t src = (size_t)j * n + row[a];
+            col[((size_t)(a / 32) * w + j) * 32 + a % 32] = j < nnb[row[a]] && nbr[src] >= 0 ? id[nbr[src]] : a;
           }
       }
       M->vnpos[l] = (int)col.size();
-      if ((rc = upv(ctx, &M->vcol[l], col)) || (rc = upv(ctx, &M->vmap[l], map)) || (rc = upv(ctx, &M->vrow[l], row)))
-        return rc;
+      if ((rc = upv(ctx, &M->vcol[l], col)) || (rc = upv(ctx, &M->vrow[l], row))) return rc;
+      ids[l] = id;
       up.swap(id);
     }
-    for (int q = 0; q < M->nlev; q++) { M->h_nnb[q] = std::vector<int32_t>(); M->h_nbr[q] = std::vector<int32_t>(); }
+    for (int l = 1; l <= lc; l++)
+      if ((rc = mg_vc_sums(ctx, l, ids[l - 1], ids[l]))) return rc;
+    for (int q = 0; q < M->nlev; q++) {
+      M->h_nnb[q] = std::vector<int32_t>(); M->h_nbr[q] = std::vector<int32_t>();
+      M->h_cptr[q] = std::vector<int32_t>(); M->h_clist[q] = std::vector<int32_t>();
+    }
     M->vc_map = true;
   }
+  // What the cycle touches of the levels >= 1 goes into one block, the coarsest
+  // level first, with the barrier count and the partial sums: the small levels
+  // share a few pages instead of one allocation (and page) per array.
   const size_t es = f32 ? sizeof(float) : sizeof(double);
-  std::vector<LayoutSeg> segs;
-  int blocks = 0;
-  auto seg = [&](int n, const int32_t *map, const double *src, void *dst) {
-    LayoutSeg g{};
-    g.block0 = blocks; g.n = n; g.map = map; g.src = src;
-    (f32 ? (void *&)g.d32 : (void *&)g.d64) = dst;
-    blocks += fs_grid(n);
-    segs.push_back(g);
+  const size_t nparts = (9 + FS_SUMK) * (size_t)FS_RED_BLOCKS;
+  char *base = nullptr;
+  size_t off = 0;
+  auto take = [&](size_t bytes) -> void * {
+    void *q = base ? base + off : nullptr;
+    off += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+    return q;
   };
-  for (int l = 0; l <= lc; l++) {
-    FS_CK(cudaMalloc(&M->vval[f32][l], es * std::max(1, M->vnpos[l])));
-    FS_CK(cudaMalloc(&M->vac[f32][l], es * M->n[l]));
-    seg(M->vnpos[l], M->vmap[l], M->anb[l], M->vval[f32][l]);
-    seg(M->n[l], M->vrow[l], M->ac[l], M->vac[f32][l]);
-    if (l == 0) { M->nseg0 = (int)segs.size(); M->seg0_blocks = blocks; }
-    FS_CK(cudaMalloc(&M->vx[f32][l], es * M->n[l == 0 ? 1 : l]));   // [0]: the result of level 1
-    if (l > 0) FS_CK(cudaMalloc(&M->vb[f32][l], es * M->n[l]));
+  int32_t *kp[FS_MG_MAXLEV] = {}, *col[FS_MG_MAXLEV] = {};
+  void *val[FS_MG_MAXLEV] = {}, *ac[FS_MG_MAXLEV] = {}, *r[FS_MG_MAXLEV] = {};
+  const double *sinv = nullptr;
+  for (int pass = 0; pass < 2; pass++) {
+    if (pass == 1) { FS_CK(cudaMalloc((void **)&base, off)); M->vallocs.push_back(base); }
+    off = 0;
+    M->vbar[f32] = (unsigned *)take(sizeof(unsigned) * FS_GRIDBAR_WORDS);
+    M->vpart[f32] = (double *)take(sizeof(double) * nparts);
+    double *si = (double *)take(sizeof(double) * M->n[lc] * M->n[lc]);
+    sinv = si;
+    M->vinv[f32] = si;
+    for (int l = lc; l >= 1; l--) {
+      ac[l] = take(es * M->n[l]);
+      M->vb[f32][l] = take(es * M->n[l]);
+      M->vx[f32][l] = take(es * M->n[l]);
+      r[l] = take(es * M->n[l]);
+      if (l < lc) kp[l] = (int32_t *)take(sizeof(int32_t) * (M->n[l + 1] + 1));
+      col[l] = (int32_t *)take(sizeof(int32_t) * M->vnpos[l]);
+      val[l] = take(es * M->vnpos[l]);
+    }
+    M->vx[f32][0] = take(es * M->n[1]);   // the result of level 1
   }
-  M->nseg = (int)segs.size(); M->seg_blocks = blocks;
-  FS_CK(cudaMalloc(&M->seg[f32], sizeof(LayoutSeg) * segs.size()));
-  FS_CK(cudaMemcpy(M->seg[f32], segs.data(), sizeof(LayoutSeg) * segs.size(), cudaMemcpyHostToDevice));
+  for (int l = 1; l <= lc; l++) {
+    if (l < lc) FS_CK(cudaMemcpy(kp[l], M->vkp[l], sizeof(int32_t) * (M->n[l + 1] + 1), cudaMemcpyDeviceToDevice));
+    FS_CK(cudaMemcpy(col[l], M->vcol[l], sizeof(int32_t) * M->vnpos[l], cudaMemcpyDeviceToDevice));
+  }
+  auto own = [&](auto **d, size_t n) -> int {
+    FS_CK(cudaMalloc((void **)d, sizeof(**d) * std::max<size_t>(n, 1)));
+    M->vallocs.push_back(*d);
+    return FS_OK;
+  };
+  kp[0] = M->vkp[0]; col[0] = M->vcol[0];
+  for (int l = 0; l <= lc; l++) {   // the FP64 matrices are the source of the next level's in either precision
+    if (!f32 && l > 0 && !M->vval[l]) { M->vval[l] = (double *)val[l]; M->vac[l] = (double *)ac[l]; }
+    if (!M->vval[l] && ((rc = own(&M->vval[l], M->vnpos[l])) || (rc = own(&M->vac[l], M->n[l])))) return rc;
+    if (f32 && l > 0) { M->vvalf[l] = (float *)val[l]; M->vacf[l] = (float *)ac[l]; }
+    if (f32 && l == 0 && ((rc = own(&M->vvalf[l], M->vnpos[l])) || (rc = own(&M->vacf[l], M->n[l])))) return rc;
+  }
+  r[0] = f32 ? (void *)M->rf[0] : (void *)M->r[0];
   auto desc = [&](auto *tag, auto **dev, const LevelDev<std::remove_pointer_t<decltype(tag)>> *levs) -> int {
     using R = std::remove_pointer_t<decltype(tag)>;
     VcDev<R> v{};
@@ -1032,14 +1205,15 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
     for (int l = 0; l <= lc; l++) {
       VcLevel<R> &d = v.L[l];
       d.n = M->n[l]; d.w = M->w[l];
-      d.col = M->vcol[l]; d.cells = M->vrow[l];
-      d.val = (const R *)M->vval[f32][l]; d.ac = (const R *)M->vac[f32][l];
-      d.kp = M->vkp[l];
+      d.col = col[l]; d.cells = M->vrow[l];
+      d.val = f32 ? (const R *)(void *)M->vvalf[l] : (const R *)(void *)M->vval[l];
+      d.ac = f32 ? (const R *)(void *)M->vacf[l] : (const R *)(void *)M->vac[l];
+      d.kp = kp[l];
       d.b = (R *)M->vb[f32][l]; d.x = l > 0 ? (R *)M->vx[f32][l] : nullptr;
-      d.r = (R *)(f32 ? (void *)M->rf[l] : (void *)M->r[l]);
+      d.r = (R *)r[l];
     }
     v.x1 = (R *)M->vx[f32][0];
-    v.sinv = M->sinv;
+    v.sinv = sinv;
     FS_CK(cudaMemcpy(&v.L0, levs, sizeof(LevelDev<R>), cudaMemcpyDeviceToHost));
     v.par0 = M->par0;
     FS_CK(cudaMalloc(dev, sizeof(VcDev<R>)));
@@ -1058,9 +1232,16 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
 // coarse levels being kept)
 static int mg_vc_values(fs_ctx *ctx, bool f32, bool level0) {
   fs_mg_dev *M = ctx->mg;
-  k_mg_layout<<<level0 ? M->seg0_blocks : M->seg_blocks, FS_BLOCK, 0, ctx->st>>>(M->seg[f32],
-                                                                             level0 ? M->nseg0 : M->nseg);
+  k_mg_level0<<<fs_grid(M->n[0]), FS_BLOCK, 0, ctx->st>>>(
+      M->n[0], M->w[0], M->vrow[0], M->ac[0], M->anb[0], M->vac[0], M->vval[0], f32 ? M->vacf[0] : nullptr,
+      f32 ? M->vvalf[0] : nullptr, f32 ? M->acf[0] : nullptr, f32 ? M->anbf[0] : nullptr);
   FS_LAUNCH_CHECK();
+  for (int l = 1; l <= M->lc && !level0; l++) {
+    k_mg_coarse<<<fs_grid((long)M->vnpos[l] + M->n[l]), FS_BLOCK, 0, ctx->st>>>(
+        M->vnpos[l], M->n[l], M->csum[l].ptr, M->csum[l].idx, M->cdiag[l].ptr, M->cdiag[l].idx, M->vac[l - 1],
+        M->vval[l - 1], M->vac[l], M->vval[l], f32 ? M->vacf[l] : nullptr, f32 ? M->vvalf[l] : nullptr);
+    FS_LAUNCH_CHECK();
+  }
   return FS_OK;
 }
 
@@ -1101,29 +1282,29 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   if (vc && (rc = mg_vc_build(ctx, f32))) return rc;
   const int refresh = std::max(1, ctx->cfg.pc_refresh);
   const bool reuse = M->built_nf == nf && M->built_f32 == f32 && M->age + 1 < refresh;
-  if (reuse) {
-    M->age++;
-    if (f32) {   // level 0 in FP32 from the current system
-      const long n = M->n[0], nw = (long)M->w[0] * M->n[0];
-      k_to_f32<<<fs_grid(n), FS_BLOCK, 0, ctx->st>>>(n, M->ac[0], M->acf[0]);
-      FS_LAUNCH_CHECK();
-      k_to_f32<<<fs_grid(nw), FS_BLOCK, 0, ctx->st>>>(nw, M->anb[0], M->anbf[0]);
-      FS_LAUNCH_CHECK();
-    }
-  } else {
+  if (reuse) M->age++;
+  else { M->built_nf = nf; M->built_f32 = f32; M->age = 0; }
+  if (vc) {
+    if ((rc = mg_vc_values(ctx, f32, reuse))) return rc;
+  } else if (!reuse) {
     if ((rc = mg_coarse_matrices(ctx, M->lc, f32))) return rc;
-    M->built_nf = nf; M->built_f32 = f32; M->age = 0;
+  } else if (f32) {   // level 0 in FP32 from the current system
+    const long n = M->n[0], nw = (long)M->w[0] * M->n[0];
+    k_to_f32<<<fs_grid(n), FS_BLOCK, 0, ctx->st>>>(n, M->ac[0], M->acf[0]);
+    FS_LAUNCH_CHECK();
+    k_to_f32<<<fs_grid(nw), FS_BLOCK, 0, ctx->st>>>(nw, M->anb[0], M->anbf[0]);
+    FS_LAUNCH_CHECK();
   }
   // team-barrier counters of the V-cycle start at zero for every launch
   FS_CK(cudaMemsetAsync(ctx->d_status + 4, 0, sizeof(int32_t) * 2, ctx->st));
-  FS_CK(cudaMemsetAsync(M->gridbar, 0, sizeof(unsigned) * FS_GRIDBAR_WORDS, ctx->st));
+  unsigned *gridbar = vc ? M->vbar[f32] : M->gridbar;
+  FS_CK(cudaMemsetAsync(gridbar, 0, sizeof(unsigned) * FS_GRIDBAR_WORDS, ctx->st));
   if (M->direct && !reuse) {
-    const int n = M->n[M->lc];
-    k_mg_dense_inverse<<<1, 1024, sizeof(double) * ((size_t)n * n + 5 * (size_t)n), ctx->st>>>(
-        n, M->nnb[M->lc], M->nbr[M->lc], M->ac[M->lc], M->anb[M->lc], M->sinv);
-    FS_LAUNCH_CHECK();
+    const int q = M->lc;
+    if ((rc = vc ? dense_inverse(ctx, M->n[q], M->w[q], M->vcol[q], M->vac[q], M->vval[q], true, M->vinv[f32])
+                 : dense_inverse(ctx, M->n[q], M->w[q], M->nbr[q], M->ac[q], M->anb[q], false, M->sinv)))
+      return rc;
   }
-  if (vc && (rc = mg_vc_values(ctx, f32, reuse))) return rc;
   auto fill = [&](auto &a) {
     a.N = ctx->N; a.W = ctx->W; a.ncf = ctx->ncf; a.cn = ctx->cn; a.ac = ctx->ac; a.anb = ctx->anb; a.bc = ctx->bc;
     a.x = ctx->kx; a.r = ctx->kr; a.r0 = ctx->kr0; a.p = ctx->kp; a.v = ctx->kv; a.s = ctx->ks; a.t = ctx->kt;
@@ -1131,14 +1312,14 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
     // one V-cycle per application: one pre- and one post-sweep (MultiGridpreSweep)
     a.lc = M->lc; a.direct = M->direct; a.sinv = M->sinv;
     a.pre = std::max(1, ctx->cfg.mg_pre); a.post = std::max(1, ctx->cfg.mg_pre);
-    a.maxit = ctx->cfg.krylov_maxit; a.tol = ctx->cfg.krylov_tol; a.part = M->red;
+    a.maxit = ctx->cfg.krylov_maxit; a.tol = ctx->cfg.krylov_tol; a.part = vc ? M->vpart[f32] : M->red;
     a.iters = ctx->d_iters + (nf - 1); a.diag = ctx->resblk + RB_DIAG;
     a.nx = 0;
     if (nf == FS_VAR_PC)
       for (int j = 0; j < ctx->pc_nguess && j < FS_GUESS_MAX; j++) a.xs[a.nx++] = ctx->pc_guess[j];
     a.fit = ctx->d_status + 6;
     a.nncnt = ctx->pc_nn ? fs_nn_counters(ctx) : nullptr;   // the network's guess is in the basis
-    a.gridbar = M->gridbar;
+    a.gridbar = gridbar;
     a.teambar = (unsigned *)(ctx->d_status + 4);
     a.status = ctx->d_status;
     a.team_extra = ctx->test_wait_extra;
