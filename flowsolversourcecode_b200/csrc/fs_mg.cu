@@ -567,10 +567,14 @@ __global__ void k_to_f32(long n, const double *a, float *b) {
 // Gauss-Jordan without pivoting, one block barrier per pivot.  Warp y holds
 // rows y + 16 a, lane x columns x + 32 b in registers; the pivot row and column
 // of step k, and the pivot's reciprocal, are read from buffers (by the parity
-// of k) that the update of step k-1 filled.  With the matrix in shared memory a
-// pivot moved 24 bytes per entry through it and took 4 us at n = 157 (0.60 ms in
-// all, a quarter of the 64x64 cavity's p' solve); every entry goes through the
-// same operations.
+// of k) that step k-1 filled.  The update is a multiplication and a subtraction
+// per entry; the pivot row, column and reciprocal are handled outside it, by the
+// warp or the lanes they belong to.  Bound by FP64 rate (64 a clock and SM: 0.4
+// us a pivot at n = 157) and the chain barrier - reciprocal - barrier.  With the
+// matrix in shared memory, or a select or branch per entry, a pivot took 4 us at
+// n = 157 (0.64 ms in all); the set-up of the 64x64 cavity's p' solve went from
+// 0.67 to 0.25 ms.  Every entry goes through the same operations as an in-place
+// elimination.
 // The agglomerated matrices are diagonally dominant.  A pure-Neumann level
 // (every row sum ~0: the pressure correction with walls only) is singular with
 // the constant null space; its last equation is replaced by x_{n-1} = 0 and the
@@ -609,37 +613,56 @@ __global__ void __launch_bounds__(512, 1) k_mg_dense_inverse(int n, int w, const
 #pragma unroll
     for (int b = 0; b < CT; b++) {
       const int i = wid + 16 * a, j = lane + 32 * b;
-      v[a][b] = i < n && j < n ? A[(long)i * n + j] : 0.;
+      v[a][b] = i < n && j > 0 && j < n ? A[(long)i * n + j] : 0.;   // column 0 is published
     }
-  for (int j = tid; j < n; j += nt) { prow[0][j] = A[j]; pcol[0][j] = A[(long)j * n]; }
+  for (int j = tid; j < 32 * CT; j += nt) {
+    prow[0][j] = j < n ? A[j] : 0.;
+    pcol[0][j] = j < n ? A[(long)j * n] : 0.;
+  }
   if (tid == 0) pinv[0] = A[0] != 0. ? 1. / A[0] : 0.;
   __syncthreads();
   for (int k = 0; k < n; k++) {
-    const int c = k & 1, d = c ^ 1;
+    const int c = k & 1, d = c ^ 1, k1 = k + 1;
     const double p = pinv[c];
     double rk[CT];
 #pragma unroll
-    for (int b = 0; b < CT; b++) {
-      const int j = lane + 32 * b;
-      rk[b] = j == k ? p : j < n ? prow[c][j] * p : 0.;
-    }
+    for (int b = 0; b < CT; b++) rk[b] = lane + 32 * b == k ? p : prow[c][lane + 32 * b] * p;
+    // every entry v - c rk (column k holds 0 since it was published) ...
 #pragma unroll
     for (int a = 0; a < RT; a++) {
-      const int i = wid + 16 * a;
-      if (i < n) {
-        const double ci = pcol[c][i];
+      const double ci = pcol[c][wid + 16 * a];
 #pragma unroll
-        for (int b = 0; b < CT; b++) {
-          const int j = lane + 32 * b;
-          const double u = i == k ? rk[b] : j == k ? -ci * p : v[a][b] - ci * rk[b];
-          v[a][b] = u;
-          if (j == k + 1) {
-            pcol[d][i] = u;
-            if (i == k + 1) pinv[d] = u != 0. ? 1. / u : 0.;
-          }
-          if (i == k + 1 && j < n) prow[d][j] = u;
-        }
+      for (int b = 0; b < CT; b++) v[a][b] = v[a][b] - ci * rk[b];
+    }
+    // ... but row k, which becomes rk; then row and column k+1 for the next step.
+    // (Bit tests, not a == k / 16: the compiler would index v with k / 16, in memory.)
+    if (wid == (k & 15)) {
+#pragma unroll
+      for (int a = 0; a < RT; a++)
+        if (1u << (k >> 4) & 1u << a)
+#pragma unroll
+          for (int b = 0; b < CT; b++) v[a][b] = rk[b];
+    }
+    if (wid == (k1 & 15)) {
+#pragma unroll
+      for (int a = 0; a < RT; a++)
+        if (1u << (k1 >> 4) & 1u << a)
+#pragma unroll
+          for (int b = 0; b < CT; b++) prow[d][lane + 32 * b] = v[a][b];
+      if (lane == (k1 & 31) && k1 < n) {   // its own store
+        const double next = prow[d][k1];
+        pinv[d] = next != 0. ? 1. / next : 0.;
       }
+    }
+    if (lane == (k1 & 31)) {
+#pragma unroll
+      for (int b = 0; b < CT; b++)
+        if (1u << (k1 >> 5) & 1u << b)
+#pragma unroll
+          for (int a = 0; a < RT; a++) {
+            pcol[d][wid + 16 * a] = v[a][b];
+            v[a][b] = 0.;
+          }
     }
     __syncthreads();
   }
