@@ -484,12 +484,12 @@ __device__ __forceinline__ void copy_words(T &dst, const T &src) {
   for (int q = threadIdx.x; q < (int)(sizeof(T) / 4); q += blockDim.x) ((int32_t *)&dst)[q] = ((const int32_t *)&src)[q];
 }
 
-// lanes per row of a level, from the threads that the cycle of PCycle gives it
+// log2 of the lanes per row of a level, from the threads that the cycle of PCycle gives it
 // (pc_scope, level_rows): it fixes the order of a row's sum
 __device__ __forceinline__ int vc_lanes(int n) {
   const long nth = (long)blockDim.x * (n > FS_PC_TEAM_MAX ? cta_count() : n > FS_PC_SMALL ? team_size() : 1);
   const long per = nth / (n > 0 ? n : 1);
-  return per < 2 ? 1 : per < 4 ? 2 : per < 8 ? 4 : 8;
+  return per < 2 ? 0 : per < 4 ? 1 : per < 8 ? 2 : 3;
 }
 
 // lanes per row and this CTA's aggregates of every level: consecutive ones
@@ -524,9 +524,10 @@ struct Warps {
   }
 };
 
+// sum over the 2^g lanes of a row
 template <class R>
-__device__ __forceinline__ R lanes_sum(R v, int G) {
-  for (int o = G >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+__device__ __forceinline__ R lanes_sum(R v, int g) {
+  for (int o = 1 << g >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
@@ -539,27 +540,26 @@ __device__ __forceinline__ R *vc_rows() {
 
 // Sums of the residuals of the CTA's rows (rs, from row e0 of level l) over its
 // aggregates: b of level l+1, and unless that is the coarsest its first sweep
-// from zero x = omega b / ac.  Gc lanes an aggregate; (P, c0, c1, d): the
-// thread's first aggregate, its rows and diagonal, loaded before the residuals
-// were done.
+// from zero x = omega b / ac.  2^gc lanes an aggregate; AggFirst: the thread's
+// first aggregate, its rows and diagonal, loaded before the residuals were done.
 template <class R>
 struct AggFirst { int P, c0, c1; R d; };
 template <class R>
-__device__ __forceinline__ AggFirst<R> vc_agg(const VcDev<R> &V, int l, int Gc, bool sweep, int P) {
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ AggFirst<R> vc_agg(const VcDev<R> &V, int l, int gc, bool sweep, int P) {
   AggFirst<R> f{P, 0, 0, (R)1};
   if (P < V.p1[l]) {
-    f.c0 = __ldg(V.L[l].kp + P) - V.e0[l] + lane % Gc;
-    f.c1 = __ldg(V.L[l].kp + P + 1) - V.e0[l];
+    const int32_t *__restrict__ kp = V.L[l].kp;
+    const int e0 = V.e0[l];
+    f.c0 = __ldg(kp + P) - e0 + ((threadIdx.x & 31) & ((1 << gc) - 1));
+    f.c1 = __ldg(kp + P + 1) - e0;
     if (sweep) f.d = __ldg(V.L[l + 1].ac + P);
   }
   return f;
 }
 template <class R>
-__device__ __forceinline__ void vc_restrict(const VcDev<R> &V, int l, int Gc, bool sweep, const R *rs, AggFirst<R> f) {
-  const VcLevel<R> &C = V.L[l + 1];
-  const int lane = threadIdx.x & 31, P1 = V.p1[l];
-  while (f.P - lane / Gc < P1) {
+__device__ __forceinline__ void vc_restrict(const VcDev<R> &V, int l, int gc, bool sweep, const R *rs, AggFirst<R> f) {
+  const int lane = threadIdx.x & 31, P1 = V.p1[l], Gc = 1 << gc;
+  while (f.P - (lane >> gc) < P1) {
     R s = (R)0;
     for (int c = f.c0; c < f.c1; c += 4 * Gc) {
       R v[4];
@@ -568,63 +568,72 @@ __device__ __forceinline__ void vc_restrict(const VcDev<R> &V, int l, int Gc, bo
 #pragma unroll
       for (int u = 0; u < 4; u++) if (c + u * Gc < f.c1) s = s + v[u];
     }
-    if (Gc > 1) s = lanes_sum(s, Gc);
-    if (f.P < P1 && lane % Gc == 0) {
-      C.b[f.P] = s;
-      if (sweep) C.x[f.P] = (R)FS_MG_OMEGA * s / f.d;
+    if (gc) s = lanes_sum(s, gc);
+    if (f.P < P1 && (lane & (Gc - 1)) == 0) {
+      V.L[l + 1].b[f.P] = s;
+      if (sweep) V.L[l + 1].x[f.P] = (R)FS_MG_OMEGA * s / f.d;
     }
-    f = vc_agg(V, l, Gc, sweep, f.P + (int)blockDim.x / Gc);
+    f = vc_agg(V, l, gc, sweep, f.P + (int)(blockDim.x >> gc));
   }
 }
 
 // Down leg of level l >= 1.  A CTA takes the aggregates [p0, p1) and with them
-// the consecutive rows [e0, e1): residuals first (G lanes a row), kept in
+// the consecutive rows [e0, e1): residuals first (2^g lanes a row), kept in
 // shared memory or, when they do not fit, in the level's r, then behind a block
-// barrier their sums.  Every phase ends with a grid barrier.
+// barrier their sums.  Every phase ends with a grid barrier.  Lane counts are
+// powers of two and kept as shifts, and a warp without rows goes straight to
+// the barrier: on a small level the other warps' index arithmetic was most of
+// the phase (32 warps a CTA share four issue slots).
 template <class R>
-__device__ __forceinline__ void vc_down(int l, int Gc, bool sweep) {
-  const VcDev<R> &V = vstate<R>();
-  R *sh = vc_rows<R>();
+__device__ __forceinline__ void vc_down(int l, int gc, bool sweep) {
   constexpr int U = 8;
+  const VcDev<R> &V = vstate<R>();
   const VcLevel<R> &F = V.L[l];
-  const int G = V.G[l], e0 = V.e0[l], e1 = V.e1[l], w = F.w;
-  R *rs = e1 - e0 <= FS_VC_ROWS ? sh : F.r + e0;
-  const int32_t *__restrict__ col = F.col;
-  const R *__restrict__ val = F.val, *__restrict__ ac = F.ac;
-  const R *x = F.x, *b = F.b;
-  const int lane = threadIdx.x & 31, q = lane % G, rpp = (int)blockDim.x / G;
-  const AggFirst<R> first = vc_agg(V, l, Gc, sweep, V.p0[l] + (int)threadIdx.x / Gc);
-  for (int a = e0 + (int)threadIdx.x / G; a - lane / G < e1; a += rpp) {
-    const bool h = a < e1;
-    const long p = ((long)(a >> 5) * w) * 32 + (a & 31);
-    const R bi = h ? b[a] : (R)0, xi = h ? x[a] : (R)0, d = h ? __ldg(ac + a) : (R)0;
-    R t = (R)0;
-    for (int j0 = q; j0 < w; j0 += U * G) {
-      int k[U];
-      R c[U], g[U];
+  const int g = V.G[l], e0 = V.e0[l], e1 = V.e1[l], lane = threadIdx.x & 31;
+  R *rs = e1 - e0 <= FS_VC_ROWS ? vc_rows<R>() : F.r + e0;
+  int a0 = e0 + (int)((threadIdx.x & ~31u) >> g);   // the warp's first row
+  const int P0 = V.p0[l] + (int)((threadIdx.x & ~31u) >> gc);
+  const bool sums = P0 < V.p1[l];
+  AggFirst<R> first{P0, 0, 0, (R)1};
+  if (sums) first = vc_agg(V, l, gc, sweep, P0 + (lane >> gc));
+  if (a0 < e1) {
+    const int32_t *__restrict__ col = F.col;
+    const R *__restrict__ val = F.val, *__restrict__ ac = F.ac;
+    const R *x = F.x, *b = F.b;
+    const int G = 1 << g, q = lane & (G - 1), w = F.w, rpp = (int)(blockDim.x >> g);
+    for (; a0 < e1; a0 += rpp) {
+      const int a = a0 + (lane >> g);
+      const bool h = a < e1;
+      const long p = ((long)(a >> 5) * w) * 32 + (a & 31);
+      const R bi = h ? b[a] : (R)0, xi = h ? x[a] : (R)0, d = h ? __ldg(ac + a) : (R)0;
+      R t = (R)0;
+      for (int j0 = q; j0 < w; j0 += U * G) {
+        int k[U];
+        R c[U], y[U];
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        const bool in = h && j0 + u * G < w;
-        k[u] = in ? __ldg(col + p + (long)(j0 + u * G) * 32) : -1;
-        c[u] = in ? __ldg(val + p + (long)(j0 + u * G) * 32) : (R)0;
+        for (int u = 0; u < U; u++) {
+          const bool in = h && j0 + u * G < w;
+          k[u] = in ? __ldg(col + p + (long)(j0 + u * G) * 32) : -1;
+          c[u] = in ? __ldg(val + p + (long)(j0 + u * G) * 32) : (R)0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) y[u] = k[u] >= 0 ? x[k[u]] : (R)0;
+#pragma unroll
+        for (int u = 0; u < U; u++) t = t + c[u] * y[u];
       }
-#pragma unroll
-      for (int u = 0; u < U; u++) g[u] = k[u] >= 0 ? x[k[u]] : (R)0;
-#pragma unroll
-      for (int u = 0; u < U; u++) t = t + c[u] * g[u];
+      if (g) t = lanes_sum(t, g);
+      if (h && q == 0) rs[a - e0] = bi - d * xi - t;
     }
-    if (G > 1) t = lanes_sum(t, G);
-    if (h && q == 0) rs[a - e0] = bi - d * xi - t;
   }
   __syncthreads();
-  vc_restrict(V, l, Gc, sweep, rs, first);
+  if (sums) vc_restrict(V, l, gc, sweep, rs, first);
   grid_barrier();
 }
 
 // The same for level 0: b = in and x = x0 in mesh order, row a is cell cells[a],
 // a thread per row.
 template <class R>
-__device__ __forceinline__ void vc_down_fine(int Gc, const double *in, const R *x0) {
+__device__ __forceinline__ void vc_down_fine(int gc, const double *in, const R *x0) {
   const VcDev<R> &V = vstate<R>();
   R *sh = vc_rows<R>();
   constexpr int U = 6;
@@ -635,7 +644,7 @@ __device__ __forceinline__ void vc_down_fine(int Gc, const double *in, const R *
   const int32_t *__restrict__ col = F.col, *__restrict__ cells = F.cells;
   const R *__restrict__ val = F.val, *__restrict__ ac = F.ac;
   int a = e0 + (int)threadIdx.x, i = a < e1 ? __ldg(cells + a) : 0, k[U];
-  AggFirst<R> first = vc_agg(V, 0, Gc, sweep, V.p0[0] + (int)threadIdx.x / Gc);
+  AggFirst<R> first = vc_agg(V, 0, gc, sweep, V.p0[0] + (int)(threadIdx.x >> gc));
 #pragma unroll
   for (int u = 0; u < U; u++) k[u] = a < e1 && u < w ? __ldg(col + (long)u * n + a) : -1;
   while (a < e1) {
@@ -661,64 +670,64 @@ __device__ __forceinline__ void vc_down_fine(int Gc, const double *in, const R *
     a = an;
   }
   __syncthreads();
-  vc_restrict(V, 0, Gc, sweep, rs, first);
+  vc_restrict(V, 0, gc, sweep, rs, first);
   grid_barrier();
 }
 
-// post-sweep of level L's rows, then the prolongation into the finer level F's
-// x (last: level 1, whose result goes to x1)
+// post-sweep of level l's rows, then the prolongation into the finer level's x
+// (level 1: the result goes to x1)
 template <class R>
 __device__ __forceinline__ void vc_up(int l) {
+  constexpr int U = 8;
   const VcDev<R> &V = vstate<R>();
   const VcLevel<R> &L = V.L[l], &F = V.L[l - 1];
-  const int G = V.G[l];
-  const bool last = l == 1;
-  R *x1 = V.x1;
-  constexpr int U = 8;
-  const int lane = threadIdx.x & 31, q = lane % G, rpw = 32 / G, n = L.n, wd = L.w;
-  const Warps w((n + rpw - 1) / rpw);
-  const int32_t *__restrict__ col = L.col, *__restrict__ kp = F.kp;
-  const R *__restrict__ val = L.val, *__restrict__ ac = L.ac;
-  const R *x = L.x, *b = L.b;
-  R *xf = F.x;
-  for (int s = w.w0; s * rpw < n; s += w.nw) {
-    const int i = s * rpw + lane / G;
-    const bool act = i < n;
-    const long p = ((long)(i >> 5) * wd) * 32 + (i & 31);
-    const R xi = act ? x[i] : (R)0, bi = act ? b[i] : (R)0, d = act ? __ldg(ac + i) : (R)1;
-    int c = 0, c1 = 0;
-    R f0 = (R)0, f1 = (R)0;
-    if (!last && act) {
-      c = __ldg(kp + i) + q;
-      c1 = __ldg(kp + i + 1);
-      if (c < c1) f0 = xf[c];
-      if (c + G < c1) f1 = xf[c + G];
-    }
-    R t = (R)0;
-    for (int j0 = q; j0 < wd; j0 += U * G) {
-      int k[U];
-      R v[U], g[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const bool in = act && j0 + u * G < wd;
-        k[u] = in ? __ldg(col + p + (long)(j0 + u * G) * 32) : -1;
-        v[u] = in ? __ldg(val + p + (long)(j0 + u * G) * 32) : (R)0;
+  const int g = V.G[l], n = L.n;
+  const Warps w((n + (32 >> g) - 1) >> (5 - g));
+  if (w.w0 << (5 - g) < n) {
+    const int lane = threadIdx.x & 31, G = 1 << g, q = lane & (G - 1), wd = L.w;
+    const int32_t *__restrict__ col = L.col, *__restrict__ kp = F.kp;
+    const R *__restrict__ val = L.val, *__restrict__ ac = L.ac;
+    const R *x = L.x, *b = L.b;
+    R *xf = F.x, *x1 = V.x1;
+    for (int s = w.w0; s << (5 - g) < n; s += w.nw) {
+      const int i = (s << (5 - g)) + (lane >> g);
+      const bool act = i < n;
+      const long p = ((long)(i >> 5) * wd) * 32 + (i & 31);
+      const R xi = act ? x[i] : (R)0, bi = act ? b[i] : (R)0, d = act ? __ldg(ac + i) : (R)1;
+      int c = 0, c1 = 0;
+      R f0 = (R)0, f1 = (R)0;
+      if (l > 1 && act) {
+        c = __ldg(kp + i) + q;
+        c1 = __ldg(kp + i + 1);
+        if (c < c1) f0 = xf[c];
+        if (c + G < c1) f1 = xf[c + G];
       }
+      R t = (R)0;
+      for (int j0 = q; j0 < wd; j0 += U * G) {
+        int k[U];
+        R v[U], y[U];
 #pragma unroll
-      for (int u = 0; u < U; u++) g[u] = k[u] >= 0 ? x[k[u]] : (R)0;
+        for (int u = 0; u < U; u++) {
+          const bool in = act && j0 + u * G < wd;
+          k[u] = in ? __ldg(col + p + (long)(j0 + u * G) * 32) : -1;
+          v[u] = in ? __ldg(val + p + (long)(j0 + u * G) * 32) : (R)0;
+        }
 #pragma unroll
-      for (int u = 0; u < U; u++) t = t + v[u] * g[u];
-    }
-    if (G > 1) t = lanes_sum(t, G);
-    if (!act) continue;
-    const R xn = xi + (R)FS_MG_OMEGA * (bi - d * xi - t) / d;
-    if (last) {
-      if (q == 0) x1[i] = xn;
-    } else {
-      const R add = (R)FS_MG_ALPHA * xn;
-      if (c < c1) xf[c] = f0 + add;
-      if (c + G < c1) xf[c + G] = f1 + add;
-      for (c += 2 * G; c < c1; c += G) xf[c] = xf[c] + add;
+        for (int u = 0; u < U; u++) y[u] = k[u] >= 0 ? x[k[u]] : (R)0;
+#pragma unroll
+        for (int u = 0; u < U; u++) t = t + v[u] * y[u];
+      }
+      if (g) t = lanes_sum(t, g);
+      if (!act) continue;
+      const R xn = xi + (R)FS_MG_OMEGA * (bi - d * xi - t) / d;
+      if (l == 1) {
+        if (q == 0) x1[i] = xn;
+      } else {
+        const R add = (R)FS_MG_ALPHA * xn;
+        if (c < c1) xf[c] = f0 + add;
+        if (c + G < c1) xf[c + G] = f1 + add;
+        for (c += 2 * G; c < c1; c += G) xf[c] = xf[c] + add;
+      }
     }
   }
   grid_barrier();
@@ -766,7 +775,7 @@ template <class R, bool GS>
 __device__ __forceinline__ void vcycle_coarse() {
   const VcDev<R> &V = vstate<R>();
   const int lc = V.lc;
-  for (int l = 1; l < lc; l++) vc_down<R>(l, GS ? 1 : V.G[l + 1], l + 1 < lc);
+  for (int l = 1; l < lc; l++) vc_down<R>(l, GS ? 0 : V.G[l + 1], l + 1 < lc);
   vc_dense<R>();
   for (int l = lc - 1; l >= 1; l--) vc_up<R>(l);
 }
@@ -862,7 +871,7 @@ __device__ __forceinline__ void vcycle_gs(const double *in, double *out) {
   for (long i = t0; i < L.n; i += nt) x[i] = (R)0.;
   grid_barrier();
   gs_colours<R>(in, false);
-  vc_down_fine<R>(1, in, x);
+  vc_down_fine<R>(0, in, x);
   vcycle_coarse<R, true>();
   const R al0 = (R)FS_MG_ALPHA0;
   for (long i = t0; i < L.n; i += nt) x[i] = x[i] + al0 * V.x1[V.par0[i]];

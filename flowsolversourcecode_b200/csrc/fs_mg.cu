@@ -89,7 +89,7 @@ struct VcLevel {
 template <class R>
 struct VcDev {
   int lc;
-  // set by each CTA of the kernel: lanes per row, its aggregates and their rows
+  // set by each CTA of the kernel: lanes per row (log2), its aggregates and their rows
   int G[FS_MG_MAXLEV], p0[FS_MG_MAXLEV], p1[FS_MG_MAXLEV], e0[FS_MG_MAXLEV], e1[FS_MG_MAXLEV];
   VcLevel<R> L[FS_MG_MAXLEV];
   R *x1;                 // result of level 1
