@@ -212,7 +212,7 @@ class Solver:
         return sizes.get(name, N)
 
     def get(self, name: str) -> np.ndarray:
-        a = np.zeros(self._size(name))
+        a = np.empty(self._size(name))
         self._chk(self.lib.fs_get_field(self.ctx, L.FIELD_ID[name], L.dptr(a), a.shape[0]), f"get {name}")
         return a
 
