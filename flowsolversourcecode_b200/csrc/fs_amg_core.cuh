@@ -484,6 +484,43 @@ __device__ __forceinline__ void copy_words(T &dst, const T &src) {
   for (int q = threadIdx.x; q < (int)(sizeof(T) / 4); q += blockDim.x) ((int32_t *)&dst)[q] = ((const int32_t *)&src)[q];
 }
 
+// Level 0's neighbour indices of a row, from the table (PAT false: slot u of row
+// a at nbr[u n + a], loaded a row ahead) or from its pattern (a byte a row ahead,
+// the offsets in shared memory)
+__device__ __forceinline__ int32_t *pat_offs() {
+  __shared__ __align__(16) int32_t s[FS_PAT_MAX * 8];
+  return s;
+}
+template <bool PAT>
+struct RowIdx;
+template <>
+struct RowIdx<false> {
+  int k[6];
+  __device__ __forceinline__ void load(const int32_t *__restrict__ nbr, const uint8_t *, int n, int w, long a, bool h) {
+#pragma unroll
+    for (int u = 0; u < 6; u++) k[u] = h && u < w ? __ldg(nbr + (long)u * n + a) : -1;
+  }
+  __device__ __forceinline__ void get(int (&o)[6], int, bool) const {
+#pragma unroll
+    for (int u = 0; u < 6; u++) o[u] = k[u];
+  }
+};
+template <>
+struct RowIdx<true> {
+  int p;
+  __device__ __forceinline__ void load(const int32_t *, const uint8_t *__restrict__ pat, int, int, long a, bool h) {
+    p = h ? __ldg(pat + a) : 0;
+  }
+  __device__ __forceinline__ void get(int (&o)[6], int i, bool h) const {
+    const int32_t *s = pat_offs() + 8 * p;
+    const int4 q = *reinterpret_cast<const int4 *>(s);
+    const int2 r = *reinterpret_cast<const int2 *>(s + 4);
+    const int f[6] = {q.x, q.y, q.z, q.w, r.x, r.y};
+#pragma unroll
+    for (int u = 0; u < 6; u++) o[u] = h && f[u] != FS_PAT_NONE ? i + f[u] : -1;
+  }
+};
+
 // log2 of the lanes per row of a level, from the threads that the cycle of PCycle gives it
 // (pc_scope, level_rows): it fixes the order of a row's sum
 __device__ __forceinline__ int vc_lanes(int n) {
@@ -632,23 +669,26 @@ __device__ __forceinline__ void vc_down(int l, int gc, bool sweep) {
 
 // The same for level 0: b = in and x = x0 in mesh order, row a is cell cells[a],
 // a thread per row.
-template <class R>
+template <class R, bool PAT>
 __device__ __forceinline__ void vc_down_fine(int gc, const double *in, const R *x0) {
+  constexpr int U = 6;
   const VcDev<R> &V = vstate<R>();
   R *sh = vc_rows<R>();
-  constexpr int U = 6;
   const VcLevel<R> &F = V.L[0];
   const int e0 = V.e0[0], e1 = V.e1[0], n = F.n, w = F.w;
   const bool sweep = V.lc > 1;
   R *rs = e1 - e0 <= FS_VC_ROWS ? sh : F.r + e0;
   const int32_t *__restrict__ col = F.col, *__restrict__ cells = F.cells;
+  const uint8_t *__restrict__ pat = V.patL;
   const R *__restrict__ val = F.val, *__restrict__ ac = F.ac;
-  int a = e0 + (int)threadIdx.x, i = a < e1 ? __ldg(cells + a) : 0, k[U];
-  AggFirst<R> first = vc_agg(V, 0, gc, sweep, V.p0[0] + (int)(threadIdx.x >> gc));
-#pragma unroll
-  for (int u = 0; u < U; u++) k[u] = a < e1 && u < w ? __ldg(col + (long)u * n + a) : -1;
+  int a = e0 + (int)threadIdx.x, i = a < e1 ? __ldg(cells + a) : 0;
+  RowIdx<PAT> ix;
+  ix.load(col, pat, n, w, a, a < e1);
+  const AggFirst<R> first = vc_agg(V, 0, gc, sweep, V.p0[0] + (int)(threadIdx.x >> gc));
   while (a < e1) {
+    int k[U];
     R c[U], g[U];
+    ix.get(k, i, true);
 #pragma unroll
     for (int u = 0; u < U; u++) {
       c[u] = k[u] >= 0 ? __ldg(val + (long)u * n + a) : (R)0;
@@ -657,8 +697,7 @@ __device__ __forceinline__ void vc_down_fine(int gc, const double *in, const R *
     const R bi = (R)in[i], xi = x0[i], d = __ldg(ac + a);
     const int an = a + (int)blockDim.x;
     i = an < e1 ? __ldg(cells + an) : 0;
-#pragma unroll
-    for (int u = 0; u < U; u++) k[u] = an < e1 && u < w ? __ldg(col + (long)u * n + an) : -1;
+    ix.load(col, pat, n, w, an, an < e1);
     R t = (R)0;
 #pragma unroll
     for (int u = 0; u < U; u++) t = t + c[u] * g[u];
@@ -780,9 +819,8 @@ __device__ __forceinline__ void vcycle_coarse() {
   for (int l = lc - 1; l >= 1; l--) vc_up<R>(l);
 }
 
-// level 0's post-sweep into out, with its correction formed on the fly; the
-// next row's indices are loaded while a row gathers
-template <class R>
+// level 0's post-sweep into out, with its correction formed on the fly
+template <class R, bool PAT>
 __device__ __forceinline__ void vc_up_fine(const double *in, double *out) {
   constexpr int U = 6;
   const VcDev<R> &V = vstate<R>();
@@ -791,15 +829,16 @@ __device__ __forceinline__ void vc_up_fine(const double *in, double *out) {
   long i = (long)cta_id() * blockDim.x + threadIdx.x;
   const int n = L.n, w = L.w;
   const int32_t *__restrict__ nbr = L.nbr, *__restrict__ par = V.par0;
+  const uint8_t *__restrict__ pat = V.pat;
   const R *__restrict__ anb = L.anb, *__restrict__ ac = L.ac;
   const R *x0 = L.x, *x1 = V.x1;
   const R al0 = (R)FS_MG_ALPHA0, om0 = (R)FS_MG_OMEGA0;
-  int k[U];
-#pragma unroll
-  for (int u = 0; u < U; u++) k[u] = i < n && u < w ? __ldg(nbr + (long)u * n + i) : -1;
+  RowIdx<PAT> ix;
+  ix.load(nbr, pat, n, w, i, i < n);
   while (i < n) {
     R c[U], y[U], z[U];
-    int q[U];
+    int k[U], q[U];
+    ix.get(k, (int)i, true);
     const int qi = __ldg(par + i);
 #pragma unroll
     for (int u = 0; u < U; u++) q[u] = k[u] >= 0 ? __ldg(par + k[u]) : 0;
@@ -812,8 +851,7 @@ __device__ __forceinline__ void vc_up_fine(const double *in, double *out) {
 #pragma unroll
     for (int u = 0; u < U; u++) z[u] = k[u] >= 0 ? x1[q[u]] : (R)0;
     const long in1 = i + nt;
-#pragma unroll
-    for (int u = 0; u < U; u++) k[u] = in1 < n && u < w ? __ldg(nbr + (long)u * n + in1) : -1;
+    ix.load(nbr, pat, n, w, in1, in1 < n);
     R t = (R)0;
 #pragma unroll
     for (int u = 0; u < U; u++) t = t + c[u] * (y[u] + al0 * z[u]);
@@ -833,9 +871,11 @@ __device__ __forceinline__ void vc_up_fine(const double *in, double *out) {
 template <class R>
 __device__ __forceinline__ void vcycle(const double *in, double *out) {
   const VcDev<R> &V = vstate<R>();
-  vc_down_fine<R>(V.G[1], in, V.L0.x);
+  if (V.npat) vc_down_fine<R, true>(V.G[1], in, V.L0.x);
+  else vc_down_fine<R, false>(V.G[1], in, V.L0.x);
   vcycle_coarse<R, false>();
-  vc_up_fine<R>(in, out);
+  if (V.npat) vc_up_fine<R, true>(in, out);
+  else vc_up_fine<R, false>(in, out);
 }
 
 // One multicolour Gauss-Seidel pass over level 0 in place: the colours in
@@ -871,7 +911,8 @@ __device__ __forceinline__ void vcycle_gs(const double *in, double *out) {
   for (long i = t0; i < L.n; i += nt) x[i] = (R)0.;
   grid_barrier();
   gs_colours<R>(in, false);
-  vc_down_fine<R>(0, in, x);
+  if (V.npat) vc_down_fine<R, true>(0, in, x);
+  else vc_down_fine<R, false>(0, in, x);
   vcycle_coarse<R, true>();
   const R al0 = (R)FS_MG_ALPHA0;
   for (long i = t0; i < L.n; i += nt) x[i] = x[i] + al0 * V.x1[V.par0[i]];
@@ -904,8 +945,8 @@ __device__ __forceinline__ void apply_prec(Sync &S, const double *in, double *ou
 // sums need: (y.e, y.y, y.f) or (e.y) alone.  The next row's indices are loaded
 // while a row gathers.  Every pass loads all it needs of a row before it
 // stores, so the stores do not hold up the loads.
-template <class R, int K>
-__device__ __forceinline__ Sum3 krylov_ax(const double *x, double *y, const double *e, const double *f) {
+template <class R, int K, bool PAT>
+__device__ __forceinline__ Sum3 krylov_ax_rows(const double *x, double *y, const double *e, const double *f) {
   constexpr int U = 6;
   const AmgKArgs<R> &A = astate<R>();
   const int n = A.N, w = A.W;
@@ -914,11 +955,13 @@ __device__ __forceinline__ Sum3 krylov_ax(const double *x, double *y, const doub
   const long nt = (long)cta_count() * blockDim.x;
   long i = (long)cta_id() * blockDim.x + threadIdx.x;
   Sum3 s{0., 0., 0.};
-  int k[U];
-#pragma unroll
-  for (int u = 0; u < U; u++) k[u] = i < n && u < w ? __ldg(nbr + (long)u * n + i) : -1;
+  const uint8_t *__restrict__ pat = PAT ? vstate<R>().pat : nullptr;
+  RowIdx<PAT> ix;
+  ix.load(nbr, pat, n, w, i, i < n);
   while (i < n) {
+    int k[U];
     double c[U], g[U];
+    ix.get(k, (int)i, true);
 #pragma unroll
     for (int u = 0; u < U; u++) {
       c[u] = k[u] >= 0 ? __ldg(anb + (long)u * n + i) : 0.;
@@ -926,8 +969,7 @@ __device__ __forceinline__ Sum3 krylov_ax(const double *x, double *y, const doub
     }
     const double aci = __ldg(ac + i), xi = x[i], ei = e[i], fi = K > 1 ? f[i] : 0.;
     const long in = i + nt;
-#pragma unroll
-    for (int u = 0; u < U; u++) k[u] = in < n && u < w ? __ldg(nbr + (long)u * n + in) : -1;
+    ix.load(nbr, pat, n, w, in, in < n);
     double t = aci * xi;
 #pragma unroll
     for (int u = 0; u < U; u++) t = t + c[u] * g[u];
@@ -941,6 +983,11 @@ __device__ __forceinline__ Sum3 krylov_ax(const double *x, double *y, const doub
     i = in;
   }
   return s;
+}
+template <class R, int MODE, int K>
+__device__ __forceinline__ Sum3 krylov_ax(const double *x, double *y, const double *e, const double *f) {
+  if (MODE != 0 && vstate<R>().npat) return krylov_ax_rows<R, K, true>(x, y, e, f);
+  return krylov_ax_rows<R, K, false>(x, y, e, f);
 }
 
 // s = r - alpha v with |s|^2 and r0.s, and x_0 = omega0 s / ac_0 of the V-cycle
@@ -1172,7 +1219,10 @@ __device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> &ap) {
   copy_words(astate<R>(), ap);
   if (MODE != 0) copy_words(vstate<R>(), *ap.vc);
   __syncthreads();
-  if (MODE != 0) vc_split<R>();
+  if (MODE != 0) {
+    vc_split<R>();
+    for (int q = threadIdx.x; q < 8 * vstate<R>().npat; q += blockDim.x) pat_offs()[q] = vstate<R>().offs[q];
+  }
   const AmgKArgs<R> &a = astate<R>();
   Sync S(a.part, a.gridbar, a.status, a.team_extra);
   unsigned gen = 0;   // team-barrier generation (the counters are zeroed before the launch)
@@ -1244,7 +1294,7 @@ __device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> &ap) {
     __syncthreads();
     if (threadIdx.x == 0) { K.k++; K.p_ready = false; }
     apply_prec<R, MODE>(S, a.p, a.y, gen);                          // y = M^-1 p
-    const double rv = grid_sums<1>(krylov_ax<R, 1>(a.y, a.v, a.r0, nullptr)).a;   // v = A y
+    const double rv = grid_sums<1>(krylov_ax<R, MODE, 1>(a.y, a.v, a.r0, nullptr)).a;   // v = A y
     if (!(rv != 0.) || !isfinite(K.rho / rv)) break;
     {
       const double alpha = K.rho / rv;
@@ -1258,7 +1308,7 @@ __device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> &ap) {
       }
     }
     apply_prec<R, MODE>(S, a.s, a.z, gen);                          // z = M^-1 s
-    const Sum3 tq = grid_sums<3>(krylov_ax<R, 3>(a.z, a.t, a.s, a.r0));   // t = A z
+    const Sum3 tq = grid_sums<3>(krylov_ax<R, MODE, 3>(a.z, a.t, a.s, a.r0));   // t = A z
     const double ts = tq.a, tt = tq.b, alpha = K.alpha;
     if (!(tt > 0.) || !(ts != 0.) || !isfinite(ts / tt)) {
       // t = A z vanished or is orthogonal to s: take the half step and stop

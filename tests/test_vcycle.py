@@ -100,17 +100,45 @@ class Hierarchy:
         return x + om * (b - _matvec(ac, nbr, anb, x)) / ac
 
 
+def _shuffled(mesh, seed):
+    """The same mesh with its cells renumbered at random (faces back in
+    upper-triangular order): neighbour offsets without a pattern."""
+    rng = np.random.default_rng(seed)
+    p = rng.permutation(mesh.n_cells).astype(np.int32)
+    F = mesh.n_internal
+    nodes = mesh.face_nodes.reshape(-1, 4).copy()
+    own, nbr = p[mesh.owner], p[mesh.neighbour]
+    swap = own[:F] > nbr
+    nodes[:F][swap] = nodes[:F][swap][:, ::-1]
+    own[:F], nbr = np.minimum(own[:F], nbr), np.maximum(own[:F], nbr)
+    order = np.concatenate([np.lexsort((nbr, own[:F])), np.arange(F, mesh.n_faces)])
+    return fm.PolyMesh(mesh.points, mesh.face_ptr, np.ascontiguousarray(nodes[order].ravel()), own[order],
+                       nbr[order[:F]], mesh.patch_names, mesh.patch_start, mesh.patch_size)
+
+
 # one coarse level; two; several; a 2-D mesh; more rows per level than a CTA's
 # shared array of residuals holds and rows shared between threads and lanes
 @pytest.mark.parametrize("dims", [(7, 6, 5), (13, 11, 9), (57, 43, 1), (41, 37, 23), (71, 67, 64)])
 @pytest.mark.parametrize("solver", ["amg_bicgs", "amg32_bicgs", "amg32gs_bicgs"])
 @pytest.mark.parametrize("neumann", [True, False])
 def test_one_iteration_matches_numpy(dims, solver, neumann):
-    from flowsolversourcecode_b200.solver import Solver
     if dims[0] > 60 and (solver == "amg32gs_bicgs" or neumann):
         pytest.skip("the largest mesh runs once per precision")
+    _one_iteration(fm.box_mesh(*dims), solver, neumann)
+
+
+# cells numbered without a pattern (the index table), at a size whose rows are
+# shared between lanes and one with a thread per row
+@pytest.mark.parametrize("dims", [(13, 11, 9), (45, 43, 40)])
+@pytest.mark.parametrize("solver", ["amg_bicgs", "amg32_bicgs", "amg32gs_bicgs"])
+def test_one_iteration_matches_numpy_shuffled(dims, solver):
+    _one_iteration(_shuffled(fm.box_mesh(*dims), 5), solver, False)
+
+
+def _one_iteration(mesh, solver, neumann):
+    from flowsolversourcecode_b200.solver import Solver
     _, case = cs.cavity(4, krylov_tol=1e-14, krylov_maxit=1)
-    s = Solver(fm.box_mesh(*dims), case)
+    s = Solver(mesh, case)
     rng = np.random.default_rng(3)
     con = s.connectivity()
     cn, cf = con["cn"].reshape(s.W, s.N), con["cf"].reshape(s.W, s.N)
