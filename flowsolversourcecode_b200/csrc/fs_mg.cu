@@ -999,6 +999,7 @@ int fs_mg_build(fs_ctx *ctx) {
   int per = std::min(std::min(a, std::min(b, c)), std::min(std::min(b2, c2), c3));
   if (per < 1) { ctx->err = "multigrid kernels do not fit on an SM"; return FS_E_CUDA; }
   M->per_sm = per;   // occupancy limit; the grid follows the launch shape at each solve
+  FS_CK(cudaStreamSynchronize(cudaStreamLegacy));   // the uploads, before the solver's stream reads them
   return FS_OK;
 }
 

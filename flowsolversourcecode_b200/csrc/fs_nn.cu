@@ -1006,7 +1006,10 @@ extern "C" int fs_nn_create(fs_ctx *ctx, int snapshot_capacity, uint64_t seed) {
     std::normal_distribution<float> d(0.f, 0.5f * sqrtf(2.f / NN_K));
     for (int q = 0; q < NN_K * NN_H; q++) th[NN_OFF_L(l) + q] = d(gen);
   }
-  FS_CK(cudaMemcpy(nn->theta, th.data(), sizeof(float) * NN_NP, cudaMemcpyHostToDevice));
+  // the clears above went to the default stream, which the solver's stream does
+  // not wait for; from here on copies go to the solver's stream
+  FS_CK(cudaStreamSynchronize(cudaStreamLegacy));
+  FS_CK(cudaMemcpyAsync(nn->theta, th.data(), sizeof(float) * NN_NP, cudaMemcpyHostToDevice, ctx->st));
   FS_CK(cudaFuncSetAttribute((const void *)k_nn_layer_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)NN_SMEM_FWD));
   FS_CK(cudaFuncSetAttribute((const void *)k_nn_layer_bwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1070,7 +1073,9 @@ extern "C" int fs_nn_params(fs_ctx *ctx, float *get, const float *set, size_t n)
   FS_CK(cudaStreamSynchronize(ctx->st));
   if (get) FS_CK(cudaMemcpy(get, ctx->nn->theta, sizeof(float) * NN_NP, cudaMemcpyDeviceToHost));
   if (set) {
-    FS_CK(cudaMemcpy(ctx->nn->theta, set, sizeof(float) * NN_NP, cudaMemcpyHostToDevice));
+    // on the solver's stream: a copy from pageable memory on another one may
+    // still be under way when it returns, and the packing reads theta
+    FS_CK(cudaMemcpyAsync(ctx->nn->theta, set, sizeof(float) * NN_NP, cudaMemcpyHostToDevice, ctx->st));
     int rc = nn_pack(ctx);
     if (rc) return rc;
     FS_CK(cudaStreamSynchronize(ctx->st));
@@ -1084,15 +1089,15 @@ extern "C" int fs_nn_eval_host(fs_ctx *ctx, const float *X, const float *wgt, co
   cudaSetDevice(ctx->dev);
   fs_nn *nn = ctx->nn;
   const int N = ctx->N, W = ctx->W;
-  FS_CK(cudaMemcpy(nn->X, X, sizeof(float) * N * NN_F, cudaMemcpyHostToDevice));
-  FS_CK(cudaMemcpy(nn->wgt, wgt, sizeof(float) * N * W, cudaMemcpyHostToDevice));
+  FS_CK(cudaMemcpyAsync(nn->X, X, sizeof(float) * N * NN_F, cudaMemcpyHostToDevice, ctx->st));
+  FS_CK(cudaMemcpyAsync(nn->wgt, wgt, sizeof(float) * N * W, cudaMemcpyHostToDevice, ctx->st));
   int rc;
   if ((rc = nn_forward(ctx, nn->X, nn->wgt, true))) return rc;
   if (target) {
     std::vector<double> t(target, target + N);
     double tt = 0.;
     for (double v : t) tt += v * v;
-    FS_CK(cudaMemcpy(nn->tbuf, target, sizeof(float) * N, cudaMemcpyHostToDevice));
+    FS_CK(cudaMemcpyAsync(nn->tbuf, target, sizeof(float) * N, cudaMemcpyHostToDevice, ctx->st));
     if ((rc = nn_backward(ctx, nn->X, nn->wgt, nn->tbuf, tt > 0. ? tt : 1.))) return rc;
     FS_CK(cudaStreamSynchronize(ctx->st));
     double l = 0.;

@@ -98,3 +98,26 @@ def test_training_and_gain(solver):
     assert sum(ic) <= sum(ib) + K // 10
     b.close()
     c.close()
+
+
+def test_alternating_parameter_sets():
+    # the packed weights of a call are those of its own parameters: uploads are
+    # ordered before the kernels that read them, also when nothing waits between
+    s = _solver(40)
+    s.nn_create(0, seed=3)
+    rng = np.random.default_rng(5)
+    calls = []
+    for _ in range(2):
+        X = rng.standard_normal((s.N, nno.F_IN)).astype(np.float32)
+        wgt = rng.uniform(0.05, 0.3, s.W * s.N).astype(np.float32)
+        calls.append(((0.12 * rng.standard_normal(nno.NPARAM)).astype(np.float32), X, wgt,
+                      rng.standard_normal(s.N).astype(np.float32)))
+    first = []
+    for _ in range(4):
+        for k, (theta, X, wgt, t) in enumerate(calls):
+            s.nn_params(set=theta.copy())
+            g = s.nn_eval(X, wgt, t)
+            if len(first) <= k:
+                first.append(g)
+            assert np.array_equal(g["y"], first[k]["y"]) and np.array_equal(g["grad"], first[k]["grad"])
+    s.close()
