@@ -130,8 +130,17 @@ __global__ void k_nn_sums_f(int N, const float *a, const float *b, double *redp)
 __global__ void k_nn_final(const double *redp, int nblk, int nq, int N, double *out, int mode) {
   const int q = threadIdx.x;
   double s = 0.;
-  if (q < nq)
-    for (int b = 0; b < nblk; b++) s += redp[b * 8 + q];
+  if (q < nq) {
+    int b = 0;
+    for (; b + 16 <= nblk; b += 16) {   // sixteen loads in flight, added in order
+      double v[16];
+#pragma unroll
+      for (int u = 0; u < 16; u++) v[u] = redp[(b + u) * 8 + q];
+#pragma unroll
+      for (int u = 0; u < 16; u++) s += v[u];
+    }
+    for (; b < nblk; b++) s += redp[b * 8 + q];
+  }
   // mode 0 (features): s_b = rms(b), mean ac, s_g = rms of the components of grad u,
   //   mean prev, s_p = rms(prev - mean prev); otherwise the raw sums
   __shared__ double t[32];
@@ -242,11 +251,23 @@ __global__ void __launch_bounds__(NN_THREADS) k_nn_out_bwd(int N, const float *H
   const int c = threadIdx.x & (NN_H - 1), rg = threadIdx.x >> 6;
   float gw = 0.f, gb = 0.f;
   const float wc = th[NN_OFF_WOUT + c];
-  for (long i = (long)blockIdx.x * 4 + rg; i < N; i += (long)gridDim.x * 4) {
-    float d = dy[i];
-    gw += H[i * NN_H + c] * d;
-    gb += d;
-    dH[i * NN_H + c] = d * wc;
+  // four rows in flight (the store held the next row's loads back), sums in row order
+  const long step = (long)gridDim.x * 4;
+  for (long i = (long)blockIdx.x * 4 + rg; i < N; i += 4 * step) {
+    float d[4], h[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const bool in = i + u * step < N;
+      d[u] = in ? dy[i + u * step] : 0.f;
+      h[u] = in ? H[(i + u * step) * NN_H + c] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (i + u * step < N) {
+        gw += h[u] * d[u];
+        gb += d[u];
+        dH[(i + u * step) * NN_H + c] = d[u] * wc;
+      }
   }
   sh[rg][c] = gw;
   sh[rg][NN_H] = 0.f;
@@ -267,11 +288,26 @@ __global__ void __launch_bounds__(NN_THREADS) k_nn_in_bwd(int N, const float *X,
   __shared__ float sh[4][NN_F + 1][NN_H];
   const int c = threadIdx.x & (NN_H - 1), rg = threadIdx.x >> 6;
   float g[NN_F + 1] = {};
-  for (long i = (long)blockIdx.x * 4 + rg; i < N; i += (long)gridDim.x * 4) {
-    float dz = mask[i * NN_H + c] ? dH[i * NN_H + c] : 0.f;
+  // four rows in flight, sums in row order
+  const long step = (long)gridDim.x * 4;
+  for (long i = (long)blockIdx.x * 4 + rg; i < N; i += 4 * step) {
+    float dz[4], x[4][NN_F];
 #pragma unroll
-    for (int f = 0; f < NN_F; f++) g[f] += X[i * NN_F + f] * dz;
-    g[NN_F] += dz;
+    for (int u = 0; u < 4; u++) {
+      const long k = i + u * step;
+      const bool in = k < N;
+      const float h = in ? dH[k * NN_H + c] : 0.f;
+      dz[u] = in && mask[k * NN_H + c] ? h : 0.f;
+#pragma unroll
+      for (int f = 0; f < NN_F; f++) x[u][f] = in ? X[k * NN_F + f] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (i + u * step < N) {
+#pragma unroll
+        for (int f = 0; f < NN_F; f++) g[f] += x[u][f] * dz[u];
+        g[NN_F] += dz[u];
+      }
   }
 #pragma unroll
   for (int f = 0; f <= NN_F; f++) sh[rg][f][c] = g[f];
@@ -697,7 +733,18 @@ __global__ void k_nn_reduce(const float *part, int nblk, int pstride, int count,
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= count) return;
   float s = 0.f;
-  for (int b = 0; b < nblk; b++) s += part[(long)b * pstride + p];
+  int b = 0;
+  // bound by the chain of one load per block's partial: sixteen in flight, added in
+  // order; with the rows in flight in k_nn_out_bwd and k_nn_in_bwd, a forward and backward
+  // call at 64,000 cells takes 1.23 ms instead of 1.27
+  for (; b + 16 <= nblk; b += 16) {
+    float v[16];
+#pragma unroll
+    for (int u = 0; u < 16; u++) v[u] = part[(long)(b + u) * pstride + p];
+#pragma unroll
+    for (int u = 0; u < 16; u++) s += v[u];
+  }
+  for (; b < nblk; b++) s += part[(long)b * pstride + p];
   grad[p] = s;
 }
 
