@@ -185,7 +185,7 @@ struct fs_ctx {
   double ens_split = 1.;        // batched ensembles: CTA groups in proportion to cells^ens_split (x p' iterations)
   bool mom_pending = false;
   alignas(8) unsigned char mom_pend[160];   // the prepared launch's arguments (Sor3Args)
-  int test_wait_extra = 0;      // fs_test_wait_timeout: extra arrivals the team barrier waits for
+  int test_wait_extra = 0;      // fs_test_wait_timeout: extra arrivals the AMG solver's barriers wait for
 };
 
 // timing events and their host-side bookkeeping are skipped while a graph is captured

@@ -1494,7 +1494,7 @@ extern "C" int fs_mg_coarse_matrix(fs_ctx *ctx, int level, double *ac, int32_t *
 }
 
 // Test of the bounded device waits (no reference counterpart): with extra > 0
-// the multigrid team barriers wait for more CTAs than the team has, so their
+// the grid barriers of the AMG solves wait for more CTAs than take part, so their
 // polls run out; the solve then ends and the iteration reports FS_E_TIMEOUT.
 extern "C" int fs_test_wait_timeout(fs_ctx *ctx, int extra) {
   if (!ctx || extra < 0 || extra > 64) return FS_E_ARG;

@@ -551,7 +551,7 @@ int fs_nn_policy(fs_ctx *ctx, double *avg_guessed, double *avg_zero, int32_t *pa
  *   the learned guess is not used inside the graph. */
 int fs_set_launch_shape(fs_ctx *ctx, int shape);
 /* Test of the bounded device waits (no reference counterpart): with extra > 0
- * the AMG preconditioner's team barriers wait for `extra` more CTAs than take
+ * the AMG solver's grid barriers wait for `extra` more CTAs than take
  * part, so their bounded polls run out (well under a second); the iteration
  * then returns FS_E_TIMEOUT and its results are not valid.  0 restores normal
  * operation. */
