@@ -204,46 +204,36 @@ def row_bytes(w: int, r: int) -> int:
 
 
 def vcycle_bytes(mg: dict, W: int, N: int, r: int) -> float:
-    """Compulsory HBM bytes of one preconditioner V-cycle (PCycle, one pre- and
-    one post-sweep): every array a phase touches is read or written once.
-      level 0   x0 = w in/ac          : in 8 + ac r + x r
-                residual              : row + in 8 + x r + r r
-                prolong (own phase)   : x r (read) + x r (write) + parent 4
-                sweep to `out` (FP64) : row + in 8 + x r + out 8
-      level l   restrict into l       : per fine row r_{l-1} r + rlist 4;
-                                        per row rptr 4 + b r + ac r + x r
-                residual, prolong+sweep as level 0 with b r instead of in 8,
-                                        the result into r (r bytes)
-      coarsest  restrict as above; dense solve n_c^2 x 8 + b r + x r
+    """Compulsory HBM bytes of one preconditioner V-cycle (one pre- and one
+    post-sweep, a phase per level and leg): every array a phase touches is read
+    or written once.  Level 0's neighbours come as a pattern byte per row (box
+    meshes); residuals stay on chip.
+      level 0   down                  : pattern 1 + (W+1) r + cell 4 + in 8 + x r
+                up into `out`         : pattern 1 + (W+1) r + parent 4 + in 8 + x r + out 8
+      level l   b and x from above 2r; down and up: row + ac r + b r + x r each;
+                the correction from below x 2r (level 1: its result r, read by level 0)
+      coarsest  b r from above; dense solve n_c^2 x 8 + b r
     Gathers of neighbour values are L2 traffic and are not counted."""
     sizes, widths, lc = mg["sizes"], mg["widths"], mg["prec_coarsest"]
-    total = 0.0
-    for l in range(lc + 1):
-        n, w = sizes[l], (W if l == 0 else widths[l])
-        row = row_bytes(w, r)
-        if l == 0:
-            total += n * (8 + 2 * r)                                  # x0 = omega in / ac
-            total += n * (row + 8 + 2 * r)                            # residual
-            total += n * (2 * r + 4)                                  # prolong
-            total += n * (row + 8 + r + 8)                            # sweep into out
-            continue
-        total += sizes[l - 1] * (r + 4) + n * (4 + 3 * r)            # restrict into l
+    total = sizes[0] * (2.0 * (1 + (W + 1) * r + 4 + 8 + r) + 8)
+    for l in range(1, lc + 1):
+        n, w = sizes[l], widths[l]
         if l == lc and mg["direct"]:
             total += n * n * 8 + n * 2 * r
             continue
-        total += n * (row + 3 * r)                                    # residual
-        total += n * (2 * r + 4) + n * (row + 3 * r)                  # prolong + sweep
+        total += n * 2 * r + 2 * n * (row_bytes(w, r) + 2 * r) + n * 2 * r
     return total
 
 
 def amg_bicgstab_bytes(mg: dict, W: int, N: int, r: int, iters: int, calls: int) -> float:
     """k_amg_bicgstab: per BiCGSTAB iteration the Krylov algebra
-      r0.r 16, p 32, v = A y (row + y 8 + v 8 + r0 8), s 24,
-      t = A z (row + z 8 + t 8 + s 8), x/r update 56
-    = 176 + 2 row bytes per row (FP64 matrix), plus two V-cycles; per launch
+      v = A y (row + y 8 + v 8 + r0 8), s (r, v, s, r0 32 + ac and x0 2r),
+      t = A z (row + z 8 + t 8 + s 8 + r0 8), x/r/p pass (x, p 32, y, z, s, t, v, r 48
+      + ac and x0 2r)
+    with rows of 8 (W+1) + 1 bytes (pattern byte), plus two V-cycles; per launch
     the set-up (b, r, r0, p, v, x: 48) and dphi (8)."""
-    row0 = row_bytes(W, 8)
-    per_it = N * (176 + 2 * row0) + 2 * vcycle_bytes(mg, W, N, r)
+    row0 = 8 * (W + 1) + 1
+    per_it = N * (168 + 4 * r + 2 * row0) + 2 * vcycle_bytes(mg, W, N, r)
     return per_it * iters + N * 56.0 * calls
 
 
