@@ -173,10 +173,11 @@ struct fs_mg_dev {
   LevelDev<float> *lev32 = nullptr;
   double *red = nullptr;                // partial sums
   int per_sm = 0;                       // co-resident CTAs per SM of the multigrid kernels
-  // preconditioner reuse (pc_refresh): the system and precision the coarse
-  // levels and the dense inverse were last built for, and the solves since
+  // preconditioner reuse (pc_refresh): the system, precision and layout (the
+  // V-cycle's, else mesh order) the coarse levels and the dense inverse were
+  // last built for, and the solves since
   int built_nf = 0, age = 0;
-  bool built_f32 = false;
+  bool built_f32 = false, built_vc = false;
   // the Krylov launch a deferred solve prepared (pc_defer): its arguments and
   // form (fs_pc_batch_form), for fs_pc_batch_launch
   AmgKArgs<double> pend64{};
@@ -1361,9 +1362,9 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   const bool vc = gs || fused;
   if (vc && (rc = mg_vc_build(ctx, f32))) return rc;
   const int refresh = std::max(1, ctx->cfg.pc_refresh);
-  const bool reuse = M->built_nf == nf && M->built_f32 == f32 && M->age + 1 < refresh;
+  const bool reuse = M->built_nf == nf && M->built_f32 == f32 && M->built_vc == vc && M->age + 1 < refresh;
   if (reuse) M->age++;
-  else { M->built_nf = nf; M->built_f32 = f32; M->age = 0; }
+  else { M->built_nf = nf; M->built_f32 = f32; M->built_vc = vc; M->age = 0; }
   if (vc) {
     if ((rc = mg_vc_values(ctx, f32, reuse))) return rc;
   } else if (!reuse) {
