@@ -438,7 +438,7 @@ struct PCycle {
         });
       if (!to_out) sweeps(l, in, L.r, post - 1);
     }
-    if (post > 1) {
+    if (post > 1 || lc == 0) {   // a hierarchy of level 0 alone has no up leg that writes out
       enter(g);
       const LevelDev<R> L0 = lev[0];
       for (long i = g.tid0(); i < L0.n; i += g.nth()) out[i] = (double)L0.r[i];
