@@ -158,6 +158,25 @@ static void free_all(fs_ctx *c) {
                   c->ac3, c->bc3, c->ac3P, c->bc3P, c->x3P, c->gm, c->d_bset, c->flow, c->bdir,
                   c->bpcoefc, c->bgd, c->bp0, c->d_patch, c->hist};
   for (void *p : ptrs) if (p) cudaFree(p);
+  if (c->h_status) cudaFreeHost(c->h_status);
+}
+
+int fs_status_fetch(fs_ctx *ctx) {
+  if (ctx->wait_open)
+    FS_CK(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->st));
+  return FS_OK;
+}
+
+static int wait_timed_out(fs_ctx *ctx) {
+  FS_CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int32_t), ctx->st));
+  ctx->err = "a bounded device wait (multigrid barrier or tensor-core completion) timed out";
+  return FS_E_TIMEOUT;
+}
+
+int fs_status_check(fs_ctx *ctx) {
+  if (!ctx->wait_open) return FS_OK;
+  ctx->wait_open = false;
+  return *ctx->h_status ? wait_timed_out(ctx) : FS_OK;
 }
 
 extern "C" {
@@ -222,6 +241,7 @@ int fs_create(const fs_mesh_in *mesh, const fs_case *cfg, int device, fs_ctx **o
   if (cudaMalloc(&ctx->d_iters, sizeof(int32_t) * FS_NITERS) != cudaSuccess) return fail(FS_E_NOMEM);
   cudaMemsetAsync(ctx->d_iters, 0, sizeof(int32_t) * FS_NITERS, ctx->st);
   if (cudaMalloc(&ctx->d_status, sizeof(int32_t) * 8) != cudaSuccess) return fail(FS_E_NOMEM);
+  if (cudaHostAlloc((void **)&ctx->h_status, sizeof(int32_t), cudaHostAllocDefault) != cudaSuccess) return fail(FS_E_NOMEM);
   cudaMemsetAsync(ctx->d_status, 0, sizeof(int32_t) * 8, ctx->st);
   if ((rc = alloc0(ctx, &ctx->flow, 1 + 2 * FS_MAX_PATCHES))) return fail(rc);
   if (cudaMalloc(&ctx->d_bset, sizeof(int32_t) * (B ? B : 1)) != cudaSuccess) return fail(FS_E_NOMEM);
@@ -446,15 +466,10 @@ static int read_residuals(fs_ctx *ctx, fs_residuals *res) {
   int32_t it[FS_NITERS];
   FS_CK(cudaMemcpyAsync(rb, ctx->resblk, sizeof(rb), cudaMemcpyDeviceToHost, ctx->st));
   FS_CK(cudaMemcpyAsync(it, ctx->d_iters, sizeof(it), cudaMemcpyDeviceToHost, ctx->st));
-  int32_t status = 0;
-  FS_CK(cudaMemcpyAsync(&status, ctx->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->st));
+  int rc;
+  if ((rc = fs_status_fetch(ctx))) return rc;
   FS_CK(cudaStreamSynchronize(ctx->st));
-  if (status) {
-    // a bounded device wait gave up: the iteration's results are not valid
-    FS_CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int32_t), ctx->st));
-    ctx->err = "a bounded device wait (multigrid barrier or tensor-core completion) timed out";
-    return FS_E_TIMEOUT;
-  }
+  if ((rc = fs_status_check(ctx))) return rc;
   fs_solver_stats_collect(ctx);
   fs_residuals r{};
   for (int q = 0; q < 5; q++) {
@@ -679,9 +694,10 @@ int fs_solve_system_host(fs_ctx *ctx, const double *ac, const double *anb, const
   int32_t it = 0;
   FS_CK(cudaMemcpyAsync(dphi, fz, sizeof(double) * N, cudaMemcpyDeviceToHost, ctx->st));
   FS_CK(cudaMemcpyAsync(&it, ctx->d_iters + 3, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->st));
+  if ((rc = fs_status_fetch(ctx))) return rc;
   FS_CK(cudaStreamSynchronize(ctx->st));
   if (iters) *iters = it;
-  return FS_OK;
+  return fs_status_check(ctx);
 }
 
 int fs_residuals_get(fs_ctx *ctx, fs_residuals *res) {
@@ -695,8 +711,10 @@ int fs_get_field(fs_ctx *ctx, int field, double *host, size_t n) {
   double *d = field_ptr(ctx, field, &m);
   if (!d || n != m) { ctx->err = "field id or size mismatch"; return FS_E_ARG; }
   FS_CK(cudaMemcpyAsync(host, d, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->st));
+  int rc = fs_status_fetch(ctx);
+  if (rc) return rc;
   FS_CK(cudaStreamSynchronize(ctx->st));
-  return FS_OK;
+  return fs_status_check(ctx);
 }
 
 int fs_set_field(fs_ctx *ctx, int field, const double *host, size_t n) {
@@ -765,8 +783,10 @@ int fs_solver_kernel_ms(fs_ctx *ctx, float *ms5) {
 
 int fs_sync(fs_ctx *ctx) {
   if (!ctx) return FS_E_ARG;
+  int rc = fs_status_fetch(ctx);
+  if (rc) return rc;
   FS_CK(cudaStreamSynchronize(ctx->st));
-  return FS_OK;
+  return fs_status_check(ctx);
 }
 
 // Ensemble of independent cases (no reference counterpart): `iters` SIMPLE
@@ -826,7 +846,9 @@ static int ensemble_run(fs_ctx **cs, int n, int iters, int launches, double *sou
     if (rc) return rc;
     if (mom_b && (rc = fs_mom_batch_create(cs, n, mom_w.data(), &MB))) { fs_pc_batch_free(PB); return rc; }
   }
-  const size_t slot = RB_SIZE + FS_NITERS / 2;  // residual block, then the int32 iteration counts
+  // residual block, then the int32 iteration counts, then the status word of the
+  // bounded waits (copied once a launch, after its last iteration)
+  const size_t slot = RB_SIZE + FS_NITERS / 2 + 1;
   double *h = nullptr;
   FS_CK(cudaHostAlloc((void **)&h, sizeof(double) * slot * n * iters, cudaHostAllocDefault));
   cudaStream_t S = nullptr;
@@ -929,6 +951,8 @@ static int ensemble_run(fs_ctx **cs, int n, int iters, int launches, double *sou
       if ((e = cudaMemcpyAsync(d, c->resblk, sizeof(double) * RB_SIZE, cudaMemcpyDeviceToHost, S)) != cudaSuccess ||
           (e = cudaMemcpyAsync(d + RB_SIZE, c->d_iters, sizeof(int32_t) * FS_NITERS, cudaMemcpyDeviceToHost, S)) !=
               cudaSuccess) { what = "residual copy"; break; }
+      if (t == iters - 1 && (e = cudaMemcpyAsync(d + RB_SIZE + FS_NITERS / 2, c->d_status, sizeof(int32_t),
+                                                 cudaMemcpyDeviceToHost, S)) != cudaSuccess) { what = "status copy"; break; }
     }
   }
   cudaError_t ec = cudaStreamEndCapture(S, &g);
@@ -942,6 +966,13 @@ static int ensemble_run(fs_ctx **cs, int n, int iters, int launches, double *sou
   for (int L = 0; L < launches; L++) {
     if ((e = cudaGraphLaunch(x, S)) != cudaSuccess) return fail("graph launch", e);
     if ((e = cudaStreamSynchronize(S)) != cudaSuccess) return fail("graph run", e);
+    for (int q = 0; q < n; q++) {
+      if (*(const int32_t *)(h + ((size_t)q * iters + iters - 1) * slot + RB_SIZE + FS_NITERS / 2) == 0) continue;
+      const int r = wait_timed_out(cs[q]);
+      if (cs[q] != ctx) ctx->err = cs[q]->err;
+      rc = rc == FS_OK ? r : rc;
+    }
+    if (rc != FS_OK) { cleanup(); return rc; }
     for (int q = 0; q < n; q++)
       for (int t = 0; t < iters; t++) {
         const double *d = h + ((size_t)q * iters + t) * slot;

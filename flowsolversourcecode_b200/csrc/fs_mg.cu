@@ -1347,6 +1347,7 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
     a.gridbar = M->gridbar; a.status = ctx->d_status;
     FS_CK(cudaMemsetAsync(M->gridbar, 0, sizeof(unsigned) * FS_GRIDBAR_WORDS, ctx->st));
     void *args[] = {&a};
+    if (!ctx->graph_mode) ctx->wait_open = true;
     FS_TIMING(FS_CK(cudaEventRecord(ctx->kev[nf - 1][0], ctx->st)));
     FS_CK(fs_coop_launch((const void *)k_mg_solve, G, fs_coop_block(ctx), args, ctx->st));
     FS_LAUNCH_CHECK();
@@ -1403,7 +1404,7 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
     a.gridbar = gridbar;
     a.teambar = (unsigned *)(ctx->d_status + 4);
     a.status = ctx->d_status;
-    a.team_extra = ctx->test_wait_extra;
+    a.team_extra = ctx->test_wait_extra >= 0 ? ctx->test_wait_extra : ctx->graph_mode ? -ctx->test_wait_extra : 0;
   };
   if (ctx->pc_defer && nf == FS_VAR_PC) {   // prepared here, launched with other contexts' by fs_pc_batch_launch
     int form = -1;
@@ -1421,6 +1422,7 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
     }
     return FS_OK;
   }
+  if (!ctx->graph_mode) ctx->wait_open = true;   // graphs copy the status word themselves
   if (!f32) {
     AmgKArgs<double> a{};
     fill(a);
@@ -1495,10 +1497,12 @@ extern "C" int fs_mg_coarse_matrix(fs_ctx *ctx, int level, double *ac, int32_t *
 }
 
 // Test of the bounded device waits (no reference counterpart): with extra > 0
-// the grid barriers of the AMG solves wait for more CTAs than take part, so their
-// polls run out; the solve then ends and the iteration reports FS_E_TIMEOUT.
+// the grid barriers of the AMG solves wait for more CTAs than take part (with
+// extra < 0 those of solves inside a captured graph alone), so their polls run
+// out; the solve then ends and the call that reads its results reports
+// FS_E_TIMEOUT.
 extern "C" int fs_test_wait_timeout(fs_ctx *ctx, int extra) {
-  if (!ctx || extra < 0 || extra > 64) return FS_E_ARG;
+  if (!ctx || extra < -64 || extra > 64) return FS_E_ARG;
   ctx->test_wait_extra = extra;
   return FS_OK;
 }

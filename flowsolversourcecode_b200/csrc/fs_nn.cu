@@ -815,6 +815,7 @@ static int nn_features(fs_ctx *ctx) {
 static int nn_forward(fs_ctx *ctx, const float *X, const float *wgt, bool train) {
   fs_nn *nn = ctx->nn;
   const int N = ctx->N, W = ctx->W;
+  ctx->wait_open = true;   // the layers wait for the tensor core, with a bound
   k_nn_in_fwd<<<fs_grid((long)N * NN_H), FS_BLOCK, 0, ctx->st>>>(N, X, nn->theta, nn->H[0], train ? nn->mask[0] : nullptr);
   FS_LAUNCH_CHECK();
   const int tiles = (N + NN_TM - 1) / NN_TM;
@@ -1104,7 +1105,9 @@ extern "C" int fs_nn_train(fs_ctx *ctx, int epochs, float lr, uint64_t seed, flo
       if ((rc = nn_pack(ctx))) return rc;
       double l = 0.;
       FS_CK(cudaMemcpyAsync(&l, nn->sc + 7, sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
+      if ((rc = fs_status_fetch(ctx))) return rc;
       FS_CK(cudaStreamSynchronize(ctx->st));
+      if ((rc = fs_status_check(ctx))) return rc;
       lsum += l / (nn->snap_tt[s] > 0. ? nn->snap_tt[s] : 1.);
     }
     float lm = (float)(lsum / nn->count);
@@ -1152,9 +1155,10 @@ extern "C" int fs_nn_eval_host(fs_ctx *ctx, const float *X, const float *wgt, co
     if (loss) *loss = (float)(l / (tt > 0. ? tt : 1.));
     if (grad) FS_CK(cudaMemcpy(grad, nn->grad, sizeof(float) * NN_NP, cudaMemcpyDeviceToHost));
   }
+  if ((rc = fs_status_fetch(ctx))) return rc;
   FS_CK(cudaStreamSynchronize(ctx->st));
   if (y) FS_CK(cudaMemcpy(y, nn->y, sizeof(float) * N, cudaMemcpyDeviceToHost));
-  return FS_OK;
+  return fs_status_check(ctx);
 }
 
 extern "C" int fs_nn_policy(fs_ctx *ctx, double *avg_guessed, double *avg_zero, int32_t *parked) {

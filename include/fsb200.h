@@ -15,7 +15,10 @@
  *     face index b = sum(NBFaces(s<set)) + j is the reference's
  *     i4-NIFaces (AssembleGolbalElementAndFaceFluxes.for:83-92).
  *   - Every call returns an int status: FS_OK (0) or a negative FS_E_* code.
- *     Nothing traps; device waits are bounded and report FS_E_TIMEOUT.
+ *     Nothing traps; device waits are bounded, and the call that hands the
+ *     results of a solve whose wait gave up to the host (an outer iteration's
+ *     residuals, fs_solve_system_host, fs_get_field, fs_sync, fs_nn_eval_host, an
+ *     ensemble run) reports FS_E_TIMEOUT, once.
  *   - Character dummies of the reference (Variable, solver, schemes) become
  *     the integer enums below.
  *   - One context is single-caller and non-reentrant (one CUDA stream).
@@ -552,9 +555,10 @@ int fs_nn_policy(fs_ctx *ctx, double *avg_guessed, double *avg_zero, int32_t *pa
 int fs_set_launch_shape(fs_ctx *ctx, int shape);
 /* Test of the bounded device waits (no reference counterpart): with extra > 0
  * the AMG solver's grid barriers wait for `extra` more CTAs than take
- * part, so their bounded polls run out (well under a second); the iteration
- * then returns FS_E_TIMEOUT and its results are not valid.  0 restores normal
- * operation. */
+ * part, so their bounded polls run out (well under a second); the call that
+ * reads the results then returns FS_E_TIMEOUT and they are not valid.  With
+ * extra < 0 only the solves of an ensemble's captured graph wait for -extra
+ * more.  0 restores normal operation. */
 int fs_test_wait_timeout(fs_ctx *ctx, int extra);
 int fs_ensemble_run(fs_ctx **ctxs, int n, int iters, int launches, double *source_out, int32_t *pc_iters_out,
                     float *ms_out);
