@@ -11,6 +11,7 @@ struct GridState {
   unsigned target;     // arrivals in all when the next barrier opens, less `arrivals`
   unsigned arrivals;   // arrivals per barrier
   unsigned *bar;       // arrival count, zero at launch, never reset
+  long limit;          // polls of a barrier before it reports a timeout
   int32_t *status;     // [0] set when a barrier timed out
   double *part;        // partial sums
   int buf;             // buffer of the next sums
@@ -28,12 +29,13 @@ __device__ __forceinline__ int cta_count() { return (int)gridDim.x; }
 #endif
 // before the first barrier, by every thread; `extra` arrivals never come (only
 // to test the timeout)
-__device__ __forceinline__ void grid_state_init(double *part, unsigned *bar, int32_t *status, int extra) {
+__device__ __forceinline__ void grid_state_init(double *part, unsigned *bar, int32_t *status, int extra, long limit) {
   if (threadIdx.x == 0) {
     GridState &G = gstate();
     G.target = 0;
     G.arrivals = (unsigned)(cta_count() + extra);
     G.bar = bar;
+    G.limit = limit;
     G.status = status;
     G.part = part;
     G.buf = 0;
@@ -57,6 +59,7 @@ __device__ __noinline__ void grid_barrier() {
     GridState &G = gstate();
     const unsigned target = G.target + G.arrivals;
     unsigned *bar = G.bar;
+    const long limit = G.limit;
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
     long spins = 0;
     unsigned seen;
@@ -65,7 +68,7 @@ __device__ __noinline__ void grid_barrier() {
       if ((int)(seen - target) >= 0) break;
       if ((++spins & 63) == 0) {
         if (*(const volatile int32_t *)G.status != 0) break;
-        if (spins > FS_PC_SPIN_LIMIT) { atomicExch(G.status, 1); break; }
+        if (spins > limit) { atomicExch(G.status, 1); break; }
       }
     }
     G.target = target;
@@ -123,7 +126,9 @@ __device__ __forceinline__ Sum3 grid_sums(Sum3 in) {
 }
 
 struct Sync {
-  __device__ Sync(double *part, unsigned *bar, int32_t *status, int extra) { grid_state_init(part, bar, status, extra); }
+  __device__ Sync(double *part, unsigned *bar, int32_t *status, int extra, long limit) {
+    grid_state_init(part, bar, status, extra, limit);
+  }
   __device__ __forceinline__ void gbar() { grid_barrier(); }
   __device__ __forceinline__ void all() { grid_barrier(); }
   __device__ __forceinline__ void sum2(double a0, double a1, double &o0, double &o1) {
@@ -1141,7 +1146,7 @@ __device__ double rhs_mean(Sync &S, const AmgKArgs<R> &a) {
 template <class R, int NX>
 __device__ __forceinline__ void guess_fit_body(const AmgKArgs<R> a) {
   constexpr int NG = NX * (NX + 1) / 2, K = NG + NX + 1;
-  Sync S(a.part, a.gridbar + FS_GRIDBAR_FIT, a.status, a.team_extra);
+  Sync S(a.part, a.gridbar + FS_GRIDBAR_FIT, a.status, a.team_extra, a.spin_limit);
   const double bmean = rhs_mean(S, a);
   double c[NX];
   bool fell_back;
@@ -1277,7 +1282,7 @@ __device__ __forceinline__ void amg_bicgstab_body(const AmgKArgs<R> &ap) {
     for (int q = threadIdx.x; q < 8 * vstate<R>().npat; q += blockDim.x) pat_offs()[q] = vstate<R>().offs[q];
   }
   const AmgKArgs<R> &a = astate<R>();
-  Sync S(a.part, a.gridbar, a.status, a.team_extra);
+  Sync S(a.part, a.gridbar, a.status, a.team_extra, a.spin_limit);
   unsigned gen = 0;   // team-barrier generation (the counters are zeroed before the launch)
   const int N = a.N;
   Scope g; g.grid = true;

@@ -125,6 +125,7 @@ struct AmgKArgs {
   unsigned *teambar;  // team barrier words of PCycle (zeroed before the launch)
   int32_t *status;    // [0] team-barrier timeout flag
   int team_extra;     // fs_test_wait_timeout
+  long spin_limit;    // polls of a grid barrier before it gives up
 };
 
 // sums of a level's matrix entries that make up the next level's: entry q from
@@ -222,7 +223,13 @@ __device__ double bsum(double v) {
 #ifndef FS_PC_TEAM_MAX
 #define FS_PC_TEAM_MAX 4096   // levels up to this many rows run on the CTA team
 #endif
-#define FS_PC_SPIN_LIMIT (1L << 20)   // polls of a barrier before it reports a timeout
+// Polls of a barrier before it reports a timeout (0.7 s on B200).  Where one CTA
+// or a team works through small levels while the others wait, the sweeps it
+// makes are the user's to choose (mg_pre, mg_post): the grid barrier's limit
+// grows by FS_PHASE_POLLS (0.2 ms) per phase of that work, each of which takes
+// microseconds.
+#define FS_PC_SPIN_LIMIT (1L << 20)
+#define FS_PHASE_POLLS 256L
 #define FS_VC_ROWS 2048        // residuals of a down leg that a CTA keeps in shared memory
 // Level 0's neighbours as a pattern per row: on meshes numbered in rows and
 // planes the offsets of a cell's neighbours take few combinations (27 on a
@@ -413,11 +420,12 @@ struct MgSolveArgs {
   int32_t *iters;
   unsigned *gridbar;
   int32_t *status;
+  long spin_limit;
 };
 
 // AlgebraicMultigrid cycle loop (AlgebraicMultiGridMainRoutine.for:330-345)
 __global__ void __launch_bounds__(FS_COOP_BLOCK) k_mg_solve(MgSolveArgs a) {
-  Sync S(a.part, a.gridbar, a.status, 0);
+  Sync S(a.part, a.gridbar, a.status, 0, a.spin_limit);
   // dphiMG = 0 on every level
   for (int l = 0; l < a.nlev; l++) {
     Scope sc; sc.grid = true;
@@ -1326,6 +1334,17 @@ static int mg_vc_values(fs_ctx *ctx, bool f32, bool level0) {
   return FS_OK;
 }
 
+// phases of one cycle of k_mg_solve (Cycle::run) if CTA 0 did all of it: the
+// visits of a level times its colour passes, residuals, restriction and prolongation
+static long mg_cycle_phases(const fs_mg_dev *M, int type, int pre, int post) {
+  const int L = M->nlev - 1;
+  long visits = 2L * L + 1;
+  if (type != 0) for (int l = L - 1; l >= 1; l--) visits += 2L * (L - l) + 1;
+  if (type == 2) for (int l = 2; l <= L - 1; l++) visits += 2L * (L - l) + 1;
+  const long colours = *std::max_element(M->ncol, M->ncol + M->nlev);
+  return visits * (std::max({pre, post, 1}) * (2 * colours + 1) + 3);
+}
+
 int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   int rc = fs_mg_build(ctx);
   if (rc) return rc;
@@ -1345,6 +1364,7 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
     a.maxcycles = ctx->cfg.mg_max_cycles; a.b0 = ctx->bc; a.x0 = ctx->dphi; a.r0 = M->r[0];
     a.rrf = rrf; a.ires = ctx->resblk + RB_ABS + (nf - 1); a.part = M->red; a.iters = ctx->d_iters + (nf - 1);
     a.gridbar = M->gridbar; a.status = ctx->d_status;
+    a.spin_limit = FS_PC_SPIN_LIMIT + FS_PHASE_POLLS * mg_cycle_phases(M, a.type, a.pre, a.post);
     FS_CK(cudaMemsetAsync(M->gridbar, 0, sizeof(unsigned) * FS_GRIDBAR_WORDS, ctx->st));
     void *args[] = {&a};
     if (!ctx->graph_mode) ctx->wait_open = true;
@@ -1402,6 +1422,9 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
     a.fit = ctx->d_status + 6;
     a.nncnt = ctx->pc_nn ? fs_nn_counters(ctx) : nullptr;   // the network's guess is in the basis
     a.gridbar = gridbar;
+    // PCycle's team and CTA 0 work on the coarse levels alone: their sweeps of two phases,
+    // restrictions, prolongations and the coarsest level's 20 sweeps
+    a.spin_limit = FS_PC_SPIN_LIMIT + (vc ? 0 : FS_PHASE_POLLS * ((2L * (a.pre + (long)a.post) + 4) * M->lc + 48));
     a.teambar = (unsigned *)(ctx->d_status + 4);
     a.status = ctx->d_status;
     a.team_extra = ctx->test_wait_extra >= 0 ? ctx->test_wait_extra : ctx->graph_mode ? -ctx->test_wait_extra : 0;

@@ -79,3 +79,20 @@ def test_ensemble_run_reports(batched):
     ens = E.Ensemble([E.build_case(q) for q in specs])
     assert np.all(np.isfinite(ens.run(iters=2, launches=1, batched=batched)["source"]))
     ens.close()
+
+
+def test_long_serial_work_is_not_a_timeout():
+    """CTA 0 does every level of this mesh alone, here for seconds a cycle, while
+    the other CTAs wait at a barrier: their limit follows the sweeps asked for."""
+    from flowsolversourcecode_b200 import mesh as fm
+    from flowsolversourcecode_b200.solver import Solver
+    _, case = cs.cavity(4, mg_post=40000, mg_max_cycles=1)
+    s = Solver(fm.box_mesh(12, 12, 12), case)
+    ac, anb, b = _system(s)
+    x, it = s.solve_system(ac, anb, b, rrf=1e-300, solver="amg")
+    assert it == 1
+    cn = s.connectivity()["cn"].reshape(s.W, s.N)
+    r = b - ac * x - np.where(cn >= 0, anb.reshape(s.W, s.N) * x[np.maximum(cn, 0)], 0.0).sum(axis=0)
+    # so many sweeps leave rounding: a few units of 1e-16 times the row sums over |b|
+    assert np.abs(r).max() < 1e-12 * np.abs(b).max()
+    s.close()
