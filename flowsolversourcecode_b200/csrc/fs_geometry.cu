@@ -204,7 +204,7 @@ static void build_colors(fs_ctx *ctx) {
 template <class T>
 static int up(fs_ctx *ctx, T **d, const T *h, size_t n) {
   FS_CK(cudaMalloc((void **)d, std::max<size_t>(n, 1) * sizeof(T)));
-  if (n) FS_CK(cudaMemcpy(*d, h, n * sizeof(T), cudaMemcpyHostToDevice));
+  if (n) FS_CK(fs_upload(ctx, *d, h, n * sizeof(T)));
   return FS_OK;
 }
 
@@ -369,7 +369,7 @@ int fs_geometry_build(fs_ctx *ctx, const fs_mesh_in *mi) {
   FS_CK(cudaMalloc(&d_bfc, sizeof(double) * 3 * std::max(B, 1)));
   auto dal = [&](double **p, size_t n) -> int {
     FS_CK(cudaMalloc((void **)p, sizeof(double) * std::max<size_t>(n, 1)));
-    FS_CK(cudaMemset(*p, 0, sizeof(double) * std::max<size_t>(n, 1)));
+    FS_CK(cudaMemsetAsync(*p, 0, sizeof(double) * std::max<size_t>(n, 1), ctx->st));
     return FS_OK;
   };
   if ((rc = dal(&ctx->vol, N)) || (rc = dal(&ctx->xc, 3L * N)) || (rc = dal(&ctx->gf, F)) ||

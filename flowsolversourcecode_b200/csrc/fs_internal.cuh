@@ -240,6 +240,16 @@ static inline cudaError_t fs_coop_launch(const void *fn, int grid, int block, vo
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
+// Host arrays go to the device on the context's stream.  That stream does not
+// wait for the default one, and a copy from pageable memory on the default
+// stream may still be under way when the call returns, so a table uploaded there
+// could reach a kernel of the context half filled.  Returns when the copy is done:
+// the host array may go.
+static inline cudaError_t fs_upload(fs_ctx *ctx, void *d, const void *h, size_t bytes) {
+  cudaError_t e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, ctx->st);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(ctx->st);
+}
+
 static inline int fs_grid(long n, int block = FS_BLOCK) {
   long g = (n + block - 1) / block;
   return (int)(g < 1 ? 1 : g);

@@ -876,7 +876,7 @@ static std::vector<int32_t> color_level(const HostLevel &L, int &ncol) {
 template <class T>
 static int upv(fs_ctx *ctx, T **d, const std::vector<T> &h) {
   FS_CK(cudaMalloc((void **)d, std::max<size_t>(h.size(), 1) * sizeof(T)));
-  if (!h.empty()) FS_CK(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+  if (!h.empty()) FS_CK(fs_upload(ctx, *d, h.data(), h.size() * sizeof(T)));
   return FS_OK;
 }
 
@@ -941,7 +941,7 @@ int fs_mg_build(fs_ctx *ctx) {
     else {
       FS_CK(cudaMalloc(&M->ac[q], sizeof(double) * n));
       FS_CK(cudaMalloc(&M->anb[q], sizeof(double) * nw));
-      FS_CK(cudaMemset(M->anb[q], 0, sizeof(double) * nw));
+      FS_CK(cudaMemsetAsync(M->anb[q], 0, sizeof(double) * nw, ctx->st));
     }
     FS_CK(cudaMalloc(&M->b[q], sizeof(double) * n));
     FS_CK(cudaMalloc(&M->x[q], sizeof(double) * n));
@@ -971,9 +971,9 @@ int fs_mg_build(fs_ctx *ctx) {
     L32[q] = e;
   }
   FS_CK(cudaMalloc(&M->lev64, sizeof(LevelDev<double>) * M->nlev));
-  FS_CK(cudaMemcpy(M->lev64, L64.data(), sizeof(LevelDev<double>) * M->nlev, cudaMemcpyHostToDevice));
+  FS_CK(fs_upload(ctx, M->lev64, L64.data(), sizeof(LevelDev<double>) * M->nlev));
   FS_CK(cudaMalloc(&M->lev32, sizeof(LevelDev<float>) * M->nlev));
-  FS_CK(cudaMemcpy(M->lev32, L32.data(), sizeof(LevelDev<float>) * M->nlev, cudaMemcpyHostToDevice));
+  FS_CK(fs_upload(ctx, M->lev32, L32.data(), sizeof(LevelDev<float>) * M->nlev));
   FS_CK(cudaMalloc(&M->red, sizeof(double) * (6 + FS_SUMK + 9) * FS_RED_BLOCKS));
   FS_CK(cudaMalloc(&M->gridbar, sizeof(unsigned) * FS_GRIDBAR_WORDS));
   for (int q = 1; q < M->nlev; q++) {
@@ -1008,7 +1008,6 @@ int fs_mg_build(fs_ctx *ctx) {
   int per = std::min(std::min(a, std::min(b, c)), std::min(std::min(b2, c2), c3));
   if (per < 1) { ctx->err = "multigrid kernels do not fit on an SM"; return FS_E_CUDA; }
   M->per_sm = per;   // occupancy limit; the grid follows the launch shape at each solve
-  FS_CK(cudaStreamSynchronize(cudaStreamLegacy));   // the uploads, before the solver's stream reads them
   return FS_OK;
 }
 
@@ -1270,8 +1269,9 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
     M->vx[f32][0] = take(es * M->n[1]);   // the result of level 1
   }
   for (int l = 1; l <= lc; l++) {
-    if (l < lc) FS_CK(cudaMemcpy(kp[l], M->vkp[l], sizeof(int32_t) * (M->n[l + 1] + 1), cudaMemcpyDeviceToDevice));
-    FS_CK(cudaMemcpy(col[l], M->vcol[l], sizeof(int32_t) * M->vnpos[l], cudaMemcpyDeviceToDevice));
+    if (l < lc)
+      FS_CK(cudaMemcpyAsync(kp[l], M->vkp[l], sizeof(int32_t) * (M->n[l + 1] + 1), cudaMemcpyDeviceToDevice, ctx->st));
+    FS_CK(cudaMemcpyAsync(col[l], M->vcol[l], sizeof(int32_t) * M->vnpos[l], cudaMemcpyDeviceToDevice, ctx->st));
   }
   auto own = [&](auto **d, size_t n) -> int {
     FS_CK(cudaMalloc((void **)d, sizeof(**d) * std::max<size_t>(n, 1)));
@@ -1306,13 +1306,12 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
     v.par0 = M->par0;
     v.npat = M->npat; v.pat = M->pat; v.patL = M->patL; v.offs = M->offs;
     FS_CK(cudaMalloc(dev, sizeof(VcDev<R>)));
-    FS_CK(cudaMemcpy(*dev, &v, sizeof(VcDev<R>), cudaMemcpyHostToDevice));
+    FS_CK(fs_upload(ctx, *dev, &v, sizeof(VcDev<R>)));
     return FS_OK;
   };
   if (f32) rc = desc((float *)nullptr, &M->vc32, M->lev32);
   else rc = desc((double *)nullptr, &M->vc64, M->lev64);
   if (rc) return rc;
-  FS_CK(cudaStreamSynchronize(cudaStreamLegacy));   // the uploads, before the solver's stream reads them
   M->vc_ready[f32] = true;
   return FS_OK;
 }
@@ -1609,7 +1608,7 @@ int fs_pc_batch_create(fs_ctx **cs, int n, const double *weight, fs_pc_batch **o
       (e = cudaMalloc(&B->d_args, B->argsz * n)) != cudaSuccess ||
       (e = cudaMalloc(&B->d_start, sizeof(int32_t) * (n + 1))) != cudaSuccess ||
       (e = cudaMalloc(&B->d_words, sizeof(unsigned) * (FS_GRIDBAR_WORDS + 2) * n)) != cudaSuccess ||
-      (e = cudaMemcpy(B->d_start, B->start.data(), sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice)) != cudaSuccess) {
+      (e = fs_upload(ctx, B->d_start, B->start.data(), sizeof(int32_t) * (n + 1))) != cudaSuccess) {
     ctx->err = std::string("batched p' set-up: ") + cudaGetErrorString(e);
     fs_pc_batch_free(B);
     return FS_E_CUDA;

@@ -1006,7 +1006,7 @@ extern "C" int fs_nn_create(fs_ctx *ctx, int snapshot_capacity, uint64_t seed) {
   nn->N = N; nn->W = W;
   auto al = [&](void **p, size_t bytes) -> int {
     FS_CK(cudaMalloc(p, std::max<size_t>(bytes, 16)));
-    FS_CK(cudaMemset(*p, 0, std::max<size_t>(bytes, 16)));
+    FS_CK(cudaMemsetAsync(*p, 0, std::max<size_t>(bytes, 16), ctx->st));
     return FS_OK;
   };
   int rc = 0;
@@ -1054,9 +1054,6 @@ extern "C" int fs_nn_create(fs_ctx *ctx, int snapshot_capacity, uint64_t seed) {
     std::normal_distribution<float> d(0.f, 0.5f * sqrtf(2.f / NN_K));
     for (int q = 0; q < NN_K * NN_H; q++) th[NN_OFF_L(l) + q] = d(gen);
   }
-  // the clears above went to the default stream, which the solver's stream does
-  // not wait for; from here on copies go to the solver's stream
-  FS_CK(cudaStreamSynchronize(cudaStreamLegacy));
   FS_CK(cudaMemcpyAsync(nn->theta, th.data(), sizeof(float) * NN_NP, cudaMemcpyHostToDevice, ctx->st));
   FS_CK(cudaFuncSetAttribute((const void *)k_nn_layer_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)NN_SMEM_FWD));
@@ -1123,8 +1120,6 @@ extern "C" int fs_nn_params(fs_ctx *ctx, float *get, const float *set, size_t n)
   FS_CK(cudaStreamSynchronize(ctx->st));
   if (get) FS_CK(cudaMemcpy(get, ctx->nn->theta, sizeof(float) * NN_NP, cudaMemcpyDeviceToHost));
   if (set) {
-    // on the solver's stream: a copy from pageable memory on another one may
-    // still be under way when it returns, and the packing reads theta
     FS_CK(cudaMemcpyAsync(ctx->nn->theta, set, sizeof(float) * NN_NP, cudaMemcpyHostToDevice, ctx->st));
     int rc = nn_pack(ctx);
     if (rc) return rc;

@@ -992,7 +992,7 @@ static int pbcg_build(fs_ctx *ctx) {
     }
   auto up = [&](int32_t **d, const std::vector<int32_t> &h) -> int {
     FS_CK(cudaMalloc((void **)d, std::max<size_t>(h.size(), 1) * sizeof(int32_t)));
-    if (!h.empty()) FS_CK(cudaMemcpy(*d, h.data(), h.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    if (!h.empty()) FS_CK(fs_upload(ctx, *d, h.data(), h.size() * sizeof(int32_t)));
     return FS_OK;
   };
   int rc;
@@ -1044,7 +1044,7 @@ static int ilu_build(fs_ctx *ctx) {
   I->nlf = nlf; I->nlb = nlb;
   auto up = [&](int32_t **d, const std::vector<int32_t> &h) -> int {
     FS_CK(cudaMalloc((void **)d, std::max<size_t>(h.size(), 1) * sizeof(int32_t)));
-    if (!h.empty()) FS_CK(cudaMemcpy(*d, h.data(), h.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    if (!h.empty()) FS_CK(fs_upload(ctx, *d, h.data(), h.size() * sizeof(int32_t)));
     return FS_OK;
   };
   int rc;
@@ -1436,8 +1436,8 @@ int fs_mom_batch_create(fs_ctx **cs, int n, const double *weight, fs_mom_batch *
       (e = cudaMalloc(&B->d_start, sizeof(int32_t) * (n + 1))) != cudaSuccess ||
       (e = cudaMalloc(&B->d_words, sizeof(unsigned) * 2 * n)) != cudaSuccess ||
       (e = cudaMalloc(&B->d_status, sizeof(int32_t *) * n)) != cudaSuccess ||
-      (e = cudaMemcpy(B->d_start, start.data(), sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(B->d_status, st.data(), sizeof(int32_t *) * n, cudaMemcpyHostToDevice)) != cudaSuccess) {
+      (e = fs_upload(ctx, B->d_start, start.data(), sizeof(int32_t) * (n + 1))) != cudaSuccess ||
+      (e = fs_upload(ctx, B->d_status, st.data(), sizeof(int32_t *) * n)) != cudaSuccess) {
     ctx->err = std::string("batched momentum set-up: ") + cudaGetErrorString(e);
     fs_mom_batch_free(B);
     return FS_E_CUDA;
