@@ -1085,6 +1085,23 @@ static size_t vc_pos(int l, int n, int w, int a, int j) {
   return l == 0 ? (size_t)j * n + a : ((size_t)(a / 32) * w + j) * 32 + a % 32;
 }
 
+// the V-cycle's number of every row of levels 0..lc: aggregate by aggregate, within
+// an aggregate in ascending original order; the coarsest level keeps its numbering
+static std::vector<std::vector<int32_t>> vc_numbers(const fs_mg_dev *M) {
+  std::vector<std::vector<int32_t>> id(M->lc + 1);
+  id[M->lc].resize(M->n[M->lc]);
+  for (int i = 0; i < M->n[M->lc]; i++) id[M->lc][i] = i;
+  for (int l = M->lc - 1; l >= 0; l--) {
+    const std::vector<int32_t> &par = M->h_parent[l], &up = id[l + 1];
+    std::vector<int32_t> at(M->n[l + 1] + 1, 0);
+    for (int i = 0; i < M->n[l]; i++) at[up[par[i]] + 1]++;
+    for (int P = 0; P < M->n[l + 1]; P++) at[P + 1] += at[P];
+    id[l].resize(M->n[l]);
+    for (int i = 0; i < M->n[l]; i++) id[l][i] = at[up[par[i]]]++;
+  }
+  return id;
+}
+
 // the entries of level l-1 that each entry and diagonal of level l sums, in the
 // reference's order (children in list order, a child's diagonal, then its slots)
 static int mg_vc_sums(fs_ctx *ctx, int l, const std::vector<int32_t> &idf, const std::vector<int32_t> &idc) {
@@ -1181,23 +1198,18 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
   const int lc = M->lc;
   int rc;
   if (!M->vc_map) {
-    std::vector<int32_t> up(M->n[lc]), id;   // new numbers of the coarser level, of this one
-    std::vector<std::vector<int32_t>> ids(lc + 1);
-    for (int i = 0; i < M->n[lc]; i++) up[i] = i;
+    const std::vector<std::vector<int32_t>> ids = vc_numbers(M);
     for (int l = lc; l >= 0; l--) {
+      const std::vector<int32_t> &id = ids[l];
       const int n = M->n[l];
       const std::vector<int32_t> &nnb = l ? M->h_nnb[l] : ctx->h_ncf, &nbr = l ? M->h_nbr[l] : ctx->h_cn;
       std::vector<int32_t> row(n);           // original row of each new one
-      if (l == lc) id = up;
-      else {
-        const std::vector<int32_t> &par = M->h_parent[l];
+      if (l < lc) {
+        const std::vector<int32_t> &par = M->h_parent[l], &up = ids[l + 1];
         const int nc = M->n[l + 1];
         std::vector<int32_t> kp(nc + 1, 0);
         for (int i = 0; i < n; i++) kp[up[par[i]] + 1]++;
         for (int P = 0; P < nc; P++) kp[P + 1] += kp[P];
-        std::vector<int32_t> at(kp.begin(), kp.end() - 1);
-        id.resize(n);
-        for (int i = 0; i < n; i++) id[i] = at[up[par[i]]]++;
         if ((rc = upv(ctx, &M->vkp[l], kp))) return rc;
         if (l == 0) {
           std::vector<int32_t> p0(n);
@@ -1222,8 +1234,6 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
       }
       M->vnpos[l] = (int)col.size();
       if ((rc = upv(ctx, &M->vcol[l], col)) || (rc = upv(ctx, &M->vrow[l], row))) return rc;
-      ids[l] = id;
-      up.swap(id);
     }
     for (int l = 1; l <= lc; l++)
       if ((rc = mg_vc_sums(ctx, l, ids[l - 1], ids[l]))) return rc;
@@ -1516,6 +1526,33 @@ extern "C" int fs_mg_coarse_matrix(fs_ctx *ctx, int level, double *ac, int32_t *
   FS_CK(cudaMemcpyAsync(nbr, M->nbr[level], sizeof(int32_t) * n * w, cudaMemcpyDeviceToHost, ctx->st));
   FS_CK(cudaStreamSynchronize(ctx->st));
   return FS_OK;
+}
+
+// The same level as the one-phase V-cycle holds it, in the numbering and slots of
+// fs_mg_coarse_matrix (0 in the slots past n_nbr; f32: the FP32 cycle's copy).
+// For tests: the two are assembled by different kernels.
+extern "C" int fs_mg_vcycle_matrix(fs_ctx *ctx, int level, int f32, double *ac, double *anb, size_t n, size_t w) {
+  if (!ctx || !ac || !anb) return FS_E_ARG;
+  int rc = fs_mg_build(ctx);
+  if (rc) return rc;
+  fs_mg_dev *M = ctx->mg;
+  if (!M->direct || level < 1 || level > M->lc || n != (size_t)M->n[level] || w != (size_t)M->w[level]) return FS_E_ARG;
+  cudaSetDevice(ctx->dev);
+  if ((rc = mg_vc_build(ctx, f32 != 0)) || (rc = mg_vc_values(ctx, f32 != 0, false))) return rc;
+  M->built_nf = 0;   // the coarse levels are this system's now
+  auto read = [&](auto *dac, auto *dval) -> int {
+    std::vector<std::remove_pointer_t<decltype(dac)>> a(n), v(M->vnpos[level]);
+    FS_CK(cudaMemcpyAsync(a.data(), dac, sizeof(a[0]) * a.size(), cudaMemcpyDeviceToHost, ctx->st));
+    FS_CK(cudaMemcpyAsync(v.data(), dval, sizeof(v[0]) * v.size(), cudaMemcpyDeviceToHost, ctx->st));
+    FS_CK(cudaStreamSynchronize(ctx->st));
+    const std::vector<int32_t> id = vc_numbers(M)[level];
+    for (size_t i = 0; i < n; i++) {
+      ac[i] = a[id[i]];
+      for (size_t j = 0; j < w; j++) anb[j * n + i] = v[vc_pos(level, (int)n, (int)w, id[i], (int)j)];
+    }
+    return FS_OK;
+  };
+  return f32 ? read(M->vacf[level], M->vvalf[level]) : read(M->vac[level], M->vval[level]);
 }
 
 // Test of the bounded device waits (no reference counterpart): with extra > 0

@@ -503,6 +503,11 @@ int fs_mg_info(fs_ctx *ctx, int32_t *widths, int max_levels, int32_t *prec_coars
  * w the level's size and ELL width (fs_mg_levels, fs_mg_info). */
 int fs_mg_coarse_matrix(fs_ctx *ctx, int level, double *ac, int32_t *n_nbr, int32_t *nbr, double *anb,
                         size_t n, size_t w);
+/* The same level (1 .. the preconditioner's coarsest) as the one-phase V-cycle of
+ * the AMG-BiCGSTAB solvers holds it, in the numbering and slots of
+ * fs_mg_coarse_matrix: ac [n], anb [w*n]; f32: the FP32 cycle's copy.  For tests;
+ * needs a level small enough for the dense inverse. */
+int fs_mg_vcycle_matrix(fs_ctx *ctx, int level, int f32, double *ac, double *anb, size_t n, size_t w);
 
 /* ----------------------------------------------------- learned p' initial guess
  * No reference counterpart: the reference starts every p' solve from zero.
