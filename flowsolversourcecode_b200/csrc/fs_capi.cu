@@ -223,7 +223,7 @@ int fs_create(const fs_mesh_in *mesh, const fs_case *cfg, int device, fs_ctx **o
     return fail(rc);
   double **cell3[] = {&ctx->ug, &ctx->vg, &ctx->wg, &ctx->pg, &ctx->pcg, &ctx->bc_int};
   for (auto p : cell3) if ((rc = alloc0(ctx, p, 3 * N))) return fail(rc);
-  if ((rc = alloc0(ctx, &ctx->gtmp, 12 * N))) return fail(rc);
+  if ((rc = alloc0(ctx, &ctx->gtmp, FS_GTMP_BLOCKS * N))) return fail(rc);
   if ((rc = alloc0(ctx, &ctx->anb, W * N))) return fail(rc);
   if ((rc = alloc0(ctx, &ctx->mdot, F)) || (rc = alloc0(ctx, &ctx->pcoef, F)) || (rc = alloc0(ctx, &ctx->bpcoef, B)) ||
       (rc = alloc0(ctx, &ctx->bpcoefc, B)) || (rc = alloc0(ctx, &ctx->bgd, B)) || (rc = alloc0(ctx, &ctx->bp0, B)) ||

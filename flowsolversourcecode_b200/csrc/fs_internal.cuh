@@ -67,6 +67,7 @@ struct fs_energy;  // temperature equation state (fs_energy.cu)
 struct fs_nn;      // learned p' initial guess (fs_nn.cu)
 struct fs_ilu;     // D-ILU level schedule (fs_solvers.cu)
 
+#define FS_GTMP_BLOCKS 12   // N-sized blocks of the gradient scratch
 #define FS_NEQ 9        // equations with residual slots: NF 1..9
 #define FS_NLEVELS 7    // unsteady time levels: u v w p k epsilon T
 #define FS_GUESS_MAX 8  // vectors of the p' initial-guess fit (history + the network's guess)
@@ -111,7 +112,7 @@ struct fs_ctx {
   double *bu = nullptr, *bv = nullptr, *bw = nullptr, *bp = nullptr, *bpc = nullptr, *bmdot = nullptr;
   double *ug = nullptr, *vg = nullptr, *wg = nullptr, *pg = nullptr, *pcg = nullptr;      // 3N
   double *bug = nullptr, *bvg = nullptr, *bwg = nullptr, *bpg = nullptr, *bpcg = nullptr; // 3B
-  double *gtmp = nullptr;                                  // 12N double buffer for GG passes
+  double *gtmp = nullptr;                                  // FS_GTMP_BLOCKS N double buffer for GG passes
   double *du1 = nullptr, *dv1 = nullptr, *dw1 = nullptr, *du2 = nullptr, *dv2 = nullptr, *dw2 = nullptr;
   double *us = nullptr, *vs = nullptr, *ws = nullptr;
 

@@ -33,6 +33,7 @@
 #include "fs_internal.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <type_traits>
 
@@ -109,7 +110,7 @@ struct AmgKArgs {
   const int32_t *ncf, *cn;
   const double *ac, *anb, *bc;
   double *x, *r, *r0, *p, *v, *s, *t, *y, *z, *dphi;
-  const LevelDev<R> *lev;
+  const LevelDev<R> *lev;   // with the one-phase V-cycle level 0 alone
   const VcDev<R> *vc;
   int lc, direct, pre, post, maxit;
   const double *sinv;
@@ -135,30 +136,19 @@ struct CoarseSums {
 };
 
 struct fs_mg_dev {
+  // hierarchy (host)
   int nlev = 0;
-  // V-cycle layout (mg_vc_build): maps and index arrays, values per precision
-  bool vc_map = false, vc_ready[2] = {false, false};
-  // coarse connectivity and child lists until then
-  std::vector<int32_t> h_nnb[FS_MG_MAXLEV], h_nbr[FS_MG_MAXLEV], h_cptr[FS_MG_MAXLEV], h_clist[FS_MG_MAXLEV];
-  int32_t *vcol[FS_MG_MAXLEV] = {}, *vrow[FS_MG_MAXLEV] = {}, *vkp[FS_MG_MAXLEV] = {}, *par0 = nullptr;
-  int vnpos[FS_MG_MAXLEV] = {};
-  CoarseSums csum[FS_MG_MAXLEV], cdiag[FS_MG_MAXLEV];   // level l's entries and diagonals from level l-1
-  // matrices in the layout: FP64 of every level, FP32 copies where the V-cycle is FP32; vectors per precision
-  double *vval[FS_MG_MAXLEV] = {}, *vac[FS_MG_MAXLEV] = {};
-  float *vvalf[FS_MG_MAXLEV] = {}, *vacf[FS_MG_MAXLEV] = {};
-  void *vb[2][FS_MG_MAXLEV] = {}, *vx[2][FS_MG_MAXLEV] = {};
-  int npat = 0;                                      // row patterns of level 0
-  uint8_t *pat = nullptr, *patL = nullptr;
-  int32_t *offs = nullptr;
-  unsigned *vbar[2] = {nullptr, nullptr};            // barrier counts, partial sums and coarsest inverse
-  double *vpart[2] = {nullptr, nullptr}, *vinv[2] = {nullptr, nullptr};
-  std::vector<void *> vallocs;
-  VcDev<double> *vc64 = nullptr;
-  VcDev<float> *vc32 = nullptr;
-  unsigned *gridbar = nullptr;
   int n[FS_MG_MAXLEV] = {}, w[FS_MG_MAXLEV] = {}, ncol[FS_MG_MAXLEV] = {};
   std::vector<int32_t> h_parent[FS_MG_MAXLEV];
-  // device
+  std::vector<int32_t> h_nnb[FS_MG_MAXLEV], h_nbr[FS_MG_MAXLEV], h_cptr[FS_MG_MAXLEV], h_clist[FS_MG_MAXLEV];
+  int lc = 0;                           // coarsest level of the preconditioner
+  bool direct = false;                  // lev[lc] inverted densely
+  int per_sm = 0;                       // co-resident CTAs per SM of the multigrid kernels
+  std::vector<void *> allocs;           // device memory of the parts built so far
+  // Mesh order (mg_mesh_build, mg_mesh_vectors): connectivity, matrices and, per
+  // precision, vectors and the FP32 matrices -- for 'amg', the general V-cycle and
+  // fs_mg_coarse_matrix
+  bool mesh_ready = false, mesh_vec[2] = {false, false};
   int32_t *nnb[FS_MG_MAXLEV] = {}, *nbr[FS_MG_MAXLEV] = {}, *parent[FS_MG_MAXLEV] = {};
   int32_t *cptr[FS_MG_MAXLEV] = {}, *clist[FS_MG_MAXLEV] = {}, *cmap[FS_MG_MAXLEV] = {};
   int32_t *rptr[FS_MG_MAXLEV] = {}, *rlist[FS_MG_MAXLEV] = {};
@@ -167,13 +157,27 @@ struct fs_mg_dev {
   double *t[FS_MG_MAXLEV] = {};
   float *acf[FS_MG_MAXLEV] = {}, *anbf[FS_MG_MAXLEV] = {}, *bf[FS_MG_MAXLEV] = {}, *xf[FS_MG_MAXLEV] = {}, *rf[FS_MG_MAXLEV] = {};
   float *tf[FS_MG_MAXLEV] = {};
-  int lc = 0;                           // coarsest level of the preconditioner
-  bool direct = false;                  // lev[lc] inverted densely
   double *sinv = nullptr;
   LevelDev<double> *lev64 = nullptr;
   LevelDev<float> *lev32 = nullptr;
   double *red = nullptr;                // partial sums
-  int per_sm = 0;                       // co-resident CTAs per SM of the multigrid kernels
+  unsigned *gridbar = nullptr;
+  // The one-phase V-cycle's layout (mg_vc_build): maps and index arrays, then
+  // matrices and vectors per precision
+  bool vc_map = false, vc_ready[2] = {false, false};
+  int32_t *vcol[FS_MG_MAXLEV] = {}, *vkp[FS_MG_MAXLEV] = {}, *cells = nullptr, *par0 = nullptr;
+  int vnpos[FS_MG_MAXLEV] = {};
+  CoarseSums csum[FS_MG_MAXLEV], cdiag[FS_MG_MAXLEV];   // level l's entries and diagonals from level l-1
+  // FP64 matrices (the source of the next level's in either precision; level 0's in the FP32 cycle: scratch), FP32 copies
+  double *vval[FS_MG_MAXLEV] = {}, *vac[FS_MG_MAXLEV] = {}, *val0[2] = {}, *ac0[2] = {};
+  float *vvalf[FS_MG_MAXLEV] = {}, *vacf[FS_MG_MAXLEV] = {}, *acm = nullptr, *anbm = nullptr;   // acm, anbm: level 0 in mesh order
+  int npat = 0;                                      // row patterns of level 0
+  uint8_t *pat = nullptr, *patL = nullptr;
+  int32_t *offs = nullptr;
+  unsigned *vbar[2] = {nullptr, nullptr};            // barrier counts, partial sums and coarsest inverse
+  double *vpart[2] = {nullptr, nullptr}, *vinv[2] = {nullptr, nullptr};
+  VcDev<double> *vc64 = nullptr;
+  VcDev<float> *vc32 = nullptr;
   // preconditioner reuse (pc_refresh): the system, precision and layout (the
   // V-cycle's, else mesh order) the coarse levels and the dense inverse were
   // last built for, and the solves since
@@ -230,6 +234,7 @@ __device__ double bsum(double v) {
 // microseconds.
 #define FS_PC_SPIN_LIMIT (1L << 20)
 #define FS_PHASE_POLLS 256L
+#define FS_VC_SLOTS 6          // slots of level 0 that the row patterns give; the others come from the index table
 #define FS_VC_ROWS 2048        // residuals of a down leg that a CTA keeps in shared memory
 // Level 0's neighbours as a pattern per row: on meshes numbered in rows and
 // planes the offsets of a cell's neighbours take few combinations (27 on a
@@ -874,160 +879,171 @@ static std::vector<int32_t> color_level(const HostLevel &L, int &ncol) {
 }
 
 template <class T>
+static int mg_alloc(fs_ctx *ctx, T **d, size_t n) {
+  FS_CK(cudaMalloc((void **)d, std::max<size_t>(n, 1) * sizeof(T)));
+  ctx->mg->allocs.push_back(*d);
+  return FS_OK;
+}
+template <class T>
 static int upv(fs_ctx *ctx, T **d, const std::vector<T> &h) {
-  FS_CK(cudaMalloc((void **)d, std::max<size_t>(h.size(), 1) * sizeof(T)));
+  int rc = mg_alloc(ctx, d, h.size());
+  if (rc) return rc;
   if (!h.empty()) FS_CK(fs_upload(ctx, *d, h.data(), h.size() * sizeof(T)));
   return FS_OK;
 }
 
+// the hierarchy and what follows from it on the host; device memory is
+// allocated by the parts that a solver uses (mg_mesh_*, mg_vc_build)
 int fs_mg_build(fs_ctx *ctx) {
   if (ctx->mg) return FS_OK;
+  // cooperative grid: smallest co-resident count of the kernels
+  int per = INT_MAX;
+  const void *kernels[] = {(const void *)k_mg_solve, (const void *)k_amg_bicgstab<double, 0>,
+                           (const void *)k_amg_bicgstab<float, 0>, (const void *)k_amg_bicgstab<double, 1>,
+                           (const void *)k_amg_bicgstab<float, 1>, (const void *)k_amg_bicgstab<float, 2>};
+  for (const void *k : kernels) {
+    int a = 0;
+    FS_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k, FS_COOP_BLOCK, 0));
+    per = std::min(per, a);
+  }
+  if (per < 1) { ctx->err = "multigrid kernels do not fit on an SM"; return FS_E_CUDA; }
+  // the dense inverse's attribute belongs to the function, shared by every
+  // context of the process: set it for the largest coarsest level any may have
+  const int sm = (int)(sizeof(double) * FS_MG_DIRECT * FS_MG_DIRECT);
+  const void *ks[] = {(const void *)k_mg_dense_inverse<1>, (const void *)k_mg_dense_inverse<2>,
+                      (const void *)k_mg_dense_inverse<3>, (const void *)k_mg_dense_inverse<4>,
+                      (const void *)k_mg_dense_inverse<5>};
+  for (const void *k : ks) FS_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   fs_mg_dev *M = new fs_mg_dev();
   ctx->mg = M;
-  std::vector<HostLevel> H(1);
-  H[0].n = ctx->N; H[0].w = ctx->W; H[0].nnb = ctx->h_ncf; H[0].nbr = ctx->h_cn;
-  std::vector<std::vector<int32_t>> cptr(FS_MG_MAXLEV), clist(FS_MG_MAXLEV);
+  M->per_sm = per;   // occupancy limit; the grid follows the launch shape at each solve
+  HostLevel f;
+  f.n = ctx->N; f.w = ctx->W; f.nnb = ctx->h_ncf; f.nbr = ctx->h_cn;
   int l = 0;
   const int maxlev = std::min(ctx->cfg.mg_max_levels, FS_MG_MAXLEV);
-  while (l + 1 < maxlev && H[l].n > 2 * ctx->cfg.mg_min_parents) {
-    H.emplace_back();
-    agglomerate(H[l], l + 1, H[l + 1], M->h_parent[l], cptr[l], clist[l]);
+  for (;;) {
+    M->n[l] = f.n; M->w[l] = f.w;
+    HostLevel c;
+    const bool more = l + 1 < maxlev && f.n > 2 * ctx->cfg.mg_min_parents;
+    if (more) agglomerate(f, l + 1, c, M->h_parent[l], M->h_cptr[l + 1], M->h_clist[l + 1]);
+    if (l > 0) { M->h_nnb[l] = std::move(f.nnb); M->h_nbr[l] = std::move(f.nbr); }
+    if (!more) break;
+    f = std::move(c);
     l++;
   }
   M->nlev = l + 1;
-  int rc;
-  std::vector<LevelDev<double>> L64(M->nlev);
-  std::vector<LevelDev<float>> L32(M->nlev);
-  for (int q = 0; q < M->nlev; q++) {
-    const HostLevel &h = H[q];
-    M->n[q] = h.n; M->w[q] = h.w;
-    std::vector<int32_t> colors = color_level(h, M->ncol[q]);
-    if ((rc = upv(ctx, &M->colors[q], colors))) return rc;
-    if (q == 0) { M->nnb[0] = ctx->ncf; M->nbr[0] = ctx->cn; }
-    else {
-      if ((rc = upv(ctx, &M->nnb[q], h.nnb))) return rc;
-      if ((rc = upv(ctx, &M->nbr[q], h.nbr))) return rc;
-    }
-    if (q + 1 < M->nlev) {
-      if ((rc = upv(ctx, &M->parent[q], M->h_parent[q]))) return rc;
-      // LHS lists and slot map (fine slot -> coarse slot / internal / none)
-      if ((rc = upv(ctx, &M->cptr[q + 1], cptr[q]))) return rc;
-      if ((rc = upv(ctx, &M->clist[q + 1], clist[q]))) return rc;
-      const HostLevel &c = H[q + 1];
-      std::vector<int32_t> cmap((size_t)h.w * h.n, -1);
-      for (int i = 0; i < h.n; i++) {
-        int P = M->h_parent[q][i];
-        for (int j = 0; j < h.nnb[i]; j++) {
-          int nb = h.nbr[(size_t)j * h.n + i];
-          if (nb < 0) continue;
-          int Q = M->h_parent[q][nb];
-          if (Q == P) { cmap[(size_t)j * h.n + i] = -2; continue; }
-          for (int k = 0; k < c.nnb[P]; k++)
-            if (c.nbr[(size_t)k * c.n + P] == Q) { cmap[(size_t)j * h.n + i] = k; break; }
-        }
-      }
-      if ((rc = upv(ctx, &M->cmap[q + 1], cmap))) return rc;
-      // restriction lists: fine rows of each coarse row in ascending order
-      std::vector<int32_t> rptr(c.n + 1, 0), rlist(h.n);
-      for (int i = 0; i < h.n; i++) rptr[M->h_parent[q][i] + 1]++;
-      for (int P = 0; P < c.n; P++) rptr[P + 1] += rptr[P];
-      std::vector<int32_t> pos(rptr.begin(), rptr.end() - 1);
-      for (int i = 0; i < h.n; i++) rlist[pos[M->h_parent[q][i]]++] = i;
-      if ((rc = upv(ctx, &M->rptr[q + 1], rptr))) return rc;
-      if ((rc = upv(ctx, &M->rlist[q + 1], rlist))) return rc;
-    }
-    size_t n = h.n, nw = (size_t)h.w * h.n;
-    if (q == 0) { M->ac[0] = ctx->ac; M->anb[0] = ctx->anb; }
-    else {
-      FS_CK(cudaMalloc(&M->ac[q], sizeof(double) * n));
-      FS_CK(cudaMalloc(&M->anb[q], sizeof(double) * nw));
-      FS_CK(cudaMemsetAsync(M->anb[q], 0, sizeof(double) * nw, ctx->st));
-    }
-    FS_CK(cudaMalloc(&M->b[q], sizeof(double) * n));
-    FS_CK(cudaMalloc(&M->x[q], sizeof(double) * n));
-    FS_CK(cudaMalloc(&M->r[q], sizeof(double) * n));
-    FS_CK(cudaMalloc(&M->t[q], sizeof(double) * n));
-    FS_CK(cudaMalloc(&M->tf[q], sizeof(float) * n));
-    FS_CK(cudaMalloc(&M->acf[q], sizeof(float) * n));
-    FS_CK(cudaMalloc(&M->anbf[q], sizeof(float) * nw));
-    FS_CK(cudaMalloc(&M->bf[q], sizeof(float) * n));
-    FS_CK(cudaMalloc(&M->xf[q], sizeof(float) * n));
-    FS_CK(cudaMalloc(&M->rf[q], sizeof(float) * n));
-  }
-  for (int q = 0; q < M->nlev; q++) {
-    int32_t *cols = M->colors[q];
-    LevelDev<double> d{};
-    d.n = M->n[q]; d.w = M->w[q]; d.ncolors = M->ncol[q];
-    d.ncf = M->nnb[q]; d.nbr = M->nbr[q]; d.color_rows = cols; d.color_ptr = cols + M->n[q];
-    d.ac = M->ac[q]; d.anb = M->anb[q]; d.b = M->b[q]; d.x = M->x[q]; d.r = M->r[q]; d.t = M->t[q];
-    d.parent = (q + 1 < M->nlev) ? M->parent[q] : nullptr;
-    d.rptr = M->rptr[q]; d.rlist = M->rlist[q];
-    L64[q] = d;
-    LevelDev<float> e{};
-    e.n = d.n; e.w = d.w; e.ncolors = d.ncolors; e.ncf = d.ncf; e.nbr = d.nbr; e.color_rows = d.color_rows;
-    e.color_ptr = d.color_ptr; e.ac = M->acf[q]; e.anb = M->anbf[q]; e.b = M->bf[q]; e.x = M->xf[q]; e.r = M->rf[q];
-    e.t = M->tf[q];
-    e.parent = d.parent; e.rptr = d.rptr; e.rlist = d.rlist;
-    L32[q] = e;
-  }
-  FS_CK(cudaMalloc(&M->lev64, sizeof(LevelDev<double>) * M->nlev));
-  FS_CK(fs_upload(ctx, M->lev64, L64.data(), sizeof(LevelDev<double>) * M->nlev));
-  FS_CK(cudaMalloc(&M->lev32, sizeof(LevelDev<float>) * M->nlev));
-  FS_CK(fs_upload(ctx, M->lev32, L32.data(), sizeof(LevelDev<float>) * M->nlev));
-  FS_CK(cudaMalloc(&M->red, sizeof(double) * (6 + FS_SUMK + 9) * FS_RED_BLOCKS));
-  FS_CK(cudaMalloc(&M->gridbar, sizeof(unsigned) * FS_GRIDBAR_WORDS));
-  for (int q = 1; q < M->nlev; q++) {
-    M->h_nnb[q] = std::move(H[q].nnb); M->h_nbr[q] = std::move(H[q].nbr);
-    M->h_cptr[q] = std::move(cptr[q - 1]); M->h_clist[q] = std::move(clist[q - 1]);
-  }
   // preconditioner: stop at the first level small enough for the dense inverse
   M->lc = M->nlev - 1;
   for (int q = 0; q < M->nlev; q++)
     if (q > 0 && M->n[q] <= FS_MG_DIRECT) { M->lc = q; break; }
   M->direct = M->lc > 0 && M->n[M->lc] <= FS_MG_DIRECT;
-  if (M->direct) {
-    size_t nn = (size_t)M->n[M->lc] * M->n[M->lc];
-    FS_CK(cudaMalloc(&M->sinv, sizeof(double) * nn));
-    // the attribute belongs to the function, shared by every context of the
-    // process: set it for the largest coarsest level any context may have
-    const int sm = (int)(sizeof(double) * FS_MG_DIRECT * FS_MG_DIRECT);
-    const void *ks[] = {(const void *)k_mg_dense_inverse<1>, (const void *)k_mg_dense_inverse<2>,
-                        (const void *)k_mg_dense_inverse<3>, (const void *)k_mg_dense_inverse<4>,
-                        (const void *)k_mg_dense_inverse<5>};
-    for (const void *k : ks) FS_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+  return FS_OK;
+}
+
+// neighbour counts and lists of a level (host)
+static const std::vector<int32_t> &mg_nnb(const fs_ctx *ctx, int l) { return l ? ctx->mg->h_nnb[l] : ctx->h_ncf; }
+static const std::vector<int32_t> &mg_nbr(const fs_ctx *ctx, int l) { return l ? ctx->mg->h_nbr[l] : ctx->h_cn; }
+
+static int mg_mesh_tables(fs_ctx *ctx) {
+  fs_mg_dev *M = ctx->mg;
+  int rc;
+  M->ncol[0] = ctx->ncolors;
+  M->colors[0] = ctx->color_rows;   // the same greedy colouring in cell order
+  M->nnb[0] = ctx->ncf; M->nbr[0] = ctx->cn;
+  M->ac[0] = ctx->ac; M->anb[0] = ctx->anb;
+  for (int q = 0; q < M->nlev; q++) {
+    const std::vector<int32_t> &nnb = mg_nnb(ctx, q), &nbr = mg_nbr(ctx, q);
+    const size_t n = M->n[q], w = M->w[q];
+    if (q > 0) {
+      HostLevel h;
+      h.n = M->n[q]; h.w = M->w[q]; h.nnb = nnb; h.nbr = nbr;
+      if ((rc = upv(ctx, &M->colors[q], color_level(h, M->ncol[q])))) return rc;
+      if ((rc = upv(ctx, &M->nnb[q], nnb)) || (rc = upv(ctx, &M->nbr[q], nbr))) return rc;
+      if ((rc = mg_alloc(ctx, &M->ac[q], n)) || (rc = mg_alloc(ctx, &M->anb[q], n * w))) return rc;
+      FS_CK(cudaMemsetAsync(M->anb[q], 0, sizeof(double) * n * w, ctx->st));
+    }
+    if (q + 1 == M->nlev) break;
+    const std::vector<int32_t> &par = M->h_parent[q], &cnn = M->h_nnb[q + 1], &cnb = M->h_nbr[q + 1];
+    const int nc = M->n[q + 1];
+    if ((rc = upv(ctx, &M->parent[q], par))) return rc;
+    // LHS lists and slot map (fine slot -> coarse slot / internal / none)
+    if ((rc = upv(ctx, &M->cptr[q + 1], M->h_cptr[q + 1])) || (rc = upv(ctx, &M->clist[q + 1], M->h_clist[q + 1])))
+      return rc;
+    std::vector<int32_t> cmap(n * w, -1);
+    for (size_t i = 0; i < n; i++) {
+      const int P = par[i];
+      for (int j = 0; j < nnb[i]; j++) {
+        const int nb = nbr[j * n + i];
+        if (nb < 0) continue;
+        const int Q = par[nb];
+        if (Q == P) { cmap[j * n + i] = -2; continue; }
+        for (int k = 0; k < cnn[P]; k++)
+          if (cnb[(size_t)k * nc + P] == Q) { cmap[j * n + i] = k; break; }
+      }
+    }
+    if ((rc = upv(ctx, &M->cmap[q + 1], cmap))) return rc;
+    // restriction lists: fine rows of each coarse row in ascending order
+    std::vector<int32_t> rptr(nc + 1, 0), rlist(n);
+    for (size_t i = 0; i < n; i++) rptr[par[i] + 1]++;
+    for (int P = 0; P < nc; P++) rptr[P + 1] += rptr[P];
+    std::vector<int32_t> pos(rptr.begin(), rptr.end() - 1);
+    for (size_t i = 0; i < n; i++) rlist[pos[par[i]]++] = (int32_t)i;
+    if ((rc = upv(ctx, &M->rptr[q + 1], rptr)) || (rc = upv(ctx, &M->rlist[q + 1], rlist))) return rc;
   }
-  // cooperative grid: smallest co-resident count of the three kernels, <= 4 CTAs/SM
-  int a = 0, b = 0, c = 0;
-  FS_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, (void *)k_mg_solve, FS_COOP_BLOCK, 0));
-  int b2 = 0, c2 = 0, c3 = 0;
-  FS_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (void *)k_amg_bicgstab<double, 0>, FS_COOP_BLOCK, 0));
-  FS_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, (void *)k_amg_bicgstab<float, 0>, FS_COOP_BLOCK, 0));
-  FS_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, (void *)k_amg_bicgstab<double, 1>, FS_COOP_BLOCK, 0));
-  FS_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c2, (void *)k_amg_bicgstab<float, 1>, FS_COOP_BLOCK, 0));
-  FS_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c3, (void *)k_amg_bicgstab<float, 2>, FS_COOP_BLOCK, 0));
-  int per = std::min(std::min(a, std::min(b, c)), std::min(std::min(b2, c2), c3));
-  if (per < 1) { ctx->err = "multigrid kernels do not fit on an SM"; return FS_E_CUDA; }
-  M->per_sm = per;   // occupancy limit; the grid follows the launch shape at each solve
+  if (M->direct && (rc = mg_alloc(ctx, &M->sinv, (size_t)M->n[M->lc] * M->n[M->lc]))) return rc;
+  if ((rc = mg_alloc(ctx, &M->red, (6 + FS_SUMK + 9) * (size_t)FS_RED_BLOCKS))) return rc;
+  return mg_alloc(ctx, &M->gridbar, FS_GRIDBAR_WORDS);
+}
+
+static int mg_mesh_tables_once(fs_ctx *ctx) {
+  if (ctx->mg->mesh_ready) return FS_OK;
+  int rc = mg_mesh_tables(ctx);
+  if (rc) return rc;
+  ctx->mg->mesh_ready = true;
+  return FS_OK;
+}
+
+// the mesh-ordered levels for cycles in R
+template <class R>
+static int mg_mesh_build(fs_ctx *ctx) {
+  constexpr bool f32 = sizeof(R) == sizeof(float);
+  int rc = mg_mesh_tables_once(ctx);
+  if (rc) return rc;
+  fs_mg_dev *M = ctx->mg;
+  if (M->mesh_vec[f32]) return FS_OK;
+  std::vector<LevelDev<R>> L(M->nlev);
+  for (int q = 0; q < M->nlev; q++) {
+    const size_t n = M->n[q];
+    LevelDev<R> d{};
+    if constexpr (f32) {
+      if ((rc = mg_alloc(ctx, &M->acf[q], n)) || (rc = mg_alloc(ctx, &M->anbf[q], n * M->w[q])) ||
+          (rc = mg_alloc(ctx, &M->bf[q], n)) || (rc = mg_alloc(ctx, &M->xf[q], n)) || (rc = mg_alloc(ctx, &M->rf[q], n)) ||
+          (rc = mg_alloc(ctx, &M->tf[q], n)))
+        return rc;
+      d.ac = M->acf[q]; d.anb = M->anbf[q]; d.b = M->bf[q]; d.x = M->xf[q]; d.r = M->rf[q]; d.t = M->tf[q];
+    } else {
+      if ((rc = mg_alloc(ctx, &M->b[q], n)) || (rc = mg_alloc(ctx, &M->x[q], n)) || (rc = mg_alloc(ctx, &M->r[q], n)) ||
+          (rc = mg_alloc(ctx, &M->t[q], n)))
+        return rc;
+      d.ac = M->ac[q]; d.anb = M->anb[q]; d.b = M->b[q]; d.x = M->x[q]; d.r = M->r[q]; d.t = M->t[q];
+    }
+    d.n = M->n[q]; d.w = M->w[q]; d.ncolors = M->ncol[q]; d.ncf = M->nnb[q]; d.nbr = M->nbr[q];
+    d.color_rows = M->colors[q]; d.color_ptr = M->colors[q] + M->n[q];
+    d.parent = q + 1 < M->nlev ? M->parent[q] : nullptr;
+    d.rptr = M->rptr[q]; d.rlist = M->rlist[q];
+    L[q] = d;
+  }
+  LevelDev<R> *dev = nullptr;
+  if ((rc = upv(ctx, &dev, L))) return rc;
+  if constexpr (f32) M->lev32 = dev; else M->lev64 = dev;
+  M->mesh_vec[f32] = true;
   return FS_OK;
 }
 
 int fs_mg_free(fs_ctx *ctx) {
   fs_mg_dev *M = ctx->mg;
   if (!M) return FS_OK;
-  for (int q = 0; q < M->nlev; q++) {
-    void *p[] = {M->colors[q], q ? M->nnb[q] : nullptr, q ? M->nbr[q] : nullptr, M->parent[q], M->cptr[q], M->clist[q],
-                 M->cmap[q], M->rptr[q], M->rlist[q], q ? M->ac[q] : nullptr, q ? M->anb[q] : nullptr, M->b[q], M->x[q],
-                 M->r[q], M->acf[q], M->anbf[q], M->bf[q], M->xf[q], M->rf[q], M->t[q], M->tf[q]};
-    for (void *x : p) if (x) cudaFree(x);
-  }
-  for (int q = 0; q < FS_MG_MAXLEV; q++) {
-    void *p[] = {M->vcol[q], M->vrow[q], M->vkp[q], M->csum[q].ptr, M->csum[q].idx, M->cdiag[q].ptr, M->cdiag[q].idx};
-    for (void *x : p) if (x) cudaFree(x);
-  }
-  for (void *x : M->vallocs) cudaFree(x);
-  cudaFree(M->par0);
-  cudaFree(M->vc64); cudaFree(M->vc32); cudaFree(M->gridbar);
-  cudaFree(M->lev64); cudaFree(M->lev32); cudaFree(M->red); cudaFree(M->sinv);
+  for (void *x : M->allocs) cudaFree(x);
   delete M;
   ctx->mg = nullptr;
   return FS_OK;
@@ -1107,7 +1123,7 @@ static std::vector<std::vector<int32_t>> vc_numbers(const fs_mg_dev *M) {
 static int mg_vc_sums(fs_ctx *ctx, int l, const std::vector<int32_t> &idf, const std::vector<int32_t> &idc) {
   fs_mg_dev *M = ctx->mg;
   const int n = M->n[l - 1], w = M->w[l - 1], nc = M->n[l], wc = M->w[l];
-  const std::vector<int32_t> &nnb = l > 1 ? M->h_nnb[l - 1] : ctx->h_ncf, &nbr = l > 1 ? M->h_nbr[l - 1] : ctx->h_cn;
+  const std::vector<int32_t> &nnb = mg_nnb(ctx, l - 1), &nbr = mg_nbr(ctx, l - 1);
   const std::vector<int32_t> &par = M->h_parent[l - 1], &cnn = M->h_nnb[l], &cnb = M->h_nbr[l];
   const std::vector<int32_t> &cptr = M->h_cptr[l], &clist = M->h_clist[l];
   const size_t np = M->vnpos[l];
@@ -1154,6 +1170,7 @@ static int mg_vc_sums(fs_ctx *ctx, int l, const std::vector<int32_t> &idf, const
 // the row patterns of level 0, when there are few enough
 static int mg_vc_patterns(fs_ctx *ctx, const std::vector<int32_t> &id) {
   fs_mg_dev *M = ctx->mg;
+  M->npat = 0;
   const int n = ctx->N, w = ctx->W;
   if (w > 8) return FS_OK;
   const std::vector<int32_t> &cn = ctx->h_cn;
@@ -1181,7 +1198,6 @@ static int mg_vc_patterns(fs_ctx *ctx, const std::vector<int32_t> &id) {
   for (int i = 0; i < n; i++) patL[id[i]] = pat[i];
   int rc;
   if ((rc = upv(ctx, &M->pat, pat)) || (rc = upv(ctx, &M->patL, patL)) || (rc = upv(ctx, &M->offs, offs))) return rc;
-  M->vallocs.push_back(M->pat); M->vallocs.push_back(M->patL); M->vallocs.push_back(M->offs);
   M->npat = np;
   return FS_OK;
 }
@@ -1192,138 +1208,155 @@ static int mg_vc_patterns(fs_ctx *ctx, const std::vector<int32_t> &id) {
 // an aggregate rows stay in ascending original order, which keeps every sum's
 // order), their sliced layout, and for the
 // precision asked for the arrays and the descriptor.
+
+// first row of each of level l+1's aggregates among level l's rows
+static std::vector<int32_t> vc_first(const fs_mg_dev *M, int l, const std::vector<std::vector<int32_t>> &ids) {
+  std::vector<int32_t> kp(M->n[l + 1] + 1, 0);
+  for (int i = 0; i < M->n[l]; i++) kp[ids[l + 1][M->h_parent[l][i]] + 1]++;
+  for (int P = 0; P < M->n[l + 1]; P++) kp[P + 1] += kp[P];
+  return kp;
+}
+
+// column indices of level l in the layout (unused slots: level 0 -1, else the row itself)
+static std::vector<int32_t> vc_columns(const fs_ctx *ctx, int l, const std::vector<int32_t> &id) {
+  const int n = ctx->mg->n[l], w = ctx->mg->w[l];
+  const std::vector<int32_t> &nnb = mg_nnb(ctx, l), &nbr = mg_nbr(ctx, l);
+  std::vector<int32_t> col(ctx->mg->vnpos[l]);
+  if (l > 0)
+    for (size_t q = 0; q < col.size(); q++) col[q] = std::min<int>((int)(q / (32 * (size_t)w) * 32 + q % 32), n - 1);
+  for (int j = 0; j < w; j++)
+    for (int i = 0; i < n; i++) {
+      const int k = j < nnb[i] ? nbr[(size_t)j * n + i] : -1;
+      if (l == 0) col[vc_pos(l, n, w, id[i], j)] = k;
+      else if (k >= 0) col[vc_pos(l, n, w, id[i], j)] = id[k];
+    }
+  return col;
+}
+
+static int mg_vc_map(fs_ctx *ctx, const std::vector<std::vector<int32_t>> &ids) {
+  fs_mg_dev *M = ctx->mg;
+  const int n = M->n[0];
+  int rc;
+  for (int l = 0; l <= M->lc; l++)
+    M->vnpos[l] = (int)((size_t)(l == 0 ? n : (M->n[l] + 31) / 32 * 32) * M->w[l]);
+  std::vector<int32_t> p0(n), cells(n);
+  for (int i = 0; i < n; i++) { p0[i] = ids[1][M->h_parent[0][i]]; cells[ids[0][i]] = i; }
+  if ((rc = upv(ctx, &M->par0, p0)) || (rc = upv(ctx, &M->cells, cells)) ||
+      (rc = upv(ctx, &M->vkp[0], vc_first(M, 0, ids))) || (rc = mg_vc_patterns(ctx, ids[0])))
+    return rc;
+  // level 0's columns: without patterns, or for the slots that they do not cover
+  M->vcol[0] = nullptr;
+  if ((M->npat == 0 || M->w[0] > FS_VC_SLOTS) && (rc = upv(ctx, &M->vcol[0], vc_columns(ctx, 0, ids[0])))) return rc;
+  for (int l = 1; l <= M->lc; l++)
+    if ((rc = mg_vc_sums(ctx, l, ids[l - 1], ids[l]))) return rc;
+  return FS_OK;
+}
+
+// What the cycle touches of the levels >= 1 goes into one block, the coarsest
+// level first, with the barrier count and the partial sums: the small levels
+// share a few pages instead of one allocation (and page) per array.  Device
+// memory with everything else of the hierarchy, 3.4 M cells: 189 bytes a cell in
+// FP64 and 195 in FP32 (24 more where level 0 has no row patterns); the
+// mesh-ordered levels of the general V-cycle take 140 and 168.
+template <class R>
+static int mg_vc_arrays(fs_ctx *ctx, const std::vector<std::vector<int32_t>> &ids) {
+  constexpr bool f32 = sizeof(R) == sizeof(float);
+  fs_mg_dev *M = ctx->mg;
+  const int lc = M->lc;
+  const size_t N = M->n[0], W = M->w[0];
+  int rc;
+  char *base = nullptr;
+  size_t off = 0;
+  auto take = [&](auto **d, size_t n) {
+    *d = base ? reinterpret_cast<std::remove_reference_t<decltype(*d)>>(base + off) : nullptr;
+    off += (std::max<size_t>(n, 1) * sizeof(**d) + 255) / 256 * 256;
+  };
+  VcDev<R> v{};
+  R *val[FS_MG_MAXLEV] = {}, *ac[FS_MG_MAXLEV] = {};
+  int32_t *kp[FS_MG_MAXLEV] = {}, *col[FS_MG_MAXLEV] = {};
+  for (int pass = 0; pass < 2; pass++) {
+    if (pass == 1 && (rc = mg_alloc(ctx, &base, off))) return rc;
+    off = 0;
+    take(&M->vbar[f32], FS_GRIDBAR_WORDS);
+    take(&M->vpart[f32], (9 + FS_SUMK) * (size_t)FS_RED_BLOCKS);
+    take(&M->vinv[f32], (size_t)M->n[lc] * M->n[lc]);
+    for (int l = lc; l >= 1; l--) {
+      VcLevel<R> &d = v.L[l];
+      take(&ac[l], M->n[l]);
+      take(&d.b, M->n[l]);
+      take(&d.x, M->n[l]);
+      take(&d.r, M->n[l]);
+      if (l < lc) take(&kp[l], M->n[l + 1] + 1);
+      take(&col[l], M->vnpos[l]);
+      take(&val[l], M->vnpos[l]);
+    }
+    take(&v.x1, M->n[1]);   // the result of level 1
+  }
+  for (int l = 1; l <= lc; l++) {
+    if (l < lc) {
+      const std::vector<int32_t> h = vc_first(M, l, ids);
+      FS_CK(fs_upload(ctx, kp[l], h.data(), sizeof(int32_t) * h.size()));
+    }
+    const std::vector<int32_t> h = vc_columns(ctx, l, ids[l]);
+    FS_CK(fs_upload(ctx, col[l], h.data(), sizeof(int32_t) * h.size()));
+  }
+  // Level 0: the matrix in the layout, x and r.  The FP32 cycle reads FP32 copies (in mesh
+  // order too, for the up leg); the FP64 matrix in the layout is then only the source of
+  // level 1's and sits in the gradient routine's scratch during the set-up.
+  R *x0 = nullptr, *r0 = nullptr;
+  if ((rc = mg_alloc(ctx, &x0, N)) || (rc = mg_alloc(ctx, &r0, N))) return rc;
+  if constexpr (f32) {
+    if ((rc = mg_alloc(ctx, &val[0], W * N)) || (rc = mg_alloc(ctx, &ac[0], N)) || (rc = mg_alloc(ctx, &M->anbm, W * N)) ||
+        (rc = mg_alloc(ctx, &M->acm, N)))
+      return rc;
+  }
+  if (f32 && W + 1 <= FS_GTMP_BLOCKS) { M->val0[f32] = ctx->gtmp; M->ac0[f32] = ctx->gtmp + W * N; }
+  else if ((rc = mg_alloc(ctx, &M->val0[f32], W * N)) || (rc = mg_alloc(ctx, &M->ac0[f32], N))) return rc;
+  // FP64 matrices of the other levels, shared by both precisions
+  for (int l = 1; l <= lc; l++) {
+    if constexpr (f32) {
+      M->vvalf[l] = val[l]; M->vacf[l] = ac[l];
+      if (!M->vc_ready[0] && ((rc = mg_alloc(ctx, &M->vval[l], M->vnpos[l])) || (rc = mg_alloc(ctx, &M->vac[l], M->n[l])))) return rc;
+    } else { M->vval[l] = val[l]; M->vac[l] = ac[l]; }
+  }
+  if constexpr (f32) { M->vvalf[0] = val[0]; M->vacf[0] = ac[0]; }
+  else { val[0] = M->val0[0]; ac[0] = M->ac0[0]; }
+  kp[0] = M->vkp[0]; col[0] = M->vcol[0];
+  v.lc = lc;
+  for (int l = 0; l <= lc; l++) {
+    VcLevel<R> &d = v.L[l];
+    d.n = M->n[l]; d.w = M->w[l];
+    d.col = col[l]; d.val = val[l]; d.ac = ac[l]; d.kp = kp[l];
+  }
+  v.L[0].cells = M->cells;
+  v.L[0].r = r0;
+  v.sinv = M->vinv[f32];
+  LevelDev<R> &q = v.L0;
+  q.n = M->n[0]; q.w = M->w[0]; q.ncolors = ctx->ncolors; q.ncf = ctx->ncf; q.nbr = ctx->cn;
+  q.color_rows = ctx->color_rows; q.color_ptr = ctx->color_rows + N;
+  if constexpr (f32) { q.ac = M->acm; q.anb = M->anbm; } else { q.ac = ctx->ac; q.anb = ctx->anb; }
+  q.x = x0; q.r = r0;
+  v.par0 = M->par0;
+  v.npat = M->npat; v.pat = M->pat; v.patL = M->patL; v.offs = M->offs;
+  VcDev<R> *dev = nullptr;
+  if ((rc = mg_alloc(ctx, &dev, 1))) return rc;
+  FS_CK(fs_upload(ctx, dev, &v, sizeof(v)));
+  for (int l = 1; l <= lc; l++) { M->vkp[l] = kp[l]; M->vcol[l] = col[l]; }
+  if constexpr (f32) M->vc32 = dev; else M->vc64 = dev;
+  M->vc_ready[f32] = true;
+  return FS_OK;
+}
+
 static int mg_vc_build(fs_ctx *ctx, bool f32) {
   fs_mg_dev *M = ctx->mg;
   if (M->vc_ready[f32]) return FS_OK;
-  const int lc = M->lc;
+  const std::vector<std::vector<int32_t>> ids = vc_numbers(M);
   int rc;
   if (!M->vc_map) {
-    const std::vector<std::vector<int32_t>> ids = vc_numbers(M);
-    for (int l = lc; l >= 0; l--) {
-      const std::vector<int32_t> &id = ids[l];
-      const int n = M->n[l];
-      const std::vector<int32_t> &nnb = l ? M->h_nnb[l] : ctx->h_ncf, &nbr = l ? M->h_nbr[l] : ctx->h_cn;
-      std::vector<int32_t> row(n);           // original row of each new one
-      if (l < lc) {
-        const std::vector<int32_t> &par = M->h_parent[l], &up = ids[l + 1];
-        const int nc = M->n[l + 1];
-        std::vector<int32_t> kp(nc + 1, 0);
-        for (int i = 0; i < n; i++) kp[up[par[i]] + 1]++;
-        for (int P = 0; P < nc; P++) kp[P + 1] += kp[P];
-        if ((rc = upv(ctx, &M->vkp[l], kp))) return rc;
-        if (l == 0) {
-          std::vector<int32_t> p0(n);
-          for (int i = 0; i < n; i++) p0[i] = up[par[i]];
-          if ((rc = upv(ctx, &M->par0, p0))) return rc;
-        }
-      }
-      for (int i = 0; i < n; i++) row[id[i]] = i;
-      std::vector<int32_t> col;
-      const int w = M->w[l];
-      if (l == 0) {
-        col.resize((size_t)w * n);
-        for (int j = 0; j < w; j++)
-          for (int a = 0; a < n; a++) col[(size_t)j * n + a] = nbr[(size_t)j * n + row[a]];
-      } else {
-        col.assign((size_t)(n + 31) / 32 * 32 * w, 0);
-        for (int a = 0; a < n; a++)
-          for (int j = 0; j < w; j++) {
-            const size_t src = (size_t)j * n + row[a];
-            col[((size_t)(a / 32) * w + j) * 32 + a % 32] = j < nnb[row[a]] && nbr[src] >= 0 ? id[nbr[src]] : a;
-          }
-      }
-      M->vnpos[l] = (int)col.size();
-      if ((rc = upv(ctx, &M->vcol[l], col)) || (rc = upv(ctx, &M->vrow[l], row))) return rc;
-    }
-    for (int l = 1; l <= lc; l++)
-      if ((rc = mg_vc_sums(ctx, l, ids[l - 1], ids[l]))) return rc;
-    if ((rc = mg_vc_patterns(ctx, ids[0]))) return rc;
-    for (int q = 0; q < M->nlev; q++) {
-      M->h_nnb[q] = std::vector<int32_t>(); M->h_nbr[q] = std::vector<int32_t>();
-      M->h_cptr[q] = std::vector<int32_t>(); M->h_clist[q] = std::vector<int32_t>();
-    }
+    if ((rc = mg_vc_map(ctx, ids))) return rc;
     M->vc_map = true;
   }
-  // What the cycle touches of the levels >= 1 goes into one block, the coarsest
-  // level first, with the barrier count and the partial sums: the small levels
-  // share a few pages instead of one allocation (and page) per array.
-  const size_t es = f32 ? sizeof(float) : sizeof(double);
-  const size_t nparts = (9 + FS_SUMK) * (size_t)FS_RED_BLOCKS;
-  char *base = nullptr;
-  size_t off = 0;
-  auto take = [&](size_t bytes) -> void * {
-    void *q = base ? base + off : nullptr;
-    off += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
-    return q;
-  };
-  int32_t *kp[FS_MG_MAXLEV] = {}, *col[FS_MG_MAXLEV] = {};
-  void *val[FS_MG_MAXLEV] = {}, *ac[FS_MG_MAXLEV] = {}, *r[FS_MG_MAXLEV] = {};
-  const double *sinv = nullptr;
-  for (int pass = 0; pass < 2; pass++) {
-    if (pass == 1) { FS_CK(cudaMalloc((void **)&base, off)); M->vallocs.push_back(base); }
-    off = 0;
-    M->vbar[f32] = (unsigned *)take(sizeof(unsigned) * FS_GRIDBAR_WORDS);
-    M->vpart[f32] = (double *)take(sizeof(double) * nparts);
-    double *si = (double *)take(sizeof(double) * M->n[lc] * M->n[lc]);
-    sinv = si;
-    M->vinv[f32] = si;
-    for (int l = lc; l >= 1; l--) {
-      ac[l] = take(es * M->n[l]);
-      M->vb[f32][l] = take(es * M->n[l]);
-      M->vx[f32][l] = take(es * M->n[l]);
-      r[l] = take(es * M->n[l]);
-      if (l < lc) kp[l] = (int32_t *)take(sizeof(int32_t) * (M->n[l + 1] + 1));
-      col[l] = (int32_t *)take(sizeof(int32_t) * M->vnpos[l]);
-      val[l] = take(es * M->vnpos[l]);
-    }
-    M->vx[f32][0] = take(es * M->n[1]);   // the result of level 1
-  }
-  for (int l = 1; l <= lc; l++) {
-    if (l < lc)
-      FS_CK(cudaMemcpyAsync(kp[l], M->vkp[l], sizeof(int32_t) * (M->n[l + 1] + 1), cudaMemcpyDeviceToDevice, ctx->st));
-    FS_CK(cudaMemcpyAsync(col[l], M->vcol[l], sizeof(int32_t) * M->vnpos[l], cudaMemcpyDeviceToDevice, ctx->st));
-  }
-  auto own = [&](auto **d, size_t n) -> int {
-    FS_CK(cudaMalloc((void **)d, sizeof(**d) * std::max<size_t>(n, 1)));
-    M->vallocs.push_back(*d);
-    return FS_OK;
-  };
-  kp[0] = M->vkp[0]; col[0] = M->vcol[0];
-  for (int l = 0; l <= lc; l++) {   // the FP64 matrices are the source of the next level's in either precision
-    if (!f32 && l > 0 && !M->vval[l]) { M->vval[l] = (double *)val[l]; M->vac[l] = (double *)ac[l]; }
-    if (!M->vval[l] && ((rc = own(&M->vval[l], M->vnpos[l])) || (rc = own(&M->vac[l], M->n[l])))) return rc;
-    if (f32 && l > 0) { M->vvalf[l] = (float *)val[l]; M->vacf[l] = (float *)ac[l]; }
-    if (f32 && l == 0 && ((rc = own(&M->vvalf[l], M->vnpos[l])) || (rc = own(&M->vacf[l], M->n[l])))) return rc;
-  }
-  r[0] = f32 ? (void *)M->rf[0] : (void *)M->r[0];
-  auto desc = [&](auto *tag, auto **dev, const LevelDev<std::remove_pointer_t<decltype(tag)>> *levs) -> int {
-    using R = std::remove_pointer_t<decltype(tag)>;
-    VcDev<R> v{};
-    v.lc = lc;
-    for (int l = 0; l <= lc; l++) {
-      VcLevel<R> &d = v.L[l];
-      d.n = M->n[l]; d.w = M->w[l];
-      d.col = col[l]; d.cells = M->vrow[l];
-      d.val = f32 ? (const R *)(void *)M->vvalf[l] : (const R *)(void *)M->vval[l];
-      d.ac = f32 ? (const R *)(void *)M->vacf[l] : (const R *)(void *)M->vac[l];
-      d.kp = kp[l];
-      d.b = (R *)M->vb[f32][l]; d.x = l > 0 ? (R *)M->vx[f32][l] : nullptr;
-      d.r = (R *)r[l];
-    }
-    v.x1 = (R *)M->vx[f32][0];
-    v.sinv = sinv;
-    FS_CK(cudaMemcpy(&v.L0, levs, sizeof(LevelDev<R>), cudaMemcpyDeviceToHost));
-    v.par0 = M->par0;
-    v.npat = M->npat; v.pat = M->pat; v.patL = M->patL; v.offs = M->offs;
-    FS_CK(cudaMalloc(dev, sizeof(VcDev<R>)));
-    FS_CK(fs_upload(ctx, *dev, &v, sizeof(VcDev<R>)));
-    return FS_OK;
-  };
-  if (f32) rc = desc((float *)nullptr, &M->vc32, M->lev32);
-  else rc = desc((double *)nullptr, &M->vc64, M->lev64);
-  if (rc) return rc;
-  M->vc_ready[f32] = true;
-  return FS_OK;
+  return f32 ? mg_vc_arrays<float>(ctx, ids) : mg_vc_arrays<double>(ctx, ids);
 }
 
 // the current matrices in the V-cycle's layout (level0: level 0 alone, the
@@ -1331,13 +1364,13 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
 static int mg_vc_values(fs_ctx *ctx, bool f32, bool level0) {
   fs_mg_dev *M = ctx->mg;
   k_mg_level0<<<fs_grid(M->n[0]), FS_BLOCK, 0, ctx->st>>>(
-      M->n[0], M->w[0], M->vrow[0], M->ac[0], M->anb[0], M->vac[0], M->vval[0], f32 ? M->vacf[0] : nullptr,
-      f32 ? M->vvalf[0] : nullptr, f32 ? M->acf[0] : nullptr, f32 ? M->anbf[0] : nullptr);
+      M->n[0], M->w[0], M->cells, ctx->ac, ctx->anb, M->ac0[f32], M->val0[f32], f32 ? M->vacf[0] : nullptr,
+      f32 ? M->vvalf[0] : nullptr, f32 ? M->acm : nullptr, f32 ? M->anbm : nullptr);
   FS_LAUNCH_CHECK();
   for (int l = 1; l <= M->lc && !level0; l++) {
     k_mg_coarse<<<fs_grid((long)M->vnpos[l] + M->n[l]), FS_BLOCK, 0, ctx->st>>>(
-        M->vnpos[l], M->n[l], M->csum[l].ptr, M->csum[l].idx, M->cdiag[l].ptr, M->cdiag[l].idx, M->vac[l - 1],
-        M->vval[l - 1], M->vac[l], M->vval[l], f32 ? M->vacf[l] : nullptr, f32 ? M->vvalf[l] : nullptr);
+        M->vnpos[l], M->n[l], M->csum[l].ptr, M->csum[l].idx, M->cdiag[l].ptr, M->cdiag[l].idx,
+        l > 1 ? M->vac[l - 1] : M->ac0[f32], l > 1 ? M->vval[l - 1] : M->val0[f32], M->vac[l], M->vval[l], f32 ? M->vacf[l] : nullptr, f32 ? M->vvalf[l] : nullptr);
     FS_LAUNCH_CHECK();
   }
   return FS_OK;
@@ -1366,6 +1399,7 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   }
   const int G = std::min(ctx->num_sms * fs_coop_per_sm(ctx, M->per_sm), FS_RED_BLOCKS);
   if (solver == FS_SOLVER_AMG) {
+    if ((rc = mg_mesh_build<double>(ctx))) return rc;
     if ((rc = mg_coarse_matrices(ctx, M->nlev - 1, false))) return rc;
     M->built_nf = 0;
     MgSolveArgs a{};
@@ -1390,7 +1424,7 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   // the one-phase V-cycle needs one pre- and one post-sweep and a dense coarsest level
   const bool fused = std::max(1, ctx->cfg.mg_pre) == 1 && M->direct && M->lc > 0;
   const bool vc = gs || fused;
-  if (vc && (rc = mg_vc_build(ctx, f32))) return rc;
+  if ((rc = vc ? mg_vc_build(ctx, f32) : f32 ? mg_mesh_build<float>(ctx) : mg_mesh_build<double>(ctx))) return rc;
   const int refresh = std::max(1, ctx->cfg.pc_refresh);
   const bool reuse = M->built_nf == nf && M->built_f32 == f32 && M->built_vc == vc && M->age + 1 < refresh;
   if (reuse) M->age++;
@@ -1446,11 +1480,11 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
     if (!f32) {
       M->pend64 = AmgKArgs<double>{};
       fill(M->pend64);
-      M->pend64.lev = M->lev64; M->pend64.vc = M->vc64;
+      M->pend64.lev = vc ? &M->vc64->L0 : M->lev64; M->pend64.vc = M->vc64;
     } else {
       M->pend32 = AmgKArgs<float>{};
       fill(M->pend32);
-      M->pend32.lev = M->lev32; M->pend32.vc = M->vc32;
+      M->pend32.lev = vc ? &M->vc32->L0 : M->lev32; M->pend32.vc = M->vc32;
     }
     return FS_OK;
   }
@@ -1458,7 +1492,7 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   if (!f32) {
     AmgKArgs<double> a{};
     fill(a);
-    a.lev = M->lev64; a.vc = M->vc64;
+    a.lev = vc ? &M->vc64->L0 : M->lev64; a.vc = M->vc64;
     void *args[] = {&a};
     if (a.nx > 0) FS_CK(fs_coop_launch(guess_fit_kernel<double>(a.nx), G, fs_coop_block(ctx), args, ctx->st));
     FS_TIMING(FS_CK(cudaEventRecord(ctx->kev[nf - 1][0], ctx->st)));
@@ -1467,7 +1501,7 @@ int fs_mg_solve(fs_ctx *ctx, int nf, double rrf, int solver) {
   } else {
     AmgKArgs<float> a{};
     fill(a);
-    a.lev = M->lev32; a.vc = M->vc32;
+    a.lev = vc ? &M->vc32->L0 : M->lev32; a.vc = M->vc32;
     void *args[] = {&a};
     if (a.nx > 0) FS_CK(fs_coop_launch(guess_fit_kernel<float>(a.nx), G, fs_coop_block(ctx), args, ctx->st));
     FS_TIMING(FS_CK(cudaEventRecord(ctx->kev[nf - 1][0], ctx->st)));
@@ -1519,7 +1553,7 @@ extern "C" int fs_mg_coarse_matrix(fs_ctx *ctx, int level, double *ac, int32_t *
   fs_mg_dev *M = ctx->mg;
   if (level < 1 || level >= M->nlev || n != (size_t)M->n[level] || w != (size_t)M->w[level]) return FS_E_ARG;
   cudaSetDevice(ctx->dev);
-  if ((rc = mg_coarse_matrices(ctx, level, false))) return rc;
+  if ((rc = mg_mesh_tables_once(ctx)) || (rc = mg_coarse_matrices(ctx, level, false))) return rc;
   FS_CK(cudaMemcpyAsync(ac, M->ac[level], sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->st));
   FS_CK(cudaMemcpyAsync(anb, M->anb[level], sizeof(double) * n * w, cudaMemcpyDeviceToHost, ctx->st));
   FS_CK(cudaMemcpyAsync(n_nbr, M->nnb[level], sizeof(int32_t) * n, cudaMemcpyDeviceToHost, ctx->st));
