@@ -158,13 +158,6 @@ static void free_all(fs_ctx *c) {
                   c->ac3, c->bc3, c->ac3P, c->bc3P, c->x3P, c->gm, c->d_bset, c->flow, c->bdir,
                   c->bpcoefc, c->bgd, c->bp0, c->d_patch, c->hist};
   for (void *p : ptrs) if (p) cudaFree(p);
-  if (c->h_status) cudaFreeHost(c->h_status);
-}
-
-int fs_status_fetch(fs_ctx *ctx) {
-  if (ctx->wait_open)
-    FS_CK(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->st));
-  return FS_OK;
 }
 
 static int wait_timed_out(fs_ctx *ctx) {
@@ -173,10 +166,17 @@ static int wait_timed_out(fs_ctx *ctx) {
   return FS_E_TIMEOUT;
 }
 
-int fs_status_check(fs_ctx *ctx) {
-  if (!ctx->wait_open) return FS_OK;
+int fs_finish(fs_ctx *ctx) {
+  int32_t status = 0;
+  if (ctx->wait_open)
+    FS_CK(cudaMemcpyAsync(&status, ctx->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->st));
+  FS_CK(cudaStreamSynchronize(ctx->st));
+  return fs_finish_status(ctx, status);
+}
+
+int fs_finish_status(fs_ctx *ctx, int32_t status) {
   ctx->wait_open = false;
-  return *ctx->h_status ? wait_timed_out(ctx) : FS_OK;
+  return status ? wait_timed_out(ctx) : FS_OK;
 }
 
 extern "C" {
@@ -241,7 +241,6 @@ int fs_create(const fs_mesh_in *mesh, const fs_case *cfg, int device, fs_ctx **o
   if (cudaMalloc(&ctx->d_iters, sizeof(int32_t) * FS_NITERS) != cudaSuccess) return fail(FS_E_NOMEM);
   cudaMemsetAsync(ctx->d_iters, 0, sizeof(int32_t) * FS_NITERS, ctx->st);
   if (cudaMalloc(&ctx->d_status, sizeof(int32_t) * 8) != cudaSuccess) return fail(FS_E_NOMEM);
-  if (cudaHostAlloc((void **)&ctx->h_status, sizeof(int32_t), cudaHostAllocDefault) != cudaSuccess) return fail(FS_E_NOMEM);
   cudaMemsetAsync(ctx->d_status, 0, sizeof(int32_t) * 8, ctx->st);
   if ((rc = alloc0(ctx, &ctx->flow, 1 + 2 * FS_MAX_PATCHES))) return fail(rc);
   if (cudaMalloc(&ctx->d_bset, sizeof(int32_t) * (B ? B : 1)) != cudaSuccess) return fail(FS_E_NOMEM);
@@ -466,10 +465,8 @@ static int read_residuals(fs_ctx *ctx, fs_residuals *res) {
   int32_t it[FS_NITERS];
   FS_CK(cudaMemcpyAsync(rb, ctx->resblk, sizeof(rb), cudaMemcpyDeviceToHost, ctx->st));
   FS_CK(cudaMemcpyAsync(it, ctx->d_iters, sizeof(it), cudaMemcpyDeviceToHost, ctx->st));
-  int rc;
-  if ((rc = fs_status_fetch(ctx))) return rc;
-  FS_CK(cudaStreamSynchronize(ctx->st));
-  if ((rc = fs_status_check(ctx))) return rc;
+  int rc = fs_finish(ctx);
+  if (rc) return rc;
   fs_solver_stats_collect(ctx);
   fs_residuals r{};
   for (int q = 0; q < 5; q++) {
@@ -694,10 +691,9 @@ int fs_solve_system_host(fs_ctx *ctx, const double *ac, const double *anb, const
   int32_t it = 0;
   FS_CK(cudaMemcpyAsync(dphi, fz, sizeof(double) * N, cudaMemcpyDeviceToHost, ctx->st));
   FS_CK(cudaMemcpyAsync(&it, ctx->d_iters + 3, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->st));
-  if ((rc = fs_status_fetch(ctx))) return rc;
-  FS_CK(cudaStreamSynchronize(ctx->st));
+  rc = fs_finish(ctx);
   if (iters) *iters = it;
-  return fs_status_check(ctx);
+  return rc;
 }
 
 int fs_residuals_get(fs_ctx *ctx, fs_residuals *res) {
@@ -711,10 +707,7 @@ int fs_get_field(fs_ctx *ctx, int field, double *host, size_t n) {
   double *d = field_ptr(ctx, field, &m);
   if (!d || n != m) { ctx->err = "field id or size mismatch"; return FS_E_ARG; }
   FS_CK(cudaMemcpyAsync(host, d, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->st));
-  int rc = fs_status_fetch(ctx);
-  if (rc) return rc;
-  FS_CK(cudaStreamSynchronize(ctx->st));
-  return fs_status_check(ctx);
+  return fs_finish(ctx);
 }
 
 int fs_set_field(fs_ctx *ctx, int field, const double *host, size_t n) {
@@ -783,10 +776,7 @@ int fs_solver_kernel_ms(fs_ctx *ctx, float *ms5) {
 
 int fs_sync(fs_ctx *ctx) {
   if (!ctx) return FS_E_ARG;
-  int rc = fs_status_fetch(ctx);
-  if (rc) return rc;
-  FS_CK(cudaStreamSynchronize(ctx->st));
-  return fs_status_check(ctx);
+  return fs_finish(ctx);
 }
 
 // Ensemble of independent cases (no reference counterpart): `iters` SIMPLE

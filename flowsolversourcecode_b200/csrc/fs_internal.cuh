@@ -139,7 +139,6 @@ struct fs_ctx {
   double *resblk = nullptr;     // device residual block, layout of fs_residuals' first 20 doubles + extras
   int32_t *d_iters = nullptr;   // linear iterations per NF (FS_NITERS slots, NF 1..9 used)
   int32_t *d_status = nullptr;  // device-side status flags
-  int32_t *h_status = nullptr;  // pinned: the bounded waits' word, as fs_status_fetch copied it
   bool wait_open = false;       // a kernel with bounded waits was launched since that word was last looked at
 
   // boundary patch per boundary face (device), outlet mass-flow scratch:
@@ -270,11 +269,11 @@ int fs_continuity_correct(fs_ctx *ctx);
 int fs_residual_reduce(fs_ctx *ctx, int nf);   // CalculateResiduals partials -> resblk slot
 // The status word of the bounded device waits: a wait that gave up leaves
 // results that are not valid, so every call that hands results to the host
-// looks at it.  fetch enqueues the copy before the call's stream synchronisation;
-// check, behind it, clears a word that is set and returns FS_E_TIMEOUT.  Neither
-// does anything when no kernel with such waits ran since the last look.
-int fs_status_fetch(fs_ctx *ctx);
-int fs_status_check(fs_ctx *ctx);
+// ends with fs_finish: it waits for the context's stream and, when a kernel with
+// such waits ran since the last look, reads the word, clears it and returns
+// FS_E_TIMEOUT if it was set.
+int fs_finish(fs_ctx *ctx);
+int fs_finish_status(fs_ctx *ctx, int32_t status);   // the same for a caller that has read the word itself
 int fs_linear_solve(fs_ctx *ctx, int nf, double *fi, double rrf, int itmax, int solver);
 // k-epsilon and outlets (fs_turb.cu)
 // Transient term of one equation (AssembleTheTransientTerm.for:52-330), by value in kernel arguments:

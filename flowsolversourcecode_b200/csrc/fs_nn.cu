@@ -1102,9 +1102,7 @@ extern "C" int fs_nn_train(fs_ctx *ctx, int epochs, float lr, uint64_t seed, flo
       if ((rc = nn_pack(ctx))) return rc;
       double l = 0.;
       FS_CK(cudaMemcpyAsync(&l, nn->sc + 7, sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
-      if ((rc = fs_status_fetch(ctx))) return rc;
-      FS_CK(cudaStreamSynchronize(ctx->st));
-      if ((rc = fs_status_check(ctx))) return rc;
+      if ((rc = fs_finish(ctx))) return rc;
       lsum += l / (nn->snap_tt[s] > 0. ? nn->snap_tt[s] : 1.);
     }
     float lm = (float)(lsum / nn->count);
@@ -1144,16 +1142,18 @@ extern "C" int fs_nn_eval_host(fs_ctx *ctx, const float *X, const float *wgt, co
     for (double v : t) tt += v * v;
     FS_CK(cudaMemcpyAsync(nn->tbuf, target, sizeof(float) * N, cudaMemcpyHostToDevice, ctx->st));
     if ((rc = nn_backward(ctx, nn->X, nn->wgt, nn->tbuf, tt > 0. ? tt : 1.))) return rc;
+    // the loss and, next to it, the status word of the bounded waits in one copy
+    FS_CK(cudaMemcpyAsync(nn->sc + 8, ctx->d_status, sizeof(int32_t), cudaMemcpyDeviceToDevice, ctx->st));
     FS_CK(cudaStreamSynchronize(ctx->st));
-    double l = 0.;
-    FS_CK(cudaMemcpy(&l, nn->sc + 7, sizeof(double), cudaMemcpyDeviceToHost));
-    if (loss) *loss = (float)(l / (tt > 0. ? tt : 1.));
+    struct { double l; int32_t status, pad; } res;
+    FS_CK(cudaMemcpy(&res, nn->sc + 7, sizeof(res), cudaMemcpyDeviceToHost));
+    if ((rc = fs_finish_status(ctx, res.status))) return rc;
+    if (loss) *loss = (float)(res.l / (tt > 0. ? tt : 1.));
     if (grad) FS_CK(cudaMemcpy(grad, nn->grad, sizeof(float) * NN_NP, cudaMemcpyDeviceToHost));
   }
-  if ((rc = fs_status_fetch(ctx))) return rc;
-  FS_CK(cudaStreamSynchronize(ctx->st));
+  if ((rc = fs_finish(ctx))) return rc;
   if (y) FS_CK(cudaMemcpy(y, nn->y, sizeof(float) * N, cudaMemcpyDeviceToHost));
-  return fs_status_check(ctx);
+  return FS_OK;
 }
 
 extern "C" int fs_nn_policy(fs_ctx *ctx, double *avg_guessed, double *avg_zero, int32_t *parked) {

@@ -317,10 +317,8 @@ int fs_adaptive_time_step(fs_ctx *ctx, double courant, double min_factor, double
   FS_LAUNCH_CHECK();
   double mx = 0.;
   FS_CK(cudaMemcpyAsync(&mx, a.out, sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
-  int rc = fs_status_fetch(ctx);
+  int rc = fs_finish(ctx);
   if (rc) return rc;
-  FS_CK(cudaStreamSynchronize(ctx->st));
-  if ((rc = fs_status_check(ctx))) return rc;
   // dtlocal = GlobalCourantNumber / max, then the change-factor clamp (:192-193)
   double dtl = courant / mx;
   dtl = fmax(dtl, min_factor * ctx->dt);
