@@ -171,6 +171,7 @@ PROTOTYPES = {
     "fs_get_connectivity": (C.c_int, [_V, _I, _I, _I, _I, _I]),
     "fs_mg_levels": (C.c_int, [_V, _I, _I, C.c_int]),
     "fs_mg_vcycle_matrix": (C.c_int, [_V, C.c_int, C.c_int, _D, _D, C.c_size_t, C.c_size_t]),
+    "fs_test_alloc_failure": (C.c_int, [_V, C.c_int]),
     "fs_mg_parents": (C.c_int, [_V, C.c_int, _I, C.c_size_t]),
     "fs_mg_info": (C.c_int, [_V, _I, C.c_int, _I, _I]),
     "fs_mg_coarse_matrix": (C.c_int, [_V, C.c_int, _D, _I, _I, _D, C.c_size_t, C.c_size_t]),

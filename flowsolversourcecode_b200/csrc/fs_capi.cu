@@ -191,7 +191,7 @@ int fs_create(const fs_mesh_in *mesh, const fs_case *cfg, int device, fs_ctx **o
   ctx->cfg = *cfg;
   ctx->dev = device;
   int rc = FS_OK;
-  auto fail = [&](int r) { fs_transient_free(ctx); fs_energy_free(ctx); fs_turb_free(ctx); free_all(ctx); if (ctx->st) cudaStreamDestroy(ctx->st); delete ctx; return r; };
+  auto fail = [&](int r) { (void)cudaGetLastError(); fs_transient_free(ctx); fs_energy_free(ctx); fs_turb_free(ctx); free_all(ctx); if (ctx->st) cudaStreamDestroy(ctx->st); delete ctx; return r; };
   if (cudaSetDevice(device) != cudaSuccess) return fail(FS_E_CUDA);
   if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess) return fail(FS_E_CUDA);
   cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);

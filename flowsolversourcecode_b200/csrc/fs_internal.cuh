@@ -187,6 +187,7 @@ struct fs_ctx {
   double ens_split = 1.;        // batched ensembles: CTA groups in proportion to cells^ens_split (x p' iterations)
   bool mom_pending = false;
   alignas(8) unsigned char mom_pend[160];   // the prepared launch's arguments (Sor3Args)
+  int test_alloc_left = 0;      // fs_test_alloc_failure: the allocation (fs_alloc) that is refused, counted down
   int test_wait_extra = 0;      // fs_test_wait_timeout: extra arrivals the AMG solver's barriers wait for (< 0: in graphs)
 };
 
@@ -203,10 +204,12 @@ struct fs_ctx {
 enum { RB_ABS = 0, RB_MAX = 9, RB_RMS = 18, RB_SCL = 27, RB_OVERALL = 36, RB_IMAX = 37,
        RB_DIAG = 38, RB_MDOTIN = 40, RB_SIZE = 41 };
 
+// reported here, and to no later launch check
 #define FS_CK(call)                                                          \
   do {                                                                       \
     cudaError_t e__ = (call);                                                \
     if (e__ != cudaSuccess) {                                                \
+      (void)cudaGetLastError();                                              \
       ctx->err = std::string(#call) + ": " + cudaGetErrorString(e__);        \
       return FS_E_CUDA;                                                      \
     }                                                                        \
@@ -238,6 +241,13 @@ static inline cudaError_t fs_coop_launch(const void *fn, int grid, int block, vo
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+// Device memory of the parts that a solver builds on first use.  Where one of
+// them cannot be had the part gives back what it holds and stays unbuilt.
+static inline cudaError_t fs_alloc(fs_ctx *ctx, void **p, size_t bytes) {
+  if (ctx->test_alloc_left > 0 && --ctx->test_alloc_left == 0) return cudaErrorMemoryAllocation;
+  return cudaMalloc(p, bytes);
 }
 
 // Host arrays go to the device on the context's stream.  That stream does not

@@ -880,7 +880,7 @@ static std::vector<int32_t> color_level(const HostLevel &L, int &ncol) {
 
 template <class T>
 static int mg_alloc(fs_ctx *ctx, T **d, size_t n) {
-  FS_CK(cudaMalloc((void **)d, std::max<size_t>(n, 1) * sizeof(T)));
+  FS_CK(fs_alloc(ctx, (void **)d, std::max<size_t>(n, 1) * sizeof(T)));
   ctx->mg->allocs.push_back(*d);
   return FS_OK;
 }
@@ -890,6 +890,19 @@ static int upv(fs_ctx *ctx, T **d, const std::vector<T> &h) {
   if (rc) return rc;
   if (!h.empty()) FS_CK(fs_upload(ctx, *d, h.data(), h.size() * sizeof(T)));
   return FS_OK;
+}
+
+// a part of the hierarchy: what a failed build holds is given back
+template <class F>
+static int mg_part(fs_ctx *ctx, F &&build) {
+  std::vector<void *> &a = ctx->mg->allocs;
+  const size_t before = a.size();
+  const int rc = build();
+  if (rc) {
+    cudaStreamSynchronize(ctx->st);
+    while (a.size() > before) { cudaFree(a.back()); a.pop_back(); }
+  }
+  return rc;
 }
 
 // the hierarchy and what follows from it on the host; device memory is
@@ -997,20 +1010,17 @@ static int mg_mesh_tables(fs_ctx *ctx) {
 
 static int mg_mesh_tables_once(fs_ctx *ctx) {
   if (ctx->mg->mesh_ready) return FS_OK;
-  int rc = mg_mesh_tables(ctx);
+  int rc = mg_part(ctx, [&] { return mg_mesh_tables(ctx); });
   if (rc) return rc;
   ctx->mg->mesh_ready = true;
   return FS_OK;
 }
 
-// the mesh-ordered levels for cycles in R
 template <class R>
-static int mg_mesh_build(fs_ctx *ctx) {
+static int mg_mesh_vectors(fs_ctx *ctx) {
   constexpr bool f32 = sizeof(R) == sizeof(float);
-  int rc = mg_mesh_tables_once(ctx);
-  if (rc) return rc;
   fs_mg_dev *M = ctx->mg;
-  if (M->mesh_vec[f32]) return FS_OK;
+  int rc;
   std::vector<LevelDev<R>> L(M->nlev);
   for (int q = 0; q < M->nlev; q++) {
     const size_t n = M->n[q];
@@ -1036,7 +1046,18 @@ static int mg_mesh_build(fs_ctx *ctx) {
   LevelDev<R> *dev = nullptr;
   if ((rc = upv(ctx, &dev, L))) return rc;
   if constexpr (f32) M->lev32 = dev; else M->lev64 = dev;
-  M->mesh_vec[f32] = true;
+  return FS_OK;
+}
+
+// the mesh-ordered levels for cycles in R
+template <class R>
+static int mg_mesh_build(fs_ctx *ctx) {
+  int rc = mg_mesh_tables_once(ctx);
+  if (rc) return rc;
+  bool &ready = ctx->mg->mesh_vec[sizeof(R) == sizeof(float)];
+  if (ready) return FS_OK;
+  if ((rc = mg_part(ctx, [&] { return mg_mesh_vectors<R>(ctx); }))) return rc;
+  ready = true;
   return FS_OK;
 }
 
@@ -1313,14 +1334,13 @@ static int mg_vc_arrays(fs_ctx *ctx, const std::vector<std::vector<int32_t>> &id
   if (f32 && W + 1 <= FS_GTMP_BLOCKS) { M->val0[f32] = ctx->gtmp; M->ac0[f32] = ctx->gtmp + W * N; }
   else if ((rc = mg_alloc(ctx, &M->val0[f32], W * N)) || (rc = mg_alloc(ctx, &M->ac0[f32], N))) return rc;
   // FP64 matrices of the other levels, shared by both precisions
+  double *fval[FS_MG_MAXLEV] = {}, *fac[FS_MG_MAXLEV] = {};
   for (int l = 1; l <= lc; l++) {
-    if constexpr (f32) {
-      M->vvalf[l] = val[l]; M->vacf[l] = ac[l];
-      if (!M->vc_ready[0] && ((rc = mg_alloc(ctx, &M->vval[l], M->vnpos[l])) || (rc = mg_alloc(ctx, &M->vac[l], M->n[l])))) return rc;
-    } else { M->vval[l] = val[l]; M->vac[l] = ac[l]; }
+    if constexpr (!f32) { fval[l] = val[l]; fac[l] = ac[l]; }
+    else if (M->vc_ready[0]) { fval[l] = M->vval[l]; fac[l] = M->vac[l]; }
+    else if ((rc = mg_alloc(ctx, &fval[l], M->vnpos[l])) || (rc = mg_alloc(ctx, &fac[l], M->n[l]))) return rc;
   }
-  if constexpr (f32) { M->vvalf[0] = val[0]; M->vacf[0] = ac[0]; }
-  else { val[0] = M->val0[0]; ac[0] = M->ac0[0]; }
+  if constexpr (!f32) { val[0] = M->val0[0]; ac[0] = M->ac0[0]; }
   kp[0] = M->vkp[0]; col[0] = M->vcol[0];
   v.lc = lc;
   for (int l = 0; l <= lc; l++) {
@@ -1341,8 +1361,12 @@ static int mg_vc_arrays(fs_ctx *ctx, const std::vector<std::vector<int32_t>> &id
   VcDev<R> *dev = nullptr;
   if ((rc = mg_alloc(ctx, &dev, 1))) return rc;
   FS_CK(fs_upload(ctx, dev, &v, sizeof(v)));
-  for (int l = 1; l <= lc; l++) { M->vkp[l] = kp[l]; M->vcol[l] = col[l]; }
-  if constexpr (f32) M->vc32 = dev; else M->vc64 = dev;
+  // nothing fails from here on: what both precisions use may change
+  for (int l = 1; l <= lc; l++) { M->vkp[l] = kp[l]; M->vcol[l] = col[l]; M->vval[l] = fval[l]; M->vac[l] = fac[l]; }
+  if constexpr (f32) {
+    for (int l = 0; l <= lc; l++) { M->vvalf[l] = val[l]; M->vacf[l] = ac[l]; }
+    M->vc32 = dev;
+  } else M->vc64 = dev;
   M->vc_ready[f32] = true;
   return FS_OK;
 }
@@ -1353,10 +1377,10 @@ static int mg_vc_build(fs_ctx *ctx, bool f32) {
   const std::vector<std::vector<int32_t>> ids = vc_numbers(M);
   int rc;
   if (!M->vc_map) {
-    if ((rc = mg_vc_map(ctx, ids))) return rc;
+    if ((rc = mg_part(ctx, [&] { return mg_vc_map(ctx, ids); }))) return rc;
     M->vc_map = true;
   }
-  return f32 ? mg_vc_arrays<float>(ctx, ids) : mg_vc_arrays<double>(ctx, ids);
+  return mg_part(ctx, [&] { return f32 ? mg_vc_arrays<float>(ctx, ids) : mg_vc_arrays<double>(ctx, ids); });
 }
 
 // the current matrices in the V-cycle's layout (level0: level 0 alone, the
@@ -1597,6 +1621,12 @@ extern "C" int fs_mg_vcycle_matrix(fs_ctx *ctx, int level, int f32, double *ac, 
 extern "C" int fs_test_wait_timeout(fs_ctx *ctx, int extra) {
   if (!ctx || extra < -64 || extra > 64) return FS_E_ARG;
   ctx->test_wait_extra = extra;
+  return FS_OK;
+}
+
+extern "C" int fs_test_alloc_failure(fs_ctx *ctx, int nth) {
+  if (!ctx || nth < 0) return FS_E_ARG;
+  ctx->test_alloc_left = nth;
   return FS_OK;
 }
 

@@ -971,6 +971,12 @@ __global__ void __launch_bounds__(FS_COOP_BLOCK, FS_KRYLOV_MINB) k_pbcg(PbcgArgs
   if (tid0 == 0) { *a.iters = iter; a.diag[0] = fres; a.diag[1] = ires; }
 }
 
+static int up_list(fs_ctx *ctx, int32_t **d, const std::vector<int32_t> &h) {
+  FS_CK(fs_alloc(ctx, (void **)d, std::max<size_t>(h.size(), 1) * sizeof(int32_t)));
+  if (!h.empty()) FS_CK(fs_upload(ctx, *d, h.data(), h.size() * sizeof(int32_t)));
+  return FS_OK;
+}
+
 // the transpose lists of 'pbcg', built once per context after the ILU levels
 static int pbcg_build(fs_ctx *ctx) {
   fs_ilu *I = ctx->ilu;
@@ -990,19 +996,14 @@ static int pbcg_build(fs_ctx *ctx) {
       const int j = cn[(size_t)si * N + i];
       if (j >= 0 && j != i) { ti[pos[j]] = i; ts[pos[j]] = si; pos[j]++; }
     }
-  auto up = [&](int32_t **d, const std::vector<int32_t> &h) -> int {
-    FS_CK(cudaMalloc((void **)d, std::max<size_t>(h.size(), 1) * sizeof(int32_t)));
-    if (!h.empty()) FS_CK(fs_upload(ctx, *d, h.data(), h.size() * sizeof(int32_t)));
-    return FS_OK;
-  };
   int rc;
-  if ((rc = up(&I->tr_ptr, ptr)) || (rc = up(&I->tr_i, ti)) || (rc = up(&I->tr_si, ts))) return rc;
-  return FS_OK;
+  if ((rc = up_list(ctx, &I->tr_ptr, ptr)) || (rc = up_list(ctx, &I->tr_i, ti)) || (rc = up_list(ctx, &I->tr_si, ts)))
+    fs_ilu_free(ctx);   // half a schedule is none
+  return rc;
 }
 
-static int ilu_build(fs_ctx *ctx) {
-  if (ctx->ilu) return FS_OK;
-  const int N = ctx->N, W = ctx->W;
+static int ilu_tables(fs_ctx *ctx) {
+  const int N = ctx->N;
   const std::vector<int32_t> &ncf = ctx->h_ncf, &cn = ctx->h_cn;
   std::vector<std::vector<std::array<int32_t, 3>>> lo(N);
   for (int i = 0; i < N; i++)
@@ -1042,20 +1043,22 @@ static int ilu_build(fs_ctx *ctx) {
   fs_ilu *I = new fs_ilu();
   ctx->ilu = I;
   I->nlf = nlf; I->nlb = nlb;
-  auto up = [&](int32_t **d, const std::vector<int32_t> &h) -> int {
-    FS_CK(cudaMalloc((void **)d, std::max<size_t>(h.size(), 1) * sizeof(int32_t)));
-    if (!h.empty()) FS_CK(fs_upload(ctx, *d, h.data(), h.size() * sizeof(int32_t)));
-    return FS_OK;
-  };
   int rc;
-  if ((rc = up(&I->lo_ptr, lo_ptr)) || (rc = up(&I->lo_i, lo_i)) || (rc = up(&I->lo_sj, lo_sj)) ||
-      (rc = up(&I->lo_si, lo_si)) || (rc = up(&I->fl_ptr, fl_ptr)) || (rc = up(&I->fl_rows, fl_rows)) ||
-      (rc = up(&I->bl_ptr, bl_ptr)) || (rc = up(&I->bl_rows, bl_rows)))
+  if ((rc = up_list(ctx, &I->lo_ptr, lo_ptr)) || (rc = up_list(ctx, &I->lo_i, lo_i)) ||
+      (rc = up_list(ctx, &I->lo_sj, lo_sj)) || (rc = up_list(ctx, &I->lo_si, lo_si)) ||
+      (rc = up_list(ctx, &I->fl_ptr, fl_ptr)) || (rc = up_list(ctx, &I->fl_rows, fl_rows)) ||
+      (rc = up_list(ctx, &I->bl_ptr, bl_ptr)) || (rc = up_list(ctx, &I->bl_rows, bl_rows)))
     return rc;
-  FS_CK(cudaMalloc(&I->dc, sizeof(double) * N));
-  FS_CK(cudaMalloc(&I->rc, sizeof(double) * N));
-  (void)W;
+  FS_CK(fs_alloc(ctx, (void **)&I->dc, sizeof(double) * N));
+  FS_CK(fs_alloc(ctx, (void **)&I->rc, sizeof(double) * N));
   return FS_OK;
+}
+
+static int ilu_build(fs_ctx *ctx) {
+  if (ctx->ilu) return FS_OK;
+  const int rc = ilu_tables(ctx);
+  if (rc) fs_ilu_free(ctx);   // half a schedule is none
+  return rc;
 }
 
 void fs_ilu_free(fs_ctx *ctx) {

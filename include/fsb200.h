@@ -565,6 +565,10 @@ int fs_set_launch_shape(fs_ctx *ctx, int shape);
  * extra < 0 only the solves of an ensemble's captured graph wait for -extra
  * more.  0 restores normal operation. */
 int fs_test_wait_timeout(fs_ctx *ctx, int extra);
+/* Test of refused device memory (no reference counterpart): the nth allocation
+ * from now of those that solvers make on first use fails (0: none).  The call
+ * returns FS_E_CUDA, and the next one starts that part anew. */
+int fs_test_alloc_failure(fs_ctx *ctx, int nth);
 int fs_ensemble_run(fs_ctx **ctxs, int n, int iters, int launches, double *source_out, int32_t *pc_iters_out,
                     float *ms_out);
 /* fs_ensemble_run_batched: the same with the cases concurrent.  Inside each
