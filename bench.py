@@ -203,19 +203,34 @@ def row_bytes(w: int, r: int) -> int:
     return r + (r + 4) * w
 
 
+def index_bytes(cn, N: int, W: int) -> int:
+    """Bytes that name a row's neighbours on level 0: a pattern byte where the
+    offsets of the neighbours take at most 64 combinations (and at most 8
+    slots), as on meshes numbered in rows and planes, else the index table."""
+    import numpy as np
+    cn = np.asarray(cn, np.int64).reshape(W, N)
+    off = np.where(cn >= 0, cn - np.arange(N), np.iinfo(np.int32).min)
+    key = np.zeros(N, np.int64)
+    for q in range(W):
+        key = key * np.int64(6364136223846793005) + off[q]
+    return 1 if W <= 8 and np.unique(key).size <= 64 else 4 * W
+
+
 def vcycle_bytes(mg: dict, W: int, N: int, r: int) -> float:
-    """Compulsory HBM bytes of one preconditioner V-cycle (one pre- and one
+    """Algorithmic bytes of one preconditioner V-cycle (one pre- and one
     post-sweep, a phase per level and leg): every array a phase touches is read
-    or written once.  Level 0's neighbours come as a pattern byte per row (box
-    meshes); residuals stay on chip.
-      level 0   down                  : pattern 1 + (W+1) r + cell 4 + in 8 + x r
-                up into `out`         : pattern 1 + (W+1) r + parent 4 + in 8 + x r + out 8
+    or written once.  More than what DRAM moves: part of the small levels stays
+    in L2 (112^3 FP64: 845 bytes a row and iteration counted, 740 measured).
+    Level 0's neighbours come as index_bytes per row (mg["index_bytes"]);
+    residuals stay on chip.
+      level 0   down                  : index + (W+1) r + cell 4 + in 8 + x r
+                up into `out`         : index + (W+1) r + parent 4 + in 8 + x r + out 8
       level l   b and x from above 2r; down and up: row + ac r + b r + x r each;
                 the correction from below x 2r (level 1: its result r, read by level 0)
       coarsest  b r from above; dense solve n_c^2 x 8 + b r
     Gathers of neighbour values are L2 traffic and are not counted."""
     sizes, widths, lc = mg["sizes"], mg["widths"], mg["prec_coarsest"]
-    total = sizes[0] * (2.0 * (1 + (W + 1) * r + 4 + 8 + r) + 8)
+    total = sizes[0] * (2.0 * (mg["index_bytes"] + (W + 1) * r + 4 + 8 + r) + 8)
     for l in range(1, lc + 1):
         n, w = sizes[l], widths[l]
         if l == lc and mg["direct"]:
@@ -230,9 +245,9 @@ def amg_bicgstab_bytes(mg: dict, W: int, N: int, r: int, iters: int, calls: int)
       v = A y (row + y 8 + v 8 + r0 8), s (r, v, s, r0 32 + ac and x0 2r),
       t = A z (row + z 8 + t 8 + s 8 + r0 8), x/r/p pass (x, p 32, y, z, s, t, v, r 48
       + ac and x0 2r)
-    with rows of 8 (W+1) + 1 bytes (pattern byte), plus two V-cycles; per launch
-    the set-up (b, r, r0, p, v, x: 48) and dphi (8)."""
-    row0 = 8 * (W + 1) + 1
+    with rows of 8 (W+1) + index bytes, plus two V-cycles; per launch the set-up
+    (b, r, r0, p, v, x: 48) and dphi (8)."""
+    row0 = 8 * (W + 1) + mg["index_bytes"]
     per_it = N * (168 + 4 * r + 2 * row0) + 2 * vcycle_bytes(mg, W, N, r)
     return per_it * iters + N * 56.0 * calls
 
@@ -272,10 +287,13 @@ def solver_roofline(stats: dict, mg: dict | None, N: int, W: int, hbm: float, fo
     if ncu_traffic and best["kernel"] in ncu_traffic:
         t = ncu_traffic[best["kernel"]]
         # DRAM bytes per (row x linear iteration) measured by ncu on a smaller
-        # case of the same kernel, scaled to one launch here
+        # case of the same kernel, scaled to one launch here; traffic_frac is
+        # their rate as a share of the measured bandwidth, next to frac, which
+        # counts bytes that L2 serves too
         traffic = t["bytes_per_row_iter"] * N * best["iters"] / best["calls"]
     return {"bound": "hbm", "kernel": best["kernel"], "achieved": round(achieved, 1), "peak": hbm,
             "unit": "GB/s", "frac": round(achieved / hbm, 4), "traffic": traffic,
+            "traffic_frac": round(traffic / (best["ms"] / best["calls"] * 1e-3) / 1e9 / hbm, 4) if traffic else None,
             "algorithmic_bytes_per_launch": best["bytes"] / best["calls"], "launches": best["calls"],
             "avg_launch_ms": best["ms"] / best["calls"],
             "iters_per_launch": best["iters"] / best["calls"]}
@@ -659,7 +677,7 @@ def main():
     # ---------------- fp64 form: device-resident leg
     s = start(Solver(mesh, case, device=local), init)
     N, W, F = s.N, s.W, s.F
-    mg = s.mg_info()
+    mg, con = s.mg_info(), s.connectivity()["cn"]
     d64 = device_leg(s, args.steps, warm, barrier, local)
     ms_max = reduce_max(d64["ms"], dist, f"cuda:{local}")
     fkeys = ("u", "v", "w", "p") + (("tke", "ted") if case.turbulence else ())
@@ -755,6 +773,7 @@ def main():
         if os.path.exists(tp):
             with open(tp) as f:
                 ncu_t = json.load(f)
+        mg["index_bytes"] = index_bytes(con, N, W)
         roof = solver_roofline(d64["stats"], mg, N, W, hbm, "fp64", ncu_t)
         roof_m = solver_roofline(dmx["stats"], mg, N, W, hbm, "mixed", ncu_t)
         for rf in (roof, roof_m):
@@ -810,8 +829,8 @@ def main():
                           "solver_ms_per_step": [round(x / args.steps, 3) for x in drr["stats"]["ms"]],
                           "lin_iters_last_step": drr["last"]["lin_iters"] if drr["last"] else None,
                           "gpu_launches": drr["launches"], "clocks": drr["clocks"]},
-            "mixed_gs": {"form": "the mixed form with symmetric multicolour Gauss-Seidel smoothing on every level of "
-                                 "the FP32 V-cycle (damped Jacobi in the mixed form)",
+            "mixed_gs": {"form": "the mixed form with symmetric multicolour Gauss-Seidel smoothing on level 0 of "
+                                 "the FP32 V-cycle (damped Jacobi below it, and on every level in the mixed form)",
                          "value": aggregate_rate(world, args.steps, msg_max), "unit": "iter/s",
                          "ms_per_step": msg_max / args.steps, "time_vs_fp64": msg_max / ms_max,
                          "field_rel_l2_vs_fp64": err_g,

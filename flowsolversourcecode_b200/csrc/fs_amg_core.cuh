@@ -468,9 +468,9 @@ struct PCycle {
 // restriction, prolongation and sweep phases cost three to four, and the passes
 // over the level that went with them.  What bounds a phase on a small level is
 // the barrier (1.2 us) and its chain of dependent loads, on a large one DRAM.
-// Measured against the phases it replaces (p' solve, B200): 128^3 75.1 -> 60.0
-// ms for 92 iterations, 295k cells 38.5 -> 24.8 ms for 130, 124k cells 29.5 ->
-// 17.0 ms for 124.  Tried and slower: a warp per chunk of aggregates with the
+// Separate phases (PCycle) take 1.65 times as long at 128^3 and 2.3 times at 124k
+// cells (p' kernels, B200: 75.1 and 29.5 ms against 45.6 and 12.9, with level 0's
+// neighbours from row patterns).  Tried and slower: a warp per chunk of aggregates with the
 // residuals in its own shared array (a chain of six dependent loads per chunk:
 // level 0 of 128^3 72 us against 63, level 1 54 against 19).
 template <class R>

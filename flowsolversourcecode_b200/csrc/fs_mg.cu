@@ -8,9 +8,11 @@
 // reference's discovery order.  Coarsening stops as in Agglomorate
 // (AgglomorateGrid.for:36-72).  The parent maps depend on connectivity only.
 //
-// Per solve: coarse matrices by a per-parent gather (AssembleElementBasedAgglomoratedLHS.for:45-150)
-// in the reference's summation order (seed, then children, each with its
-// slots), so they are bit-identical to the CPU restatement.
+// Per solve: coarse matrices (AssembleElementBasedAgglomoratedLHS.for:45-150) in
+// the reference's summation order (seed, then children, each with its slots),
+// so they are bit-identical to the CPU restatement: entry by entry from static
+// lists in the layout of the one-phase V-cycle (k_mg_coarse), by a per-parent
+// gather in mesh order for 'amg' and the general V-cycle (k_mg_lhs).
 //
 // Cycles run inside ONE persistent cooperative kernel.  Levels with more than
 // FS_MG_SMALL rows are processed by the whole grid (grid barriers between
@@ -24,12 +26,15 @@
 //                     multicolour symmetric Gauss-Seidel in place of the
 //                     sequential sweep, coarse corrections kept between cycles
 //                     as the reference does.
-//   k_amg_bicgstab  : FP64 BiCGSTAB right-preconditioned by one V-cycle
-//                     (PCycle: damped Jacobi, fused restrict/prolong phases,
-//                     dense FP64 inverse of the coarsest level) -- no reference
-//                     row; templated on the V-cycle precision (double, or float
+//   k_amg_bicgstab  : FP64 BiCGSTAB right-preconditioned by one V-cycle with
+//                     over-weighted coarse corrections -- no reference row;
+//                     templated on the V-cycle precision (double, or float
 //                     with FP32 copies of every level's matrix: iterative
-//                     refinement).
+//                     refinement) and its form: damped Jacobi in one phase per
+//                     level and leg with a dense FP64 inverse of the coarsest
+//                     level (MODE 1), the same with Gauss-Seidel smoothing on
+//                     level 0 (MODE 2), and PCycle (MODE 0) for more than one
+//                     sweep or no level small enough for the inverse.
 #include "fs_internal.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
@@ -124,7 +129,7 @@ struct AmgKArgs {
   int32_t *nncnt;     // [fallbacks, uses] of the initial guess, or nullptr
   unsigned *gridbar;  // grid barrier counts: the solve's, then (FS_GRIDBAR_FIT) the guess fit's; zero at launch
   unsigned *teambar;  // team barrier words of PCycle (zeroed before the launch)
-  int32_t *status;    // [0] team-barrier timeout flag
+  int32_t *status;    // [0] set when a bounded wait gave up (grid or team barrier)
   int team_extra;     // fs_test_wait_timeout
   long spin_limit;    // polls of a grid barrier before it gives up
 };
